@@ -37,7 +37,7 @@
 using namespace swg;
 using namespace swg::sdev;
 
-static_assert(KICK_FP64_TILE == 8 && ENC_TILE == 128, "tile sizes of the batched kernels");
+static_assert(KICK_FP64_TILE == 10 && ENC_TILE == 128, "tile sizes of the batched kernels");
 
 // Arguments of the ensemble recursion kernel: the shared base plus per-system tables.
 struct EnsRecArgs {

@@ -5,216 +5,219 @@
 //
 // Every per-body sum must add its terms one at a time in ascending partner order
 // to reproduce the reference's rounding, which leaves no parallelism inside one
-// body's sum.  The expensive part of a term (three differences, r^2, sqrt, an
-// IEEE divide: ~32 FP64 instructions) has no such constraint, so a block of 256
-// threads owns RT receivers and walks the partners in rounds of PT = 256/RT:
-// all 256 threads compute one term each into shared memory, then RT threads
-// fold their receiver's PT terms in order (3 dependent adds per term).  GB300's
-// FP64 pipe (~1 TFLOP/s measured) is then fed from every SM instead of from the
-// npl/128 blocks a thread-per-receiver kernel would launch.
+// body's sum; the terms themselves have no such constraint.  A block therefore owns RT
+// receivers: each of RT term warps forms one receiver's terms, 32 partners a round (one per
+// lane), and the fold warp adds the rounds' terms in order, one lane per (receiver,
+// component), so that one addition of the narrow FP64 pipe serves 3 RT sums.  The terms pass
+// through a ring in shared memory.
 //
-// Modes (see kick.cu): KICK_DIRECT adds Gm_j/(r^2 sqrt r^2) * dx straight into
-// acc; KICK_SPLIT keeps ahi (partners j > i) and ahj (j < i) separately with
-// irij3 = 1/(r^2 sqrt r^2) and finishes acc = (acc + ahi) + ahj.
+// Bound: the FP64 pipe, at 16 cycles per warp instruction and SM (19 for DADD, so additions
+// are issued as DFMA with a factor of one: the same rounding).  The square root, the
+// quotient and the products are formed outside that pipe (fp64_exact.cuh, the same bits), which
+// leaves five additions per pair and 3.2 for the fold: 8.2 instructions, 131 cycles, per 32
+// pairs and SM against ~40 before.  65,537 tp x 2047 pl: 10.3 -> 2.6 ms (16,384 pl: 22.6 -> 5.4 ms),
+// FP64 pipe 72%, ALU pipe 66%, issue slots 63% busy (ncu); four blocks of 40 registers per SM
+// (three of 56: 2.8 ms, two: 3.9 ms): the long chains of dependent instructions want warps.
+//
 #include <cuda_runtime.h>
 
+#include "fp64_exact.cuh"
 #include "swg_internal.cuh"
 
 namespace swg {
 
-constexpr int FT = 256;  // threads per block
-constexpr int FP64_RT = 8;  // receivers per block (FT / FP64_RT partners per round)
+constexpr int FP64_RT = KICK_FP64_TILE;  // receivers per block of the batched forms
+constexpr int FP64_RTMAX = 10;           // most receivers per block (30 of the fold warp's 32 lanes)
+constexpr int PT = 32;                   // partners per round
 
-// Receivers [i0, i0 + RT) of one system against all its partners, whole block.
-template <bool RAD, int MODE, int RT>
-__device__ __forceinline__ void fp64_plpl_group(int npl, int nplm, const double *__restrict__ r,
-                                                const double *__restrict__ Gm, const double *__restrict__ R,
-                                                double *__restrict__ acc, int acc_is_zero, int i0) {
-    constexpr int PT = FT / RT;
-    __shared__ double sx[PT], sy[PT], sz[PT], sg[PT], sr[PT];
-    __shared__ double tx[RT][PT + 1], ty[RT][PT + 1], tz[RT][PT + 1];
-    __shared__ unsigned char tf[RT][PT];
-    const int t = threadIdx.x;
-    const int rr = t / PT, pp = t % PT;
-    const int i = i0 + rr;  // receiver of this thread's terms
-    double xi = 0, yi = 0, zi = 0, Ri = 0;
-    if (i < npl) {
-        xi = r[3 * i + 0];
-        yi = r[3 * i + 1];
-        zi = r[3 * i + 2];
-        if (RAD) Ri = R[i];
-    }
-    const int jend = (i < nplm) ? npl : nplm;  // partner range of receiver i
-    // accumulators: thread t < RT owns receiver i0 + t
-    const int ia = i0 + t;
-    double ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
-    if (MODE == KICK_DIRECT && t < RT && ia < npl && !acc_is_zero) {
-        ax = acc[3 * ia + 0];
-        ay = acc[3 * ia + 1];
-        az = acc[3 * ia + 2];
-    }
-    const int blk_jend = (i0 < nplm) ? npl : nplm;
-    for (int j0 = 0; j0 < blk_jend; j0 += PT) {
-        if (t < PT && j0 + t < npl) {
-            const int jl = j0 + t;
-            sx[t] = r[3 * jl + 0];
-            sy[t] = r[3 * jl + 1];
-            sz[t] = r[3 * jl + 2];
-            sg[t] = Gm[jl];
-            if (RAD) sr[t] = R[jl];
+static_assert(3 * FP64_RTMAX <= 32, "one fold warp");
+__host__ __device__ constexpr int fp64_threads(int rt) { return 32 * (rt + 1); }
+// doubles per partner of a stage (odd: conflict-free columns) and bytes of the ring
+__host__ __device__ constexpr int term_stride(int rt) { return (3 * rt) | 1; }
+
+// Opaque one: an addition as fma(a, 1, b) stays a DFMA.
+__constant__ double c_one = 1.0;
+__constant__ double c_mone = -1.0;
+__device__ __forceinline__ double add1(double a, double b) { return fma(a, c_one, b); }
+__device__ __forceinline__ double sub1(double a, double b) { return fma(b, c_mone, a); }
+
+enum { KICK_TP = 2 };  // beside KICK_DIRECT and KICK_SPLIT
+
+// Terms of ST = 2 rounds: a ring between the term warps and the fold warp.  Barrier 1 + s:
+// a round's terms are in stage s (term warps arrive, the fold warp waits); barrier 3 + s: its
+// sums are made (the fold warp arrives, the term warps wait).  Three, four and six stages
+// measured no faster.
+constexpr int ST = 2;
+template <int BASE>
+__device__ __forceinline__ void bar_sync(int s, int n) {  // constant barrier numbers: five per block
+    if (s) asm volatile("bar.sync %0, %1;" ::"n"(BASE + 1), "r"(n) : "memory");
+    else asm volatile("bar.sync %0, %1;" ::"n"(BASE), "r"(n) : "memory");
+}
+template <int BASE>
+__device__ __forceinline__ void bar_arrive(int s, int n) {
+    if (s) asm volatile("bar.arrive %0, %1;" ::"n"(BASE + 1), "r"(n) : "memory");
+    else asm volatile("bar.arrive %0, %1;" ::"n"(BASE), "r"(n) : "memory");
+}
+constexpr int FULL = 1, EMPTY = 3;
+
+// A float not below 2 R^2, so that bound(R_i) + bound(R_j) >= (R_i + R_j)^2: R cut to its
+// leading 24 bits and one unit more (a conversion would take the FP64 pipe), infinity out of
+// range.
+__device__ __forceinline__ float radius_bound(double R) {
+    const int hi = __double2hiint(R), lo = __double2loint(R);
+    if (!x_ok(hi)) return (hi | lo) == 0 ? 0.0f : __int_as_float(0x7f800000);
+    const float f = __int_as_float(__funnelshift_l(lo, hi - ((1023 - 127) << 20), 3) + 1);
+    return __fmul_ru(2.0f, __fmul_ru(f, f));
+}
+
+// Product of a factor f (x_ok unless bad) and a displacement: x_mul where both operands are in
+// range, the zero itself for a zero displacement; elsewhere bad.
+__device__ __forceinline__ double mul_disp(double f, double d, bool &bad) {
+    const int h = __double2hiint(d) & 0x7fffffff;
+    const bool zero = (h | __double2loint(d)) == 0;
+    bad |= !x_ok(h) && !zero;
+    const double p = x_mul(f, d);
+    return zero ? d : p;
+}
+
+// Square of a displacement: zero for a zero one, bad out of range.
+__device__ __forceinline__ double sqr_disp(double d, bool &bad) {
+    const int h = __double2hiint(d) & 0x7fffffff;
+    const bool zero = (h | __double2loint(d)) == 0;
+    bad |= !x_ok(h) && !zero;
+    const double p = x_sqr(d);
+    return zero ? 0.0 : p;
+}
+
+// Receivers [i0, i0 + RT) (those below nrecv) of one system against all its partners, whole
+// block of fp64_threads(RT) threads; sh: fp64_shared(RT) bytes.  MODE: KICK_DIRECT and
+// KICK_SPLIT (pl-pl), KICK_TP (swiftest_kick.f90:374-415: acc -= Gm_j / (r^2 sqrt r^2)
+// (r_tp - r_j), masked).
+template <bool RAD, int MODE>
+__device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int nplm, const double *__restrict__ rr,
+                                           const double *__restrict__ rp, const double *__restrict__ Gm,
+                                           const double *__restrict__ R, const int32_t *__restrict__ lmask,
+                                           double *__restrict__ acc, int acc_is_zero, int i0, double *sh) {
+    const int nth = fp64_threads(RT), ts = term_stride(RT);
+    const int w = (int)(threadIdx.x >> 5) - 1, lane = threadIdx.x & 31;
+    constexpr bool plpl = MODE != KICK_TP;
+    const int jmax = plpl && i0 >= nplm ? nplm : npart;  // partners of the block's receivers
+    const int rounds = (jmax + PT - 1) / PT;
+    if (w >= 0) {  // term warps: warp w + 1 of the block
+        // a term that leaves the sum as it is, signed zeros included
+        const double neutral = plpl ? -0.0 : 0.0;
+        const int i = i0 + w;
+        const bool on = i < nrecv && (plpl || lmask[i] != 0);
+        double xi = 0, yi = 0, zi = 0;
+        float rbi = 0;
+        if (on) {
+            xi = rr[3 * i + 0];
+            yi = rr[3 * i + 1];
+            zi = rr[3 * i + 2];
+            if (RAD) rbi = radius_bound(R[i]);
         }
-        __syncthreads();
-        const int j = j0 + pp;
-        unsigned char flag = 0;
-        double fx = 0, fy = 0, fz = 0;
-        if (i < npl && j < jend && j != i) {
-            const double rx = sx[pp] - xi;
-            const double ry = sy[pp] - yi;
-            const double rz = sz[pp] - zi;
-            const double rji2 = rx * rx + ry * ry + rz * rz;
-            bool ok = true;
-            if (RAD) {
-                const double rs = Ri + sr[pp];
-                ok = rji2 > rs * rs;
-            }
-            if (ok) {
+        const int jend = !on ? 0 : (plpl && i >= nplm ? nplm : npart);
+        double *out = sh + lane * ts + 3 * w;
+        for (int r = 0; r < rounds; r++) {
+            const int j = r * PT + lane, st = r % ST;
+            double fx = neutral, fy = neutral, fz = neutral;
+            if (j < jend && (!plpl || j != i)) {
+                const double g = Gm[j];
+                const double xj = rp[3 * j + 0], yj = rp[3 * j + 1], zj = rp[3 * j + 2];
+                const double dx = plpl ? sub1(xj, xi) : sub1(xi, xj);
+                const double dy = plpl ? sub1(yj, yi) : sub1(yi, yj);
+                const double dz = plpl ? sub1(zj, zi) : sub1(zi, zj);
+                bool bad = false, near = false;
+                const double r2 = add1(add1(sqr_disp(dx, bad), sqr_disp(dy, bad)), sqr_disp(dz, bad));
+                const int h = __double2hiint(r2);
+                bad |= !x_ok(h) || !x_ok(__double2hiint(g));
+                if (RAD) near = !(__int_as_float((h - ((1023 - 127) << 20)) << 3) > __fadd_ru(rbi, radius_bound(R[j])));
+                const double s = x_sqrt(r2, bad);
+                const double p = x_mul(r2, s);
                 double fac;
-                if (MODE == KICK_DIRECT) {
-                    fac = sg[pp] / (rji2 * sqrt(rji2));
-                    flag = 1;
+                if (MODE == KICK_SPLIT) {
+                    const XNum one = {1.0f, 0.0f, 0x3ff00000, 0};
+                    fac = g * x_div(one, p, bad);
                 } else {
-                    const double irij3 = 1.0 / (rji2 * sqrt(rji2));
-                    fac = sg[pp] * irij3;
-                    flag = j > i ? 1 : 2;
+                    fac = x_div(x_num(g), p, bad);
                 }
-                fx = fac * rx;
-                fy = fac * ry;
-                fz = fac * rz;
-            }
-        }
-        tx[rr][pp] = fx;
-        ty[rr][pp] = fy;
-        tz[rr][pp] = fz;
-        tf[rr][pp] = flag;
-        __syncthreads();
-        if (t < RT && ia < npl) {
-#pragma unroll 4
-            for (int p = 0; p < PT; p++) {
-                const unsigned char f = tf[t][p];
-                if (f == 1) {
-                    ax = ax + tx[t][p];
-                    ay = ay + ty[t][p];
-                    az = az + tz[t][p];
-                } else if (f == 2) {
-                    bx = bx + tx[t][p];
-                    by = by + ty[t][p];
-                    bz = bz + tz[t][p];
+                fx = mul_disp(fac, dx, bad);
+                fy = mul_disp(fac, dy, bad);
+                fz = mul_disp(fac, dz, bad);
+                if (bad || near) {  // rare: native operations
+                    const double q2 = dx * dx + dy * dy + dz * dz;
+                    const double q = q2 * sqrt(q2);
+                    fac = MODE == KICK_SPLIT ? g * (1.0 / q) : g / q;
+                    fx = fac * dx;
+                    fy = fac * dy;
+                    fz = fac * dz;
+                    if (RAD) {
+                        const double rs = R[i] + R[j];
+                        if (!(q2 > rs * rs)) fx = fy = fz = neutral;
+                    }
                 }
             }
+            __syncwarp();
+            if (r >= ST) bar_sync<EMPTY>(st, nth);
+            double *o = out + st * PT * ts;
+            o[0] = fx;
+            o[1] = fy;
+            o[2] = fz;
+            __syncwarp();
+            bar_arrive<FULL>(st, nth);
         }
-        // the next round's first barrier orders these reads before the next term writes
+        return;
     }
-    if (t < RT && ia < npl) {
-        if (MODE == KICK_DIRECT) {
-            acc[3 * ia + 0] = ax;
-            acc[3 * ia + 1] = ay;
-            acc[3 * ia + 2] = az;
-        } else {
-            const double a0 = acc_is_zero ? 0.0 : acc[3 * ia + 0];
-            const double a1 = acc_is_zero ? 0.0 : acc[3 * ia + 1];
-            const double a2 = acc_is_zero ? 0.0 : acc[3 * ia + 2];
-            acc[3 * ia + 0] = a0 + ax + bx;
-            acc[3 * ia + 1] = a1 + ay + by;
-            acc[3 * ia + 2] = a2 + az + bz;
-        }
-    }
-}
-
-// pl -> tp (swiftest_kick.f90:374-415): acc -= Gm_j/(r^2 sqrt r^2) * (r_tp - r_j), masked
-template <int RT>
-__device__ __forceinline__ void fp64_tp_group(int ntp, int npl, const double *__restrict__ rtp,
-                                              const double *__restrict__ rpl, const double *__restrict__ Gm,
-                                              const int32_t *__restrict__ lmask, double *__restrict__ acc,
-                                              int acc_is_zero, int i0) {
-    constexpr int PT = FT / RT;
-    __shared__ double sx[PT], sy[PT], sz[PT], sg[PT];
-    __shared__ double tx[RT][PT + 1], ty[RT][PT + 1], tz[RT][PT + 1];
-    const int t = threadIdx.x;
-    const int rr = t / PT, pp = t % PT;
-    const int i = i0 + rr;
-    const bool iact = i < ntp && lmask[i] != 0;
-    double xi = 0, yi = 0, zi = 0;
-    if (iact) {
-        xi = rtp[3 * i + 0];
-        yi = rtp[3 * i + 1];
-        zi = rtp[3 * i + 2];
-    }
-    const int ia = i0 + t;
-    const bool aact = t < RT && ia < ntp && lmask[ia] != 0;
-    double ax = 0, ay = 0, az = 0;
-    if (aact && !acc_is_zero) {
-        ax = acc[3 * ia + 0];
-        ay = acc[3 * ia + 1];
-        az = acc[3 * ia + 2];
-    }
-    for (int j0 = 0; j0 < npl; j0 += PT) {
-        if (t < PT && j0 + t < npl) {
-            const int jl = j0 + t;
-            sx[t] = rpl[3 * jl + 0];
-            sy[t] = rpl[3 * jl + 1];
-            sz[t] = rpl[3 * jl + 2];
-            sg[t] = Gm[jl];
-        }
-        __syncthreads();
-        double fx = 0, fy = 0, fz = 0;
-        if (iact && j0 + pp < npl) {
-            const double rx = xi - sx[pp];
-            const double ry = yi - sy[pp];
-            const double rz = zi - sz[pp];
-            const double rji2 = rx * rx + ry * ry + rz * rz;
-            const double fac = sg[pp] / (rji2 * sqrt(rji2));
-            fx = fac * rx;
-            fy = fac * ry;
-            fz = fac * rz;
-        }
-        tx[rr][pp] = fx;
-        ty[rr][pp] = fy;
-        tz[rr][pp] = fz;
-        __syncthreads();
-        if (aact) {
-            const int np = min(PT, npl - j0);
-#pragma unroll 4
+    // the fold warp: lane f owns component f % 3 of receiver f / 3
+    const int f = threadIdx.x, ia = i0 + f / 3, d = f % 3;
+    const bool own = f < 3 * RT && ia < nrecv, fold = own && (plpl || lmask[ia] != 0);
+    double v = 0.0, vb = 0.0;
+    if (MODE != KICK_SPLIT && fold && !acc_is_zero) v = acc[3 * ia + d];
+    for (int r = 0; r < rounds; r++) {
+        const int j0 = r * PT, np = min(PT, jmax - j0), st = r % ST;
+        bar_sync<FULL>(st, nth);
+        if (fold) {
+            const double *t = sh + st * PT * ts + f;
+#pragma unroll 8
             for (int p = 0; p < np; p++) {
-                ax = ax - tx[t][p];
-                ay = ay - ty[t][p];
-                az = az - tz[t][p];
+                if (MODE == KICK_SPLIT && j0 + p == ia) {  // partners below, then above the receiver
+                    vb = v;
+                    v = 0.0;
+                }
+                v = MODE == KICK_TP ? sub1(v, t[p * ts]) : add1(t[p * ts], v);
             }
         }
+        __syncwarp();
+        if (r + ST < rounds) bar_arrive<EMPTY>(st, nth);
     }
-    if (aact) {
-        acc[3 * ia + 0] = ax;
-        acc[3 * ia + 1] = ay;
-        acc[3 * ia + 2] = az;
-    } else if (t < RT && ia < ntp && acc_is_zero) {
-        acc[3 * ia + 0] = 0.0;
-        acc[3 * ia + 1] = 0.0;
-        acc[3 * ia + 2] = 0.0;
+    if (!own) return;
+    if (MODE == KICK_SPLIT) {
+        if (ia >= jmax) {  // no partner above the receiver
+            vb = v;
+            v = 0.0;
+        }
+        acc[3 * ia + d] = (acc_is_zero ? 0.0 : acc[3 * ia + d]) + v + vb;
+    } else if (fold) {
+        acc[3 * ia + d] = v;
+    } else if (acc_is_zero) {
+        acc[3 * ia + d] = 0.0;
     }
 }
 
-template <bool RAD, int MODE, int RT>
-__global__ void __launch_bounds__(FT) k_kick_plpl_fp64(int npl, int nplm, const double *__restrict__ r,
-                                                      const double *__restrict__ Gm, const double *__restrict__ R,
-                                                      double *__restrict__ acc, int acc_is_zero) {
-    fp64_plpl_group<RAD, MODE, RT>(npl, nplm, r, Gm, R, acc, acc_is_zero, blockIdx.x * RT);
+template <bool RAD, int MODE>
+__global__ void __launch_bounds__(fp64_threads(FP64_RTMAX), 4)
+    k_kick_plpl_fp64(int RT, int npl, int nplm, const double *__restrict__ r, const double *__restrict__ Gm,
+                     const double *__restrict__ R, double *__restrict__ acc, int acc_is_zero) {
+    extern __shared__ double sh[];
+    fp64_group<RAD, MODE>(RT, npl, npl, nplm, r, r, Gm, R, nullptr, acc, acc_is_zero, blockIdx.x * RT, sh);
 }
 
-template <int RT>
-__global__ void __launch_bounds__(FT) k_kick_tp_fp64(int ntp, int npl, const double *__restrict__ rtp,
-                                                    const double *__restrict__ rpl, const double *__restrict__ Gm,
-                                                    const int32_t *__restrict__ lmask, double *__restrict__ acc,
-                                                    int acc_is_zero) {
-    fp64_tp_group<RT>(ntp, npl, rtp, rpl, Gm, lmask, acc, acc_is_zero, blockIdx.x * RT);
+__global__ void __launch_bounds__(fp64_threads(FP64_RTMAX), 4)
+    k_kick_tp_fp64(int RT, int ntp, int npl, const double *__restrict__ rtp, const double *__restrict__ rpl,
+                   const double *__restrict__ Gm, const int32_t *__restrict__ lmask, double *__restrict__ acc,
+                   int acc_is_zero) {
+    extern __shared__ double sh[];
+    fp64_group<false, KICK_TP>(RT, ntp, npl, 0, rtp, rpl, Gm, nullptr, lmask, acc, acc_is_zero, blockIdx.x * RT, sh);
 }
 
 // Batched (ensemble) forms: block b takes item b = (system s, first receiver r0) of a
@@ -224,60 +227,76 @@ __global__ void __launch_bounds__(FT) k_kick_tp_fp64(int ntp, int npl, const dou
 // system does (KICK_SPLIT when the semi-interacting bodies outnumber the others); without
 // it every system is fully interacting (KICK_DIRECT).  With sys_flag, the pl-pl form kicks
 // only systems whose flag equals `phase`.
-template <bool RAD, int RT>
-__global__ void __launch_bounds__(FT) k_kick_plpl_fp64_batched(const int4 *__restrict__ items,
-                                                              const int32_t *__restrict__ poff,
-                                                              const int32_t *__restrict__ npl,
-                                                              const double *__restrict__ r,
-                                                              const double *__restrict__ Gm,
-                                                              const double *__restrict__ R, double *__restrict__ acc,
-                                                              int acc_is_zero, const int32_t *__restrict__ sys_flag,
-                                                              int phase, const int32_t *__restrict__ nplm) {
+template <bool RAD>
+__global__ void __launch_bounds__(fp64_threads(FP64_RT), 4)
+    k_kick_plpl_fp64_batched(const int4 *__restrict__ items, const int32_t *__restrict__ poff,
+                             const int32_t *__restrict__ npl, const double *__restrict__ r,
+                             const double *__restrict__ Gm, const double *__restrict__ R, double *__restrict__ acc,
+                             int acc_is_zero, const int32_t *__restrict__ sys_flag, int phase,
+                             const int32_t *__restrict__ nplm) {
+    extern __shared__ double sh[];
     const int4 w = items[blockIdx.x];
     if (sys_flag && sys_flag[w.x] != phase) return;  // another launch's system
     const int o = poff[w.x], n = npl[w.x], m = nplm ? nplm[w.x] : n;
+    const double *rs = r + 3 * (size_t)o, *Rs = RAD ? R + o : nullptr;
+    double *as = acc + 3 * (size_t)o;
     if (n - m > m)  // block-uniform
-        fp64_plpl_group<RAD, KICK_SPLIT, RT>(n, m, r + 3 * (size_t)o, Gm + o, RAD ? R + o : nullptr,
-                                             acc + 3 * (size_t)o, acc_is_zero, w.y);
+        fp64_group<RAD, KICK_SPLIT>(FP64_RT, n, n, m, rs, rs, Gm + o, Rs, nullptr, as, acc_is_zero, w.y, sh);
     else
-        fp64_plpl_group<RAD, KICK_DIRECT, RT>(n, m, r + 3 * (size_t)o, Gm + o, RAD ? R + o : nullptr,
-                                              acc + 3 * (size_t)o, acc_is_zero, w.y);
+        fp64_group<RAD, KICK_DIRECT>(FP64_RT, n, n, m, rs, rs, Gm + o, Rs, nullptr, as, acc_is_zero, w.y, sh);
 }
 
-template <int RT>
-__global__ void __launch_bounds__(FT) k_kick_tp_fp64_batched(const int4 *__restrict__ items,
-                                                            const int32_t *__restrict__ toff,
-                                                            const int32_t *__restrict__ ntp,
-                                                            const int32_t *__restrict__ poff,
-                                                            const int32_t *__restrict__ npl,
-                                                            const double *__restrict__ rtp,
-                                                            const double *__restrict__ rpl,
-                                                            const double *__restrict__ Gm,
-                                                            const int32_t *__restrict__ lmask,
-                                                            double *__restrict__ acc, int acc_is_zero) {
+__global__ void __launch_bounds__(fp64_threads(FP64_RT), 4)
+    k_kick_tp_fp64_batched(const int4 *__restrict__ items, const int32_t *__restrict__ toff,
+                           const int32_t *__restrict__ ntp, const int32_t *__restrict__ poff,
+                           const int32_t *__restrict__ npl, const double *__restrict__ rtp,
+                           const double *__restrict__ rpl, const double *__restrict__ Gm,
+                           const int32_t *__restrict__ lmask, double *__restrict__ acc, int acc_is_zero) {
+    extern __shared__ double sh[];
     const int4 w = items[blockIdx.x];
     const int ot = toff[w.x], op = poff[w.x];
-    fp64_tp_group<RT>(ntp[w.x], npl[w.x], rtp + 3 * (size_t)ot, rpl + 3 * (size_t)op, Gm + op, lmask + ot,
-                      acc + 3 * (size_t)ot, acc_is_zero, w.y);
+    fp64_group<false, KICK_TP>(FP64_RT, ntp[w.x], npl[w.x], 0, rtp + 3 * (size_t)ot, rpl + 3 * (size_t)op, Gm + op,
+                               nullptr, lmask + ot, acc + 3 * (size_t)ot, acc_is_zero, w.y, sh);
 }
 
+constexpr size_t fp64_shared(int rt) { return sizeof(double) * ST * PT * term_stride(rt); }
+
 static inline int div_up_i(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
+
+// Receivers per block of a single system's kick.  An SM's time per round of 32 partners is the
+// work of its blocks (TERM_C cycles per receiver, FOLD_C per fold warp), at least the
+// fold's chain of 32 dependent additions (~2100 cycles); the fullest SM sets the time, and the
+// smallest blocks that reach it leave the least to wait for.
+static int fp64_rt(int num_sms, int n) {
+    constexpr int TERM_C = 130, FOLD_C = 512, CHAIN_C = 2100;
+    int best = 1;
+    int64_t cost = INT64_MAX;
+    for (int rt = 1; rt <= FP64_RTMAX; rt++) {
+        const int64_t per_sm = div_up_i(div_up_i(n, rt), num_sms > 0 ? num_sms : 152);
+        const int64_t c = per_sm * (rt * TERM_C + FOLD_C), t = c > CHAIN_C ? c : CHAIN_C;
+        if (t < cost) {
+            cost = t;
+            best = rt;
+        }
+    }
+    return best;
+}
 
 int kick_plpl_fp64(swg_ctx *c, int32_t npl, int32_t nplm, const double *r, const double *Gm, const double *R,
                    double *acc, int mode, int acc_is_zero) {
     if (npl <= 0) return SWG_OK;
-    constexpr int RT = 8;
-    const int grid = div_up_i(npl, RT);
+    const int rt = fp64_rt(c->num_sms, npl), grid = div_up_i(npl, rt), th = fp64_threads(rt);
+    const cudaStream_t st = c->stream;
     if (mode == KICK_DIRECT) {
         if (R)
-            k_kick_plpl_fp64<true, KICK_DIRECT, RT><<<grid, FT, 0, c->stream>>>(npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<true, KICK_DIRECT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
         else
-            k_kick_plpl_fp64<false, KICK_DIRECT, RT><<<grid, FT, 0, c->stream>>>(npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<false, KICK_DIRECT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
     } else {
         if (R)
-            k_kick_plpl_fp64<true, KICK_SPLIT, RT><<<grid, FT, 0, c->stream>>>(npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<true, KICK_SPLIT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
         else
-            k_kick_plpl_fp64<false, KICK_SPLIT, RT><<<grid, FT, 0, c->stream>>>(npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<false, KICK_SPLIT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
     }
     c->launches++;
     return launch_status(c, "kick_plpl_fp64");
@@ -286,8 +305,9 @@ int kick_plpl_fp64(swg_ctx *c, int32_t npl, int32_t nplm, const double *r, const
 int kick_tp_fp64(swg_ctx *c, int32_t ntp, int32_t npl, const double *rtp, const double *rpl, const double *Gm,
                  const int32_t *lmask, double *acc, int acc_is_zero) {
     if (ntp <= 0) return SWG_OK;
-    constexpr int RT = 8;
-    k_kick_tp_fp64<RT><<<div_up_i(ntp, RT), FT, 0, c->stream>>>(ntp, npl, rtp, rpl, Gm, lmask, acc, acc_is_zero);
+    const int rt = fp64_rt(c->num_sms, ntp);
+    k_kick_tp_fp64<<<div_up_i(ntp, rt), fp64_threads(rt), fp64_shared(rt), c->stream>>>(rt, ntp, npl, rtp, rpl, Gm, lmask, acc,
+                                                                          acc_is_zero);
     c->launches++;
     return launch_status(c, "kick_tp_fp64");
 }
@@ -296,12 +316,13 @@ int kick_plpl_fp64_batched(swg_ctx *c, bool rad, int nitems, const int4 *items, 
                            const int32_t *npl, const double *r, const double *Gm, const double *R, double *acc,
                            int acc_is_zero, const int32_t *sys_flag, int phase, const int32_t *nplm) {
     if (nitems <= 0) return SWG_OK;
+    constexpr int th = fp64_threads(FP64_RT);
     if (rad)
-        k_kick_plpl_fp64_batched<true, FP64_RT><<<nitems, FT, 0, c->stream>>>(items, poff, npl, r, Gm, R, acc,
-                                                                              acc_is_zero, sys_flag, phase, nplm);
+        k_kick_plpl_fp64_batched<true><<<nitems, th, fp64_shared(FP64_RT), c->stream>>>(items, poff, npl, r, Gm, R, acc, acc_is_zero,
+                                                                     sys_flag, phase, nplm);
     else
-        k_kick_plpl_fp64_batched<false, FP64_RT><<<nitems, FT, 0, c->stream>>>(items, poff, npl, r, Gm, nullptr, acc,
-                                                                               acc_is_zero, sys_flag, phase, nplm);
+        k_kick_plpl_fp64_batched<false><<<nitems, th, fp64_shared(FP64_RT), c->stream>>>(items, poff, npl, r, Gm, nullptr, acc,
+                                                                      acc_is_zero, sys_flag, phase, nplm);
     c->launches++;
     return launch_status(c, "kick_plpl_fp64_batched");
 }
@@ -310,8 +331,8 @@ int kick_tp_fp64_batched(swg_ctx *c, int nitems, const int4 *items, const int32_
                          const int32_t *poff, const int32_t *npl, const double *rtp, const double *rpl,
                          const double *Gm, const int32_t *lmask, double *acc, int acc_is_zero) {
     if (nitems <= 0) return SWG_OK;
-    k_kick_tp_fp64_batched<FP64_RT><<<nitems, FT, 0, c->stream>>>(items, toff, ntp, poff, npl, rtp, rpl, Gm, lmask,
-                                                                  acc, acc_is_zero);
+    k_kick_tp_fp64_batched<<<nitems, fp64_threads(FP64_RT), fp64_shared(FP64_RT), c->stream>>>(items, toff, ntp, poff, npl, rtp, rpl, Gm,
+                                                                            lmask, acc, acc_is_zero);
     c->launches++;
     return launch_status(c, "kick_tp_fp64_batched");
 }
