@@ -22,28 +22,72 @@ namespace sdev {
 enum { CB_VB = 0, CB_RB = 3, CB_PTBEG = 6, CB_PTEND = 9, CB_N = 12 };
 
 // ---------------------------------------------------------------- small kernels
-// Ordered sums of the reference's O(N) serial loops.  exact == 1: the terms are formed
-// by the whole block into shared memory, chunk by chunk, and thread 0 adds them one at
-// a time in the reference's index order, which reproduces its rounding.  exact == 0:
-// thread t adds its own terms t, t + RB, t + 2 RB, ... in registers, then the block
-// combines the partial sums as a tree (warp shuffles, then one warp over the warp
-// sums): a fixed order, so results are deterministic, with no serial chain.  The block
-// may have any multiple of 32 threads up to RB.
+// Ordered sums of the reference's O(N) serial loops.  exact == 1: blk_serial_sums, the
+// reference's rounding.  exact == 0: thread t adds its own terms t, t + RB, t + 2 RB, ... in
+// registers, then the block combines the partial sums as a tree (warp shuffles, then one warp
+// over the warp sums): a fixed order, so results are deterministic, with no serial chain.  The
+// block may have any multiple of 32 threads from 64 up to RB.
 constexpr int RB = 1024;  // most threads of the reduction kernels
 
 struct Sum3 {
     double x, y, z;
 };
 
-// Sum over i of sign*term(i) for i = 0..n-1 (reverse: n-1..0); term_fn(i, x, y, z)
-// writes the components and returns the 0/1 mask.
-// shared-memory workspace of ordered_sum3 (one per kernel)
+constexpr int SCH = 256;  // terms per chunk of the serial sums
+// shared-memory workspace of the ordered sums (one per kernel)
 struct SumScratch {
-    double cx[RB], cy[RB], cz[RB];
+    double t[2][4][SCH + 1];  // two chunks of up to four components (offset: conflict-free columns)
     double rx[RB / 32], ry[RB / 32], rz[RB / 32];
-    unsigned char cm[RB];
+    double sum[4];
     Sum3 acc;
 };
+
+// Sums of NC components (up to four) over i = 0 .. n-1 (reverse: n-1 .. 0), one addition at a
+// time in that order, whole block; the sums are left in sh.sum.  term_fn(i, t) writes the NC
+// terms of index i and returns whether they count; one that does not is added as -0.0, which
+// leaves every sum as it is.  Lane c of warp 0 adds component c, so one FP64 addition (64 cycles,
+// the chain's dependent latency) serves all components, while the other warps form the next
+// chunk's terms: 64 cycles a term (192 with one lane adding three components in turn: the
+// linear drift of 2000 bodies took 236 us, now 86 us; an integer prefix scan over the terms of
+// one binade gives the same bits but restarts at every change of binade, and was no faster).
+template <int NC, class TermFn>
+__device__ void blk_serial_sums(int n, bool reverse, TermFn term_fn, SumScratch &sh) {
+    const int w = threadIdx.x >> 5, c = threadIdx.x & 31, chunks = (n + SCH - 1) / SCH;
+    auto form = [&](int k, int first, int step) {
+        for (int q = first; q < SCH && k * SCH + q < n; q += step) {
+            const int i = k * SCH + q;
+            double t[NC];
+            const bool on = term_fn(reverse ? n - 1 - i : i, t);
+#pragma unroll
+            for (int d = 0; d < NC; d++) sh.t[k & 1][d][q] = on ? t[d] : -0.0;
+        }
+    };
+    __syncthreads();  // a previous sum's result may still be being read
+    form(0, threadIdx.x, blockDim.x);
+    double s = 0.0;
+    for (int k = 0; k < chunks; k++) {
+        __syncthreads();
+        if (w > 0) {
+            form(k + 1, threadIdx.x - 32, blockDim.x - 32);
+        } else if (c < NC) {
+            const double *t = sh.t[k & 1][c];
+            const int cnt = min(SCH, n - k * SCH);
+#pragma unroll 16
+            for (int q = 0; q < cnt; q++) s = s + t[q];
+        }
+    }
+    if (w == 0 && c < NC) sh.sum[c] = s;
+    __syncthreads();
+}
+
+// The three components of a sum divided by q, whole block: three lanes divide (in every warp
+// of a 1024-thread block the quotients would hold the FP64 pipe for 6 us).
+__device__ __forceinline__ Sum3 blk_quotient(const Sum3 &a, double q, SumScratch &sh) {
+    __syncthreads();  // a previous result may still be being read
+    if (threadIdx.x < 3) sh.sum[threadIdx.x] = (threadIdx.x == 0 ? a.x : threadIdx.x == 1 ? a.y : a.z) / q;
+    __syncthreads();
+    return {sh.sum[0], sh.sum[1], sh.sum[2]};
+}
 
 __device__ __forceinline__ void warp_sum3(double &x, double &y, double &z) {
     for (int off = 16; off > 0; off >>= 1) {
@@ -53,42 +97,23 @@ __device__ __forceinline__ void warp_sum3(double &x, double &y, double &z) {
     }
 }
 
+// Sum over i of sign*term(i) for i = 0..n-1 (reverse: n-1..0); term_fn(i, x, y, z)
+// writes the components and returns the 0/1 mask.
 template <class TermFn>
 __device__ Sum3 ordered_sum3(int n, bool reverse, bool exact, TermFn term_fn, double sign, SumScratch &sh) {
-    double *cx = sh.cx, *cy = sh.cy, *cz = sh.cz, *rx = sh.rx, *ry = sh.ry, *rz = sh.rz;
-    unsigned char *cm = sh.cm;
+    double *rx = sh.rx, *ry = sh.ry, *rz = sh.rz;
     Sum3 &acc = sh.acc;
-    __syncthreads();  // a previous sum's result may still be being read
     if (exact) {
-        if (threadIdx.x == 0) acc = {0.0, 0.0, 0.0};
-        __syncthreads();
-        const int nb = blockDim.x;
-        for (int c0 = 0; c0 < n; c0 += nb) {
-            const int k = threadIdx.x;
-            const int idx = reverse ? n - 1 - (c0 + k) : c0 + k;
-            double tx = 0, ty = 0, tz = 0;
-            unsigned char m = 0;
-            if (c0 + k < n) m = term_fn(idx, tx, ty, tz);
-            const int cnt = min(nb, n - c0);
-            cx[k] = tx;
-            cy[k] = ty;
-            cz[k] = tz;
-            cm[k] = m;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double ax = acc.x, ay = acc.y, az = acc.z;
-                for (int q = 0; q < cnt; q++) {
-                    if (!cm[q]) continue;
-                    ax = ax + sign * cx[q];
-                    ay = ay + sign * cy[q];
-                    az = az + sign * cz[q];
-                }
-                acc = {ax, ay, az};
-            }
-            __syncthreads();
-        }
-        return acc;
+        blk_serial_sums<3>(n, reverse,
+                           [&](int i, double *t) {
+                               const bool on = term_fn(i, t[0], t[1], t[2]);
+                               for (int d = 0; d < 3; d++) t[d] = sign * t[d];
+                               return on;
+                           },
+                           sh);
+        return {sh.sum[0], sh.sum[1], sh.sum[2]};
     }
+    __syncthreads();  // a previous sum's result may still be being read
     double ax = 0.0, ay = 0.0, az = 0.0;
     for (int q = threadIdx.x; q < n; q += blockDim.x) {
         double tx, ty, tz;
@@ -129,7 +154,8 @@ static __device__ void blk_lindrift_pl(int npl, const double *__restrict__ Gm,
         return lmask[i] != 0;
     };
     const Sum3 s = ordered_sum3(npl, false, exact != 0, term, 1.0, sh);
-    const double ptx = s.x / GMcb, pty = s.y / GMcb, ptz = s.z / GMcb;
+    const Sum3 pt = blk_quotient(s, GMcb, sh);
+    const double ptx = pt.x, pty = pt.y, ptz = pt.z;
     for (int i = threadIdx.x; i < npl; i += blockDim.x) {
         if (!lmask[i]) continue;
         if (exact) {
@@ -158,16 +184,31 @@ static __device__ void blk_vh2vb_pl(int npl, const double *__restrict__ Gm,
         y = z = 0.0;
         return 1;
     };
-    const Sum3 g = ordered_sum3(npl, false, exact != 0, gm, 1.0, sh);
-    const double Gmtot = GMcb + g.x;
     auto term = [&](int i, double &x, double &y, double &z) -> unsigned char {
         x = Gm[i] * vh[3 * i + 0];
         y = Gm[i] * vh[3 * i + 1];
         z = Gm[i] * vh[3 * i + 2];
         return 1;
     };
-    const Sum3 s = ordered_sum3(npl, false, exact != 0, term, -1.0, sh);
-    const double cx = s.x / Gmtot, cy = s.y / Gmtot, cz = s.z / Gmtot;
+    Sum3 g, s;
+    if (exact) {  // the mass and the momentum in one pass
+        blk_serial_sums<4>(npl, false,
+                           [&](int i, double *t) {
+                               term(i, t[0], t[1], t[2]);
+                               for (int d = 0; d < 3; d++) t[d] = -t[d];
+                               t[3] = Gm[i];
+                               return true;
+                           },
+                           sh);
+        s = {sh.sum[0], sh.sum[1], sh.sum[2]};
+        g.x = sh.sum[3];
+    } else {
+        g = ordered_sum3(npl, false, false, gm, 1.0, sh);
+        s = ordered_sum3(npl, false, false, term, -1.0, sh);
+    }
+    const double Gmtot = GMcb + g.x;
+    const Sum3 c = blk_quotient(s, Gmtot, sh);
+    const double cx = c.x, cy = c.y, cz = c.z;
     if (threadIdx.x == 0) {
         dcb[CB_VB + 0] = cx;
         dcb[CB_VB + 1] = cy;
