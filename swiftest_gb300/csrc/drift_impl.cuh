@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fp64_exact.cuh"
 #include "swg_internal.cuh"
 
 namespace swg {
@@ -14,14 +15,20 @@ __device__ constexpr double DANBYB = 1.0e-13;
 constexpr int NLAG1 = 50;
 constexpr int NLAG2 = 40;
 
+// |x| < 4 from the exponent alone (NaN: no)
+__device__ __forceinline__ bool less_than_4(double x) { return (__double2hiint(x) & 0x7fffffff) < 0x40100000; }
+
 __device__ __forceinline__ void d_scget(double angle, double &sx, double &cx) {
-    const int nper = (int)(angle / TWOPI);
+    const int nper = (int)xdiv(angle, TWOPI);
     double x = angle - nper * TWOPI;
     if (x < 0.0) x = x + TWOPI;
     sx = sin(x);
-    cx = sqrt(1.0 - sx * sx);
+    cx = xsqrt(1.0 - sx * sx);
     if ((x > PIBY2) && (x < PI3BY2)) cx = -cx;
 }
+
+static __constant__ double STUMPFF_Q2[6] = {182.0, 132.0, 90.0, 56.0, 30.0, 12.0};
+static __constant__ double STUMPFF_Q3[6] = {210.0, 156.0, 110.0, 72.0, 42.0, 20.0};
 
 __device__ __forceinline__ void d_stumpff(double x, double &c0, double &c1, double &c2, double &c3) {
     int n = 0;
@@ -29,12 +36,15 @@ __device__ __forceinline__ void d_stumpff(double x, double &c0, double &c1, doub
         n = n + 1;
         x = x / 4.0;
     }
-    c2 = (1.0 - x * (1.0 - x * (1.0 - x * (1.0 - x * (1.0 - x * (1.0 - x / 182.0) / 132.0) / 90.0) / 56.0) / 30.0) /
-                    12.0) /
-         2.0;
-    c3 = (1.0 - x * (1.0 - x * (1.0 - x * (1.0 - x * (1.0 - x * (1.0 - x / 210.0) / 156.0) / 110.0) / 72.0) / 42.0) /
-                    20.0) /
-         6.0;
+    // nested as c = 1 - x c / q for the divisors q, innermost first
+    c2 = c3 = 1.0;
+#pragma unroll 1
+    for (int k = 0; k < 6; k++) {
+        c2 = 1.0 - xdiv(x * c2, STUMPFF_Q2[k]);
+        c3 = 1.0 - xdiv(x * c3, STUMPFF_Q3[k]);
+    }
+    c2 = c2 / 2.0;
+    c3 = xdiv(c3, 6.0);
     c1 = 1.0 - x * c3;
     c0 = 1.0 - x * c2;
     for (int i = n; i >= 1; i--) {
@@ -45,26 +55,28 @@ __device__ __forceinline__ void d_stumpff(double x, double &c0, double &c1, doub
     }
 }
 
-__device__ inline void d_kepmd(double dm, double es, double ec, double &x, double &s, double &c) {
-    const double a0 = 39916800.0, a1 = 6652800.0, a2 = 332640.0, a3 = 7920.0, a4 = 110.0;
-    const double fac1 = 1.0 / (1.0 - ec);
-    const double q = fac1 * dm;
-    const double fac2 = es * es * fac1 - ec / 3.0;
-    double xx = q * (1.0 - 0.5 * fac1 * q * (es - q * fac2));
-    double y = xx * xx;
-    double ss = xx * (a0 - y * (a1 - y * (a2 - y * (a3 - y * (a4 - y))))) / a0;
-    double cc = sqrt(1.0 - ss * ss);
-    const double f = xx - ec * ss + es * (1.0 - cc) - dm;
-    const double fp = 1.0 - ec * cc + es * ss;
-    const double fpp = ec * ss + es * cc;
-    const double fppp = ec * cc - es * ss;
-    double dx = -(f / fp);
-    dx = -(f / (fp + dx * fpp / 2.0));
-    dx = -(f / (fp + dx * fpp / 2.0 + dx * dx * fppp * SIXTH));
+template <class xd>
+__device__ inline void d_kepmd(xd dm, xd es, xd ec, xd &x, xd &s, xd &c) {
+    const xd a0 = 39916800.0, a1 = 6652800.0, a2 = 332640.0, a3 = 7920.0, a4 = 110.0, one = 1.0;
+    const xd fac1 = one / (one - ec);
+    const xd q = fac1 * dm;
+    const xd fac2 = es * es * fac1 - ec / 3.0;
+    xd xx = q * (one - xd(x_half(fac1.v)) * q * (es - q * fac2));
+    xd y = xx * xx;
+    xd ss = xx * (a0 - y * (a1 - y * (a2 - y * (a3 - y * (a4 - y))))) / a0;
+    xd cc = xsqrt((one - ss * ss).v);
+    const xd ecs = ec * ss, ecc = ec * cc, ess = es * ss, esc = es * cc;
+    const xd f = xx - ecs + es * (one - cc) - dm;
+    const xd fp = one - ecc + ess;
+    const xd fpp = ecs + esc;
+    const xd fppp = ecc - ess;
+    xd dx = -(f / fp);
+    dx = -(f / (fp + xd(x_half((dx * fpp).v))));
+    dx = -(f / (fp + xd(x_half((dx * fpp).v)) + dx * dx * fppp * SIXTH));
     xx = xx + dx;
     y = xx * xx;
     ss = xx * (a0 - y * (a1 - y * (a2 - y * (a3 - y * (a4 - y))))) / a0;
-    cc = sqrt(1.0 - ss * ss);
+    cc = xsqrt((one - ss * ss).v);
     x = xx;
     s = ss;
     c = cc;
@@ -100,20 +112,21 @@ __device__ inline void d_p3solve(double dt, double r0, double mu, double alpha, 
 __device__ inline void d_kepu_guess(double dt, double r0, double mu, double alpha, double u, double &s) {
     const double thresh = 0.4, danbyk = 0.85;
     if (alpha > 0.0) {
-        if (dt / r0 <= thresh) {
-            s = dt / r0 - (dt * dt * u) / (2.0 * r0 * r0 * r0);
+        const double dr = xdiv(dt, r0);
+        if (dr <= thresh) {
+            s = dr - xdiv(dt * dt * u, 2.0 * r0 * r0 * r0);
         } else {
-            const double a = mu / alpha;
-            const double en = sqrt(mu / (a * a * a));
-            const double ec = 1.0 - r0 / a;
-            const double es = u / (en * a * a);
-            const double e = sqrt(ec * ec + es * es);
+            const double a = xdiv(mu, alpha);
+            const double en = xsqrt(xdiv(mu, a * a * a));
+            const double ec = 1.0 - xdiv(r0, a);
+            const double es = xdiv(u, en * a * a);
+            const double e = xsqrt(ec * ec + es * es);
             const double y = en * dt - es;
             double sy, cy;
             d_scget(y, sy, cy);
             const double sigma = copysign(1.0, es * cy + ec * sy);
             const double x = y + sigma * danbyk * e;
-            s = x / sqrt(alpha);
+            s = xdiv(x, xsqrt(alpha));
         }
     } else {
         int iflag;
@@ -145,11 +158,11 @@ __device__ inline void d_kepu_new(double &s, double dt, double r0, double mu, do
         fp = r0 * c0 + u * c1 + mu * c2;
         const double fpp = (-(r0 * alpha) + mu) * c1 + u * c0;
         const double fppp = (-(r0 * alpha) + mu) * c0 - u * alpha * c1;
-        double ds = -(f / fp);
-        ds = -(f / (fp + ds * fpp / 2.0));
-        ds = -(f / (fp + ds * fpp / 2.0 + ds * ds * fppp / 6.0));
+        double ds = -xdiv(f, fp);
+        ds = -xdiv(f, fp + ds * fpp / 2.0);
+        ds = -xdiv(f, fp + ds * fpp / 2.0 + xdiv(ds * ds * fppp, 6.0));
         s = s + ds;
-        const double fdt = f / dt;
+        const double fdt = xdiv(f, dt);
         if (fdt * fdt < DANBYB * DANBYB) {
             iflag = 0;
             return;
@@ -174,9 +187,9 @@ __device__ inline void d_kepu_lag(double &s, double dt, double r0, double mu, do
         const double fpp = (-(r0 * alpha) + mu) * c1 + u * c0;
         const double lnm1 = (double)ln - 1.0;
         const double disc = fabs(lnm1 * lnm1 * fp * fp - lnm1 * (double)ln * f * fpp);
-        const double ds = -((double)ln * f / (fp + copysign(1.0, fp) * sqrt(disc)));
+        const double ds = -xdiv((double)ln * f, fp + copysign(1.0, fp) * xsqrt(disc));
         s = s + ds;
-        const double fdt = f / dt;
+        const double fdt = xdiv(f, dt);
         if (fdt * fdt < DANBYB * DANBYB) {
             iflag = 0;
             return;
@@ -200,59 +213,17 @@ __device__ inline void d_kepu(double dt, double r0, double mu, double alpha, dou
     }
 }
 
-__device__ inline void d_drift_dan(double mu, double &rx0, double &ry0, double &rz0, double &vx0, double &vy0, double &vz0,
-                            double dt0, int &iflag) {
-    double dt = dt0;
-    iflag = 0;
-    const double r0 = sqrt(rx0 * rx0 + ry0 * ry0 + rz0 * rz0);
-    const double v0s = vx0 * vx0 + vy0 * vy0 + vz0 * vz0;
-    const double u = rx0 * vx0 + ry0 * vy0 + rz0 * vz0;
-    const double alpha = 2.0 * mu / r0 - v0s;
-    if (alpha > 0.0) {
-        const double a = mu / alpha;
-        const double asq = a * a;
-        const double en = sqrt(mu / (a * asq));
-        const double ec = 1.0 - r0 / a;
-        const double es = u / (en * asq);
-        const double esq = ec * ec + es * es;
-        const double dm = dt * en - (double)(int)(dt * en / TWOPI) * TWOPI;
-        dt = dm / en;
-        if ((esq < E2MAX) && (dm * dm < DM2MAX) && (esq * (dm * dm) < E2DM2MAX)) {
-            double xkep, s, c;
-            d_kepmd(dm, es, ec, xkep, s, c);
-            const double fchk = (xkep - ec * s + es * (1.0 - c) - dm);
-            if (fchk * fchk > DANBYB * DANBYB) {
-                iflag = 1;
-                return;
-            }
-            const double fp = 1.0 - ec * c + es * s;
-            const double f = a / r0 * (c - 1.0) + 1.0;
-            const double g = dt + (s - xkep) / en;
-            const double fdot = -(a / (r0 * fp) * en * s);
-            const double gdot = (c - 1.0) / fp + 1.0;
-            const double rx = rx0 * f + vx0 * g;
-            const double ry = ry0 * f + vy0 * g;
-            const double rz = rz0 * f + vz0 * g;
-            const double vx = rx0 * fdot + vx0 * gdot;
-            const double vy = ry0 * fdot + vy0 * gdot;
-            const double vz = rz0 * fdot + vz0 * gdot;
-            rx0 = rx;
-            ry0 = ry;
-            rz0 = rz;
-            vx0 = vx;
-            vy0 = vy;
-            vz0 = vz;
-            iflag = 0;
-            return;
-        }
-    }
+// The universal-variable branch of drift_dan.  Out of line: it is the rare branch of a step, and
+// inlined it doubles the code and sets the registers of the kernels.
+static __device__ __noinline__ void d_drift_kepu(double mu, double &rx0, double &ry0, double &rz0, double &vx0, double &vy0,
+                                          double &vz0, double dt, double r0, double alpha, double u, int &iflag) {
     double fp, c1, c2, c3;
     d_kepu(dt, r0, mu, alpha, u, fp, c1, c2, c3, iflag);
     if (iflag == 0) {
-        const double f = 1.0 - mu / r0 * c2;
+        const double f = 1.0 - xdiv(mu, r0) * c2;
         const double g = dt - mu * c3;
-        const double fdot = -(mu / (fp * r0) * c1);
-        const double gdot = 1.0 - mu / fp * c2;
+        const double fdot = -(xdiv(mu, fp * r0) * c1);
+        const double gdot = 1.0 - xdiv(mu, fp) * c2;
         const double rx = rx0 * f + vx0 * g;
         const double ry = ry0 * f + vy0 * g;
         const double rz = rz0 * f + vz0 * g;
@@ -268,14 +239,67 @@ __device__ inline void d_drift_dan(double mu, double &rx0, double &ry0, double &
     }
 }
 
+template <class XK, class xd>
+__device__ inline void d_drift_dan(double mu, double &rx0, double &ry0, double &rz0, double &vx0, double &vy0, double &vz0,
+                            double dt0, int &iflag) {
+    double dt = dt0;
+    iflag = 0;
+    const xd X = rx0, Y = ry0, Z = rz0, U = vx0, V = vy0, W = vz0, one = 1.0;
+    const double r0 = xsqrt((X * X + Y * Y + Z * Z).v);
+    const xd v0s = U * U + V * V + W * W;
+    const double u = (X * U + Y * V + Z * W).v;
+    const double alpha = (xd(2.0 * mu) / r0 - v0s).v;
+    if (x_greater(alpha, 0.0)) {
+        const xd a = xdiv(mu, alpha);
+        const xd asq = a * a;
+        const xd en = xsqrt((xd(mu) / (a * asq)).v);
+        const xd ec = one - xd(r0) / a;
+        const xd es = xd(u) / (en * asq);
+        const xd esq = ec * ec + es * es;
+        const xd den = xd(dt) * en;
+        // dt en - int(dt en / 2 pi) 2 pi, whose integer is zero below 4
+        const xd dm = less_than_4(den.v) ? den.v : den.v - (double)(int)xdiv(den.v, TWOPI) * TWOPI;
+        const xd dm2 = dm * dm;
+        dt = (dm / en).v;
+        if (x_less(esq.v, E2MAX) && x_less(dm2.v, DM2MAX) && x_less((esq * dm2).v, E2DM2MAX)) {
+            XK kx, ks, kc;
+            d_kepmd<XK>(dm.v, es.v, ec.v, kx, ks, kc);
+            const xd xkep = kx.v, s = ks.v, c = kc.v;
+            const xd fchk = (xkep - ec * s + es * (one - c) - dm);
+            if (x_greater(x_abs(fchk.v), DANBYB)) {  // fchk^2 > DANBYB^2, the same decision
+                iflag = 1;
+                return;
+            }
+            const xd fp = one - ec * c + es * s;
+            const xd c1 = c - one;
+            const xd f = a / r0 * c1 + one;
+            const xd g = xd(dt) + (s - xkep) / en;
+            const xd fdot = -(a / (xd(r0) * fp) * en * s);
+            const xd gdot = c1 / fp + one;
+            rx0 = (X * f + U * g).v;
+            ry0 = (Y * f + V * g).v;
+            rz0 = (Z * f + W * g).v;
+            vx0 = (X * fdot + U * gdot).v;
+            vy0 = (Y * fdot + V * gdot).v;
+            vz0 = (Z * fdot + W * gdot).v;
+            iflag = 0;
+            return;
+        }
+    }
+    d_drift_kepu(mu, rx0, ry0, rz0, vx0, vy0, vz0, dt, r0, alpha, u, iflag);
+}
+
+// WIDE: the form for kernels that fill the GPU (products of the Kepler solver by integer
+// instructions: of about 130 FP64 instructions 30 fewer); the same bits.
+template <bool WIDE = false>
 __device__ inline int d_drift_one(double mu, double &rx, double &ry, double &rz, double &vx, double &vy, double &vz,
                            double dt) {
     int iflag;
-    d_drift_dan(mu, rx, ry, rz, vx, vy, vz, dt, iflag);
+    d_drift_dan<xd<WIDE>, xd<false>>(mu, rx, ry, rz, vx, vy, vz, dt, iflag);
     if (iflag != 0) {
         const double dttmp = 0.1 * dt;
         for (int i = 1; i <= 10; i++) {
-            d_drift_dan(mu, rx, ry, rz, vx, vy, vz, dttmp, iflag);
+            d_drift_dan<xd<false>, xd<false>>(mu, rx, ry, rz, vx, vy, vz, dttmp, iflag);
             if (iflag != 0) break;
         }
     }
@@ -301,11 +325,22 @@ __device__ inline int d_drift_one(double mu, double &rx, double &ry, double &rz,
 // below FP64 resolution.  sin and cos are formed once in FP64 at the FP32 root (the
 // reference's degree-11 sine polynomial, cos from sqrt(1 - sin^2)) and carried to the
 // polished root by their Taylor expansion to second order in dx.
-__device__ inline void d_kepmd_fast(double dm, double es, double ec, double &x, double &s, double &c) {
+//
+// WIDE: the form for kernels that fill the GPU, which the FP64 pipe bounds: products
+// (other than those of a fused multiply-add) and square roots by integer instructions, as in
+// xd<true> (547,900 bodies: 145 -> 69 us).  Otherwise (the recursion, which waits for each
+// result) the shortest chains.
+template <bool WIDE>
+__device__ __forceinline__ double d_mul(double a, double b) {
+    return WIDE ? xmul(a, b) : a * b;
+}
+
+template <bool WIDE>
+__device__ inline void d_kepmd_fast(double dm, double es, double ec, float dmf, float esf, float ecf, double &x,
+                                    double &s, double &c) {
     const double a0 = 39916800.0, a1 = 6652800.0, a2 = 332640.0, a3 = 7920.0, a4 = 110.0;
     const double inv_a0 = 1.0 / 39916800.0;
     // FP32 root: sin x as its Taylor series to x^11 in nested form
-    const float dmf = (float)dm, esf = (float)es, ecf = (float)ec;
     const float fac1 = 1.0f / (1.0f - ecf);
     const float q = fac1 * dmf;
     const float fac2 = fmaf(esf * esf, fac1, -ecf * (1.0f / 3.0f));
@@ -329,59 +364,73 @@ __device__ inline void d_kepmd_fast(double dm, double es, double ec, double &x, 
         xf += dx;
     }
     // FP64 Halley step at the FP32 root
-    const double xx = (double)xf;
-    const double y = xx * xx;
-    const double ss = xx * fma(-y, fma(-y, fma(-y, fma(-y, a4 - y, a3), a2), a1), a0) * inv_a0;
-    const double cc = sqrt(fma(-ss, ss, 1.0));
-    const double f = fma(es, 1.0 - cc, fma(-ec, ss, xx)) - dm;
+    const double xx = x_to_double(xf);
+    const double y = d_mul<WIDE>(xx, xx);
+    const double ss =
+        d_mul<WIDE>(d_mul<WIDE>(xx, fma(-y, fma(-y, fma(-y, fma(-y, xsub(a4, y), a3), a2), a1), a0)), inv_a0);
+    const double cc = xsqrt(fma(-ss, ss, 1.0));
+    const double f = xsub(fma(es, xsub(1.0, cc), fma(-ec, ss, xx)), dm);
     const double fp = fma(es, ss, fma(-ec, cc, 1.0));
-    const double fpp = fma(ec, ss, es * cc);
-    const double dx = -(2.0 * f * fp) / fma(2.0 * fp, fp, -f * fpp);
-    x = xx + dx;
-    s = fma(dx, fma(-0.5 * ss, dx, cc), ss);  // sin(x + dx) = s + c dx - s dx^2 / 2
-    c = fma(dx, fma(-0.5 * cc, dx, -ss), cc);  // cos(x + dx) = c - s dx - c dx^2 / 2
+    const double fpp = fma(ec, ss, d_mul<WIDE>(es, cc));
+    const double dx = xdiv(-d_mul<WIDE>(f, fp), fma(fp, fp, -d_mul<WIDE>(x_half(f), fpp)));
+    x = xadd(xx, dx);
+    s = fma(dx, fma(-x_half(ss), dx, cc), ss);  // sin(x + dx) = s + c dx - s dx^2 / 2
+    c = fma(dx, fma(-x_half(cc), dx, -ss), cc);  // cos(x + dx) = c - s dx - c dx^2 / 2
 }
 
 // inv_mu: 1/mu when the caller has it (the same value, formed once), else 0
+template <bool WIDE>
 __device__ inline void d_drift_dan_fast(double mu, double &rx0, double &ry0, double &rz0, double &vx0, double &vy0,
                                         double &vz0, double dt0, int &iflag, double inv_mu0 = 0.0) {
     iflag = 0;
-    const double r2 = fma(rz0, rz0, fma(ry0, ry0, rx0 * rx0));
-    const double inv_r0 = rsqrt(r2);
-    const double v0s = fma(vz0, vz0, fma(vy0, vy0, vx0 * vx0));
-    const double u = fma(rz0, vz0, fma(ry0, vy0, rx0 * vx0));
+    const double r2 = fma(rz0, rz0, fma(ry0, ry0, d_mul<WIDE>(rx0, rx0)));
+    double r0, inv_r0;
+    if (WIDE) {
+        r0 = xsqrt(r2);
+        inv_r0 = xdiv(1.0, r0);
+    } else {
+        inv_r0 = x_rsqrt(r2);
+        r0 = r2 * inv_r0;
+    }
+    const double v0s = fma(vz0, vz0, fma(vy0, vy0, d_mul<WIDE>(vx0, vx0)));
+    const double u = fma(rz0, vz0, fma(ry0, vy0, d_mul<WIDE>(rx0, vx0)));
     const double alpha = fma(2.0 * mu, inv_r0, -v0s);
-    if (alpha > 0.0) {
-        const double inv_mu = inv_mu0 != 0.0 ? inv_mu0 : 1.0 / mu;
-        const double rsa = rsqrt(alpha);
-        const double a = mu * rsa * rsa;                 // mu / alpha
-        const double ia = alpha * inv_mu;                // 1 / a
-        const double en = alpha * (alpha * rsa) * inv_mu;  // sqrt(mu / a^3)
-        const double inv_en = mu * (rsa * rsa * rsa);
-        const double ec = fma(-(r2 * inv_r0), ia, 1.0);
-        const double es = u * inv_en * ia * ia;
-        const double esq = fma(ec, ec, es * es);
-        const double den = dt0 * en;
-        const double dm = fma(-(double)(int)(den * (1.0 / TWOPI)), TWOPI, den);
-        if ((esq < E2MAX) && (dm * dm < DM2MAX) && (esq * (dm * dm) < E2DM2MAX)) {
-            const double dt = dm * inv_en;
+    if (x_greater(alpha, 0.0)) {
+        const double inv_mu = inv_mu0 != 0.0 ? inv_mu0 : xdiv(1.0, mu);
+        const double rsa = WIDE ? xdiv(1.0, xsqrt(alpha)) : x_rsqrt(alpha);
+        const double rsa2 = d_mul<WIDE>(rsa, rsa);
+        const double a = d_mul<WIDE>(mu, rsa2);                   // mu / alpha
+        const double ia = d_mul<WIDE>(alpha, inv_mu);             // 1 / a
+        const double en = d_mul<WIDE>(d_mul<WIDE>(alpha, rsa), ia);  // sqrt(mu / a^3)
+        const double inv_en = d_mul<WIDE>(a, rsa);
+        const double ec = fma(-r0, ia, 1.0);
+        const double es = d_mul<WIDE>(d_mul<WIDE>(u, rsa), ia);   // u / (en a^2)
+        const double den = d_mul<WIDE>(dt0, en);
+        const double dm = less_than_4(den) ? den : fma(-(double)(int)(den * (1.0 / TWOPI)), TWOPI, den);
+        // the branch limits in FP32: either side of them both branches are valid
+        const float dmf = x_to_float(dm), esf = x_to_float(es), ecf = x_to_float(ec);
+        const float esq = fmaf(ecf, ecf, esf * esf), dm2 = dmf * dmf;
+        if (esq < (float)E2MAX && dm2 < (float)DM2MAX && esq * dm2 < (float)E2DM2MAX) {
+            const double dt = d_mul<WIDE>(dm, inv_en);
             double xkep, s, c;
-            d_kepmd_fast(dm, es, ec, xkep, s, c);
-            const double fchk = fma(es, 1.0 - c, fma(-ec, s, xkep)) - dm;
-            if (fchk * fchk > DANBYB * DANBYB) {
+            d_kepmd_fast<WIDE>(dm, es, ec, dmf, esf, ecf, xkep, s, c);
+            const double c1 = xsub(c, 1.0);
+            const double fchk = xsub(fma(-es, c1, fma(-ec, s, xkep)), dm);
+            if (x_greater(x_abs(fchk), DANBYB)) {
                 iflag = 1;
                 return;
             }
             const double fp = fma(es, s, fma(-ec, c, 1.0));
-            const double inv_fp = 1.0 / fp;
-            const double ar = a * inv_r0;
-            const double f = fma(ar, c - 1.0, 1.0);
-            const double g = fma(s - xkep, inv_en, dt);
-            const double fdot = -(ar * inv_fp * en * s);
-            const double gdot = fma(c - 1.0, inv_fp, 1.0);
-            const double rx = fma(rx0, f, vx0 * g), ry = fma(ry0, f, vy0 * g), rz = fma(rz0, f, vz0 * g);
-            const double vx = fma(rx0, fdot, vx0 * gdot), vy = fma(ry0, fdot, vy0 * gdot),
-                         vz = fma(rz0, fdot, vz0 * gdot);
+            const double inv_fp = xdiv(1.0, fp);
+            const double ar = d_mul<WIDE>(a, inv_r0);
+            const double f = fma(ar, c1, 1.0);
+            const double g = fma(xsub(s, xkep), inv_en, dt);
+            const double fdot = d_mul<WIDE>(-d_mul<WIDE>(d_mul<WIDE>(ar, en), s), inv_fp);
+            const double gdot = fma(c1, inv_fp, 1.0);
+            const double rx = fma(rx0, f, d_mul<WIDE>(vx0, g)), ry = fma(ry0, f, d_mul<WIDE>(vy0, g)),
+                         rz = fma(rz0, f, d_mul<WIDE>(vz0, g));
+            const double vx = fma(rx0, fdot, d_mul<WIDE>(vx0, gdot)), vy = fma(ry0, fdot, d_mul<WIDE>(vy0, gdot)),
+                         vz = fma(rz0, fdot, d_mul<WIDE>(vz0, gdot));
             rx0 = rx;
             ry0 = ry;
             rz0 = rz;
@@ -391,17 +440,18 @@ __device__ inline void d_drift_dan_fast(double mu, double &rx0, double &ry0, dou
             return;
         }
     }
-    d_drift_dan(mu, rx0, ry0, rz0, vx0, vy0, vz0, dt0, iflag);  // universal variables: the reference form
+    d_drift_dan<xd<false>, xd<false>>(mu, rx0, ry0, rz0, vx0, vy0, vz0, dt0, iflag);  // universal variables: the reference form
 }
 
+template <bool WIDE = false>
 __device__ inline int d_drift_one_fast(double mu, double &rx, double &ry, double &rz, double &vx, double &vy,
                                        double &vz, double dt, double inv_mu = 0.0) {
     int iflag;
-    d_drift_dan_fast(mu, rx, ry, rz, vx, vy, vz, dt, iflag, inv_mu);
+    d_drift_dan_fast<WIDE>(mu, rx, ry, rz, vx, vy, vz, dt, iflag, inv_mu);
     if (iflag != 0) {
         const double dttmp = 0.1 * dt;
         for (int i = 1; i <= 10; i++) {
-            d_drift_dan_fast(mu, rx, ry, rz, vx, vy, vz, dttmp, iflag, inv_mu);
+            d_drift_dan_fast<false>(mu, rx, ry, rz, vx, vy, vz, dttmp, iflag, inv_mu);
             if (iflag != 0) break;
         }
     }

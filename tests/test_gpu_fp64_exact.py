@@ -7,6 +7,7 @@ import pytest
 from oracle import oracle as O
 from swiftest_gb300 import SWG_FP64
 from swiftest_gb300 import initial_conditions as IC
+from swiftest_gb300.api import NBodySystem
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,34 @@ def test_kick_tp_bits(ctx, kind, ntp, npl):
     acc = np.random.default_rng(1).normal(size=(ntp, 3)) * 1e-3
     a = ctx.kick_getacch_int_all_tp(r[npl:], r[:npl], g[:npl], lmask=m, acc=acc, precision=SWG_FP64)
     assert np.array_equal(_bits(a), _bits(O.kick_tp(r[npl:], r[:npl], g[:npl], lmask=m, acc=acc)))
+
+
+@pytest.mark.parametrize("n", [39999, 40001])  # both forms of the drift kernels' dispatch
+@pytest.mark.parametrize("dt", [0.003, 0.08])
+def test_drift_forms(ctx, n, dt):
+    rng = np.random.default_rng(n)
+    a, e = rng.uniform(0.4, 5.0, n), rng.uniform(0.0, 0.5, n)
+    inc = np.where(np.arange(n) % 5 == 0, 0.0, 0.01)  # zero z components among them
+    r, v = IC.el2xv(IC.GMCB, a, e, inc, *rng.uniform(0, 2 * np.pi, (3, n)))
+    x, w, f = ctx.drift_all(IC.GMCB, r, v, dt)
+    ox, ow, of = O.drift_all(IC.GMCB, r, v, dt)
+    assert np.array_equal(f, of)
+    small = IC.GMCB / a ** 3 * dt * dt < 0.1  # the branch without CUDA's math functions: same bits
+    assert np.array_equal(_bits(x[small]), _bits(ox[small])) and np.array_equal(_bits(w[small]), _bits(ow[small]))
+    assert np.abs(x - ox).max() < 1e-9 and np.abs(w - ow).max() < 1e-8
+    # the mixed path's form, through a step whose one massive body pulls by 1e-13 of the
+    # central body: a few units in the last place over kick and drift
+    cb, pl, _ = IC.make_system(seed=1, npl=1, ntp=0, mmin=1e-13, mmax=1.1e-13)
+    got = []
+    for prec in ("FP64", "MIXED"):
+        s = NBodySystem(ctx, "HELIO", cb, pl, {"rh": r, "vh": v}, dt=dt, lclose=False, precision=prec)
+        s.step(1)
+        got.append(s.get_tp())
+        s.close()
+    (xr, vr, sr), (xm, vm, sm) = got
+    assert np.array_equal(sr, sm)
+    scale = np.linalg.norm(xr, axis=1, keepdims=True), np.linalg.norm(vr, axis=1, keepdims=True)
+    # 64 units in the last place: a velocity of 2 pi a^-1/2 moves the body by up to 0.4 (3 for
+    # the large steps) of its radius, so errors of a few units in mean motion stay below
+    assert (np.abs(xm - xr) / scale[0]).max() < 64 * 2.0 ** -52
+    assert (np.abs(vm - vr) / scale[1]).max() < 64 * 2.0 ** -52
