@@ -165,7 +165,7 @@ __device__ __forceinline__ double x_div(const XNum &g, double p, bool &bad) {
 // double cut to its leading 24 bits, and a normal (or zero) float as a double.
 __device__ __forceinline__ float x_to_float(double x) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
-    if (!x_ok(hi & 0x7fffffff)) return (float)x;
+    if (!x_ok(hi & 0x7fffffff)) return ((hi & 0x7fffffff) | lo) == 0 ? 0.0f : (float)x;
     return __int_as_float((__funnelshift_l(lo, hi - ((1023 - 127) << 20), 3) & 0x7fffffff) | (hi & 0x80000000));
 }
 __device__ __forceinline__ double x_to_double(float f) {

@@ -377,9 +377,9 @@ __device__ __forceinline__ void d_enc_one(double xr, double yr, double zr, doubl
             if (v2 <= VSMALL) {
                 r2min = r2;
             } else {
-                const double tmin = -vdotr / v2;
+                const double tmin = xdiv(-vdotr, v2);
                 if (tmin < dt)
-                    r2min = r2 - vdotr * vdotr / v2;
+                    r2min = r2 - xdiv(vdotr * vdotr, v2);
                 else
                     r2min = r2 + 2.0 * vdotr * dt + v2 * (dt * dt);
             }
@@ -409,7 +409,7 @@ __device__ __forceinline__ void d_enc_one_fast(double xr, double yr, double zr, 
             if (v2 <= VSMALL) {
                 r2min = r2;
             } else {
-                const double iv2 = 1.0 / v2;
+                const double iv2 = xdiv(1.0, v2);
                 const double tmin = -vdotr * iv2;
                 if (tmin < dt)
                     r2min = fma(-(vdotr * vdotr), iv2, r2);
@@ -428,16 +428,14 @@ __device__ __forceinline__ void d_enc_one_fast(double xr, double yr, double zr, 
 // x**(-1.5) of the shell kick (symba_kick.f90:204,307): sqrt(x) and x*sqrt(x) as
 // double-double pairs (Dekker's error-free transformations with fma residuals),
 // then one Newton step on the reciprocal.  Within half an ulp except in rare
-// near-tie cases, and the same bits as the host evaluation of the same sequence.
-__device__ __forceinline__ double pow_m1p5(double x) {
+// near-tie cases, and the same bits as the host evaluation of the same sequence.  s, p, y0: the
+// rounded sqrt(x), x * s and 1 / p, which the kick has already formed.
+__device__ __forceinline__ double pow_m1p5(double x, double s, double p, double y0) {
     if (!(x > 0.0) || isinf(x)) return pow(x, -1.5);
-    const double s = sqrt(x);
     const double rs = fma(-s, s, x);
-    const double ds = rs / (2.0 * s);
-    const double p = x * s;
+    const double ds = xdiv(rs, 2.0 * s);
     const double ep = fma(x, s, -p);
     const double ql = ep + x * ds;
-    const double y0 = 1.0 / p;
     const double err = fma(-y0, p, 1.0) - y0 * ql;
     return fma(y0, err, y0);
 }
@@ -450,7 +448,7 @@ __device__ __forceinline__ double d_powi(double x, int m) {
         x = x * x;
         if (n % 2) y = y * x;
     }
-    return m < 0 ? 1.0 / y : y;
+    return m < 0 ? xdiv(1.0, y) : y;
 }
 
 // Encounter lists live in one int32 allocation per kind: [i1 | i2 | lvdotr | status | level],
@@ -480,6 +478,150 @@ struct RecArgs {
 // [2, 2 + MAXLEV) loop counters, [2 + MAXLEV, 2 + 2 MAXLEV) phases.
 constexpr int MAXLEV = 48;
 constexpr int REC_STATE = 2 + 2 * MAXLEV;
+
+// One pair's list check (symba_encounter_check_list_plpl / _pltp, symba_encounter_check.f90:90-235):
+// encounter_check_one at the summed encounter radii, and not overlapping already.  Most pairs
+// are far from every threshold: FP32 on the FP64 differences (cut to 24 bits, so each term is
+// within 2e-7 and the sums within 1e-6 of their magnitudes) decides with margins of 1e-5 to 4e-5,
+// and the rest take the FP64 test; the decisions are the FP64 test's.  rhs1, rhs2: rhill * rhscale of
+// the two bodies (rhs2 zero for a test particle), rsp: RSHELL^irec, rad: the sum of the radii.
+__device__ __forceinline__ bool d_list_pair(bool fast, bool isp, const double *xr, const double *vr, double rhs1,
+                                            double rhs2, double rsp, double rad1, double rad2, double dt, int &lvd) {
+    const float x = x_to_float(xr[0]), y = x_to_float(xr[1]), z = x_to_float(xr[2]);
+    const float u = x_to_float(vr[0]), v = x_to_float(vr[1]), w = x_to_float(vr[2]);
+    const float rc = (x_to_float(rhs1) + x_to_float(rhs2)) * x_to_float(rsp), c2 = rc * rc;
+    const float ra = x_to_float(rad1) + x_to_float(rad2), dtf = x_to_float(dt);
+    const float r2 = fmaf(z, z, fmaf(y, y, x * x)), v2 = fmaf(w, w, fmaf(v, v, u * u));
+    const float vd = fmaf(z, w, fmaf(y, v, x * u));
+    const float avd = 1e-5f * fmaf(fabsf(z), fabsf(w), fmaf(fabsf(y), fabsf(v), fabsf(x) * fabsf(u)));
+    if (r2 > 1e-30f && v2 > 1e-30f && c2 > 1e-30f && r2 < 1e30f && v2 < 1e30f && c2 < 1e30f) {
+        int le = -1;  // not decided
+        if (r2 > c2 * 1.00001f) {
+            if (vd > avd) {
+                lvd = 0;
+                return false;
+            }
+            if (vd < -avd) {
+                const float tmin = -vd / v2;
+                const float r2min = tmin < dtf ? fmaf(vd, tmin, r2) : fmaf(dtf, fmaf(v2, dtf, 2.0f * vd), r2);
+                if (r2min > fmaf(4e-5f, r2, c2)) {
+                    lvd = 1;
+                    return false;
+                }
+                if (r2min < fmaf(-4e-5f, r2, c2)) le = 1;
+            }
+        } else if (r2 < c2 * 0.99999f) {
+            le = 1;
+        }
+        if (le == 1 && r2 > ra * ra * 1.00001f) {
+            lvd = 1;
+            return true;
+        }
+    }
+    const double renci = rhs1 * rsp;  // d_renc(rhill_i, rhscale, irec)
+    const double rcrit = isp ? renci + rhs2 * rsp : renci;
+    int le;
+    if (fast)
+        d_enc_one_fast(xr[0], xr[1], xr[2], vr[0], vr[1], vr[2], rcrit, dt, le, lvd);
+    else
+        d_enc_one(xr[0], xr[1], xr[2], vr[0], vr[1], vr[2], rcrit, dt, le, lvd);
+    if (!le) return false;
+    const double rs = isp ? rad1 + rad2 : rad1;
+    return xr[0] * xr[0] + xr[1] * xr[1] + xr[2] * xr[2] > rs * rs;
+}
+
+// A pair that certainly does not collide in collision_check_one: not overlapping, and not
+// receding after an approach, or receding too slowly for the step (FP32 with the margins of
+// d_list_pair; false where it cannot tell).
+__device__ __forceinline__ bool d_collision_far(double xr, double yr, double zr, double vxr, double vyr, double vzr,
+                                                double rlim, double dt, bool lvdotr) {
+    const float x = x_to_float(xr), y = x_to_float(yr), z = x_to_float(zr);
+    const float u = x_to_float(vxr), v = x_to_float(vyr), w = x_to_float(vzr);
+    const float rl = x_to_float(rlim), dtf = x_to_float(dt);
+    const float r2 = fmaf(z, z, fmaf(y, y, x * x)), v2 = fmaf(w, w, fmaf(v, v, u * u));
+    if (!(r2 > 1e-30f && r2 < 1e30f && v2 < 1e30f && r2 > rl * rl * 1.00001f)) return false;
+    if (!lvdotr) return true;
+    const float vd = fmaf(z, w, fmaf(y, v, x * u));
+    const float avd = 1e-5f * fmaf(fabsf(z), fabsf(w), fmaf(fabsf(y), fabsf(v), fabsf(x) * fabsf(u)));
+    return vd < -avd || r2 > v2 * dtf * dtf * 1.0001f;
+}
+
+// (rhill sum)^2 rhscale^2 of a pair: the square of its level-0 shell radius
+__device__ __forceinline__ double d_shell_base(bool isp, double rhill1, double rhill2, double rs2) {
+    if (!isp) return (rhill1 * rhill1) * rs2;
+    const double rhs = rhill1 + rhill2;
+    return (rhs * rhs) * rs2;
+}
+
+// The kick factors of one pair at level irec (symba_kick_list_plpl / _pltp, symba_kick.f90:126-340):
+// kp / km: the +1 / -1 kick acts (r^2 not below the next shell); fp / fm: its factor.  base:
+// d_shell_base.  Mixed path: isb = 1 / sqrt(base), so 1 / sqrt(ri) is a product with the table ik[k] =
+// RSHELL^-k / (1 - RSHELL); the -1 kick's inner limit is the +1 kick's outer one.  FP64 path: the
+// reference's operations, with IEEE square roots and quotients (fp64_exact.cuh) and the correctly
+// rounded r^-1.5 shared with the oracle.
+struct KickFac {
+    bool kp, km;
+    double fp, fm;
+};
+__device__ __forceinline__ KickFac d_kick_factors(bool fast, bool both, double base, double isb, const double *dx,
+                                                  double shell_p, double shell_m, double ik_p, double ik_m) {
+    KickFac k;
+    const double ri_p = base * shell_p, ri_m = base * shell_m;
+    constexpr double R2 = RSHELL * RSHELL;
+    if (fast) {
+        const double r2 = fma(dx[2], dx[2], fma(dx[1], dx[1], dx[0] * dx[0]));
+        k.kp = !x_less(r2, ri_p * R2);
+        const bool out_p = !x_less(r2, ri_p);
+        k.km = both && out_p;
+        if (!k.kp) return k;
+        const double y = x_rsqrt(r2), r = r2 * y, ir3 = (y * y) * y;
+        auto shell = [&](double q) {  // rr = (1 - r / sqrt(ri)) / (1 - RSHELL); 1 - 3 rr^2 + 2 rr^3 as 1 + rr^2 (2 rr - 3)
+            const double rr = fma(-r, q, 1.0 / (1.0 - RSHELL));
+            return ir3 * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
+        };
+        k.fp = k.fm = ir3;
+        if (!out_p) k.fp = shell(isb * ik_p);
+        else if (k.km && x_less(r2, ri_m)) k.fm = shell(isb * ik_m);
+        return k;
+    }
+    const double r2 = dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
+    k.kp = !x_less(r2, ri_p * R2);
+    k.km = both && !x_less(r2, ri_m * R2);
+    if (!k.kp && !k.km) return k;
+    const bool shp = k.kp && x_less(r2, ri_p), shm = k.km && x_less(r2, ri_m);
+    const double r = xsqrt(r2), r3 = r2 * r, ir3 = xdiv(1.0, r3);
+    k.fp = k.fm = ir3;
+    if (shp || shm) {
+        const double p = pow_m1p5(r2, r, r3, ir3);
+        auto shell = [&](double ri) {
+            const double s = xsqrt(ri), rr = xdiv(s - r, s * (1.0 - RSHELL));
+            return p * (1.0 - 3.0 * (rr * rr) + 2.0 * (rr * rr * rr));
+        };
+        if (shp) k.fp = shell(ri_p);
+        if (shm) k.fm = shell(ri_m);
+    }
+    return k;
+}
+
+// Component c's terms of one pair (t: the entry's terms + c): +1 kick of index1 and index2 at 0 and
+// 3, -1 kick at 6 and 9 (a pl-tp entry: the tp's at 0 and 6).
+__device__ __forceinline__ void kick_terms(bool fast, bool isp, const KickFac &f, double gm1, double gm2, double dc,
+                                           double *t) {
+    if (fast) {  // G m dc shared by the signs
+        const double g1 = gm1 * dc, g2 = gm2 * dc;
+        if (f.kp) t[0] = f.fp * (isp ? g2 : g1);
+        if (f.kp && isp) t[3] = f.fp * g1;
+        if (f.km) t[6] = f.fm * (isp ? g2 : g1);
+        if (f.km && isp) t[9] = f.fm * g1;
+        return;
+    }
+    for (int sg = 0; sg < 2; sg++) {
+        if (!(sg == 0 ? f.kp : f.km)) continue;
+        const double fac = sg == 0 ? f.fp : f.fm;
+        t[6 * sg] = (isp ? fac * gm2 : fac * gm1) * dc;
+        if (isp) t[6 * sg + 3] = (fac * gm1) * dc;
+    }
+}
 
 // Item index of this thread in the recursion kernel's block loops (blockDim a multiple
 // of 128): items k, k+1, k+2, k+3 go to warps 0-3, one per SM sub-partition, then to the
@@ -515,20 +657,10 @@ static __device__ void blk_list_check(const RecArgs &a, int irec, double dt, int
                 xr[d] = rj[d] - a.rh[3 * i + d];
                 vr[d] = vj[d] - a.vb[3 * i + d];
             }
-            const double renci = a.rhill[i] * a.rhscale * rs_pow[irec];  // d_renc(rhill_i, rhscale, irec)
-            const double rcrit = isp ? renci + a.rhill[j] * a.rhscale * rs_pow[irec] : renci;
-            int le, lvd;
-            if (a.fast)
-                d_enc_one_fast(xr[0], xr[1], xr[2], vr[0], vr[1], vr[2], rcrit, dt, le, lvd);
-            else
-                d_enc_one(xr[0], xr[1], xr[2], vr[0], vr[1], vr[2], rcrit, dt, le, lvd);
+            int lvd;
+            const bool le = d_list_pair(a.fast, isp, xr, vr, a.rhill[i] * a.rhscale, isp ? a.rhill[j] * a.rhscale : 0.0,
+                                        rs_pow[irec], a.radius[i], isp ? a.radius[j] : 0.0, dt, lvd);
             lv[q] = lvd;
-            if (le) {
-                const double rs = isp ? a.radius[i] + a.radius[j] : a.radius[i];
-                const double rlim2 = isp ? rs * rs : a.radius[i] * a.radius[i];
-                const double rji2 = xr[0] * xr[0] + xr[1] * xr[1] + xr[2] * xr[2];
-                le = rji2 > rlim2;
-            }
             le_out = (uint8_t)le;
         }
         a.lenc[k] = le_out;
@@ -574,9 +706,9 @@ static __device__ void blk_list_check(const RecArgs &a, int irec, double dt, int
 // (r^2 < rim1).  terms: 12 doubles per entry, the +1 pair terms then the -1 pair terms.
 // The reference's lmask refresh at entry is kept by the step loop instead (lmask ==
 // status /= INACTIVE wherever the recursion runs).
-// pw[m] = d_powi(RSHELL, m), m <= 2 MAXLEV.
+// pw[m] = d_powi(RSHELL, m), m <= 2 MAXLEV; ik[k] = RSHELL^-k / (1 - RSHELL) (mixed path).
 static __device__ void blk_kick_lists(const RecArgs &a, int nbpl, int nbtp, double dt, int irec, bool both,
-                                      const double *pw) {
+                                      const double *pw, const double *ik) {
     const int64_t npp = a.npp, npt = a.npt;
     if (npp + npt == 0) return;
     const int irm1 = irec - 1;
@@ -605,65 +737,18 @@ static __device__ void blk_kick_lists(const RecArgs &a, int nbpl, int nbtp, doub
             }
             continue;
         }
-        double base;
-        if (isp) {
-            const double rhs = a.rhill[i] + a.rhill[j];
-            base = (rhs * rhs) * rs2;
-        } else {
-            base = (a.rhill[i] * a.rhill[i]) * rs2;
-        }
-        const double ri_p = base * shell_p, ri_m = base * shell_m;
+        const double base = d_shell_base(isp, a.rhill[i], isp ? a.rhill[j] : 0.0, rs2);
         const double *rj = isp ? &a.rh[3 * j] : &a.trh[3 * j];
         double dx[3];
         for (int d = 0; d < 3; d++) dx[d] = rj[d] - a.rh[3 * i + d];
-        const double r2 = a.fast ? fma(dx[2], dx[2], fma(dx[1], dx[1], dx[0] * dx[0]))
-                                 : dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
-        const bool kp = !(r2 < ri_p * (RSHELL * RSHELL));
-        const bool km = both && !(r2 < ri_m * (RSHELL * RSHELL));
+        const KickFac f = d_kick_factors(a.fast, both, base, a.fast ? x_rsqrt(base) : 0.0, dx, shell_p, shell_m,
+                                         ik[irec], ik[irec - 1]);
         if (c == 0) {
-            a.good[k] = kp ? 1 : 2;
-            a.good2[k] = both ? (km ? 1 : 2) : 0;
+            a.good[k] = f.kp ? 1 : 2;
+            a.good2[k] = both ? (f.km ? 1 : 2) : 0;
         }
-        if (!kp && !km) continue;
-        const bool shp = kp && r2 < ri_p, shm = km && r2 < ri_m;
-        // FP64 path: IEEE square root and divide, and the correctly rounded r^-1.5 shared
-        // with the oracle; mixed path: r and r^-3 from one reciprocal square root
-        double r, ir3;
-        if (a.fast) {
-            const double y = rsqrt(r2);
-            r = r2 * y;
-            ir3 = (y * y) * y;
-        } else {
-            r = sqrt(r2);
-            ir3 = 1.0 / (r2 * r);
-        }
-        double p = ir3;
-        if (!a.fast && (shp || shm)) p = pow_m1p5(r2);
-        auto shell = [&](double ri) {
-            // rr = (sqrt(ri) - r) / (sqrt(ri) (1 - RSHELL)); mixed path as (1 - r / sqrt(ri)) / (1 - RSHELL)
-            if (a.fast) {  // 1 - 3 rr^2 + 2 rr^3 as 1 + rr^2 (2 rr - 3)
-                const double rr = fma(-r, rsqrt(ri), 1.0) * (1.0 / (1.0 - RSHELL));
-                return p * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
-            }
-            const double rr = (sqrt(ri) - r) / (sqrt(ri) * (1.0 - RSHELL));
-            return p * (1.0 - 3.0 * (rr * rr) + 2.0 * (rr * rr * rr));
-        };
-        double *t = &a.terms[12 * k];
         const double dc = c == 0 ? dx[0] : (c == 1 ? dx[1] : dx[2]);
-        for (int sg = 0; sg < 2; sg++) {
-            if (!(sg == 0 ? kp : km)) continue;
-            const bool sh = sg == 0 ? shp : shm;
-            const double fac = sh ? shell(sg == 0 ? ri_p : ri_m) : ir3;
-            double *ts = t + 6 * sg;
-            const double faci = fac * a.Gm[i];
-            if (isp) {
-                const double facj = fac * a.Gm[j];
-                ts[c] = facj * dc;
-                ts[3 + c] = faci * dc;
-            } else {
-                ts[c] = faci * dc;
-            }
-        }
+        kick_terms(a.fast, isp, f, a.Gm[i], isp ? a.Gm[j] : 0.0, dc, &a.terms[12 * k + c]);
     }
     __syncthreads();
     // ordered per-body accumulation and the velocity kicks, +1 then -1; three items per body,
@@ -761,8 +846,9 @@ static __device__ void blk_collision_check(const RecArgs &a, int irec, double dt
         const double *vj = isp ? &a.vb[3 * j] : &a.tvb[3 * j];
         const double xr = a.rh[3 * i] - rj[0], yr = a.rh[3 * i + 1] - rj[1], zr = a.rh[3 * i + 2] - rj[2];
         const double vxr = a.vb[3 * i] - vj[0], vyr = a.vb[3 * i + 1] - vj[1], vzr = a.vb[3 * i + 2] - vj[2];
-        const double Gmtot = isp ? a.Gm[i] + a.Gm[j] : a.Gm[i];
         const double rlim = isp ? a.radius[i] + a.radius[j] : a.radius[i];
+        if (d_collision_far(xr, yr, zr, vxr, vyr, vzr, rlim, dt, l[2 * cap + q] != 0)) continue;
+        const double Gmtot = isp ? a.Gm[i] + a.Gm[j] : a.Gm[i];
         if (d_collision_one(xr, yr, zr, vxr, vyr, vzr, Gmtot, rlim, dt, l[2 * cap + q] != 0)) {
             st[q] = ST_COLLIDED;
             *s_coll = 1;
@@ -986,8 +1072,9 @@ static __device__ void blk_build_adjacency(const RecArgs &a, int nbpl, int nbtp)
 // written back at the end (or at a pause for a collision).
 struct RecStage {
     double *r, *v;                 // per slot: position, velocity (3 each)
-    double *gm, *rhill, *rad;      // per slot: G*m, Hill radius, radius (0 for test particles)
+    double *gm, *rhs, *rad;        // per slot: G*m, Hill radius * rhscale, radius (0 for test particles)
     double *terms;                 // 12 per entry
+    double *base, *isb;            // per entry: d_shell_base and (mixed path) 1 / its square root
     int32_t *lev, *st, *gidx;      // per slot: levelg / tlevelg, status / tstatus, global index
     int32_t *s1, *s2;              // per entry: slots of index1 and index2
     int32_t *est, *elev, *elv;     // per entry: status, level, lvdotr
@@ -1001,7 +1088,7 @@ constexpr size_t REC_STAGE_MAX = 160 * 1024, REC_STAGE_ENS = 64 * 1024;
 // (a pl-tp entry names one pl and one tp), and 2 npp + npt adjacency entries.
 __host__ __device__ inline size_t rec_stage_bytes(int64_t npp, int64_t npt) {
     const int64_t n = npp + npt, nb = 2 * n;
-    return (size_t)(9 * nb + 12 * n) * 8 + (size_t)(4 * nb + 5 * n + 2 * npp + npt) * 4 + (size_t)(3 * n + 16);
+    return (size_t)(9 * nb + 14 * n) * 8 + (size_t)(4 * nb + 5 * n + 2 * npp + npt) * 4 + (size_t)(3 * n + 16);
 }
 static __device__ RecStage rec_stage_carve(void *base, int64_t npp, int64_t npt) {
     const int64_t n = npp + npt, nb = 2 * n;
@@ -1010,10 +1097,12 @@ static __device__ RecStage rec_stage_carve(void *base, int64_t npp, int64_t npt)
     S.r = d;
     S.v = d + 3 * nb;
     S.gm = d + 6 * nb;
-    S.rhill = d + 7 * nb;
+    S.rhs = d + 7 * nb;
     S.rad = d + 8 * nb;
     S.terms = d + 9 * nb;
-    int32_t *i = (int32_t *)(S.terms + 12 * n);
+    S.base = S.terms + 12 * n;
+    S.isb = S.base + n;
+    int32_t *i = (int32_t *)(S.isb + n);
     S.lev = i;
     S.st = i + nb;
     S.gidx = i + 2 * nb;
@@ -1044,7 +1133,7 @@ static __device__ void stg_load(const RecArgs &a, const RecStage &S, int nbpl, i
             S.v[3 * b + d] = w[d];
         }
         S.gm[b] = isp ? a.Gm[g] : 0.0;
-        S.rhill[b] = isp ? a.rhill[g] : 0.0;
+        S.rhs[b] = isp ? a.rhill[g] * a.rhscale : 0.0;
         S.rad[b] = isp ? a.radius[g] : 0.0;
         S.lev[b] = isp ? a.levelg[g] : a.tlevelg[g];
         S.st[b] = isp ? a.status[g] : a.tstatus[g];
@@ -1060,6 +1149,8 @@ static __device__ void stg_load(const RecArgs &a, const RecStage &S, int nbpl, i
         const int i = l[q] - 1, j = l[cap + q] - 1;
         S.s1[k] = a.mark_pl[i] - 1;
         S.s2[k] = isp ? a.mark_pl[j] - 1 : a.mark_tp[j] - 1;
+        S.base[k] = d_shell_base(isp, a.rhill[i], isp ? a.rhill[j] : 0.0, a.rhscale * a.rhscale);
+        S.isb[k] = a.fast ? x_rsqrt(S.base[k]) : 0.0;
         S.elv[k] = l[2 * cap + q];
         S.est[k] = l[3 * cap + q];
         S.elev[k] = l[4 * cap + q];
@@ -1109,20 +1200,9 @@ static __device__ void stg_list_check(const RecArgs &a, const RecStage &S, int i
                 xr[d] = S.r[3 * b2 + d] - S.r[3 * b1 + d];
                 vr[d] = S.v[3 * b2 + d] - S.v[3 * b1 + d];
             }
-            const double renci = S.rhill[b1] * a.rhscale * rs_pow[irec];  // d_renc(rhill_i, rhscale, irec)
-            const double rcrit = isp ? renci + S.rhill[b2] * a.rhscale * rs_pow[irec] : renci;
-            int le, lvd;
-            if (a.fast)
-                d_enc_one_fast(xr[0], xr[1], xr[2], vr[0], vr[1], vr[2], rcrit, dt, le, lvd);
-            else
-                d_enc_one(xr[0], xr[1], xr[2], vr[0], vr[1], vr[2], rcrit, dt, le, lvd);
+            int lvd;
+            const bool le = d_list_pair(a.fast, isp, xr, vr, S.rhs[b1], S.rhs[b2], rs_pow[irec], S.rad[b1], S.rad[b2], dt, lvd);
             S.elv[k] = lvd;
-            if (le) {
-                const double rs = isp ? S.rad[b1] + S.rad[b2] : S.rad[b1];
-                const double rlim2 = isp ? rs * rs : S.rad[b1] * S.rad[b1];
-                const double rji2 = xr[0] * xr[0] + xr[1] * xr[1] + xr[2] * xr[2];
-                le = rji2 > rlim2;
-            }
             le_out = (uint8_t)le;
         }
         S.lenc[k] = le_out;
@@ -1143,19 +1223,17 @@ static __device__ void stg_list_check(const RecArgs &a, const RecStage &S, int i
 }
 // blk_kick_lists on the stage (same pair terms, same per-body order)
 static __device__ void stg_kick_lists(const RecArgs &a, const RecStage &S, int nbpl, int nbtp, double dt, int irec,
-                                      bool both, const double *pw) {
-    const int64_t npp = a.npp, n = a.npp + a.npt;
+                                      bool both, const double *pw, const double *ik) {
+    const int npp = (int)a.npp, n = (int)(a.npp + a.npt);  // the stage holds a few hundred entries
     if (n == 0) return;
     const int irm1 = irec - 1;
-    const double rs2 = a.rhscale * a.rhscale;
     const double shell_p = pw[2 * irec], shell_m = pw[2 * (irec - 1)];
     const bool do_pp = a.npl > 0, do_pt = a.npl > 0 && a.ntp > 0;
     // three items per pair, one per vector component c: each forms the pair's factors (the
     // same instructions in every lane, which costs a warp no more FP64 issue than one lane)
     // and writes only its component's terms
-    for (int64_t kc = spread_tid(); kc < 3 * n; kc += blockDim.x) {
-        const int64_t k = kc / 3;
-        const int c = (int)(kc - 3 * k);
+    for (int kc = spread_tid(); kc < 3 * n; kc += blockDim.x) {
+        const int k = kc / 3, c = kc - 3 * k;
         const bool isp = k < npp;
         const int b1 = S.s1[k], b2 = S.s2[k];
         const bool g = (isp ? do_pp : do_pt) && (S.est[k] == ST_ACTIVE) && (S.lev[b1] >= irm1) && (S.lev[b2] >= irm1);
@@ -1166,61 +1244,16 @@ static __device__ void stg_kick_lists(const RecArgs &a, const RecStage &S, int n
             }
             continue;
         }
-        double base;
-        if (isp) {
-            const double rhs = S.rhill[b1] + S.rhill[b2];
-            base = (rhs * rhs) * rs2;
-        } else {
-            base = (S.rhill[b1] * S.rhill[b1]) * rs2;
-        }
-        const double ri_p = base * shell_p, ri_m = base * shell_m;
         double dx[3];
         for (int d = 0; d < 3; d++) dx[d] = S.r[3 * b2 + d] - S.r[3 * b1 + d];
-        const double r2 = a.fast ? fma(dx[2], dx[2], fma(dx[1], dx[1], dx[0] * dx[0]))
-                                 : dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
-        const bool kp = !(r2 < ri_p * (RSHELL * RSHELL));
-        const bool km = both && !(r2 < ri_m * (RSHELL * RSHELL));
+        const KickFac f =
+            d_kick_factors(a.fast, both, S.base[k], S.isb[k], dx, shell_p, shell_m, ik[irec], ik[irec - 1]);
         if (c == 0) {
-            S.good[k] = kp ? 1 : 2;
-            S.good2[k] = both ? (km ? 1 : 2) : 0;
+            S.good[k] = f.kp ? 1 : 2;
+            S.good2[k] = both ? (f.km ? 1 : 2) : 0;
         }
-        if (!kp && !km) continue;
-        const bool shp = kp && r2 < ri_p, shm = km && r2 < ri_m;
-        double r, ir3;
-        if (a.fast) {
-            const double y = rsqrt(r2);
-            r = r2 * y;
-            ir3 = (y * y) * y;
-        } else {
-            r = sqrt(r2);
-            ir3 = 1.0 / (r2 * r);
-        }
-        double p = ir3;
-        if (!a.fast && (shp || shm)) p = pow_m1p5(r2);
-        auto shell = [&](double ri) {
-            if (a.fast) {  // 1 - 3 rr^2 + 2 rr^3 as 1 + rr^2 (2 rr - 3)
-                const double rr = fma(-r, rsqrt(ri), 1.0) * (1.0 / (1.0 - RSHELL));
-                return p * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
-            }
-            const double rr = (sqrt(ri) - r) / (sqrt(ri) * (1.0 - RSHELL));
-            return p * (1.0 - 3.0 * (rr * rr) + 2.0 * (rr * rr * rr));
-        };
-        double *t = &S.terms[12 * k];
         const double dc = c == 0 ? dx[0] : (c == 1 ? dx[1] : dx[2]);
-        for (int sg = 0; sg < 2; sg++) {
-            if (!(sg == 0 ? kp : km)) continue;
-            const bool sh = sg == 0 ? shp : shm;
-            const double fac = sh ? shell(sg == 0 ? ri_p : ri_m) : ir3;
-            double *ts = t + 6 * sg;
-            const double faci = fac * S.gm[b1];
-            if (isp) {
-                const double facj = fac * S.gm[b2];
-                ts[c] = facj * dc;
-                ts[3 + c] = faci * dc;
-            } else {
-                ts[c] = faci * dc;
-            }
-        }
+        kick_terms(a.fast, isp, f, S.gm[b1], S.gm[b2], dc, &S.terms[12 * k + c]);
     }
     __syncthreads();
     // three items per body, one per vector component c: each adds its component of the
@@ -1295,8 +1328,9 @@ static __device__ void stg_collision_check(const RecArgs &a, const RecStage &S, 
         const double *ri = &S.r[3 * b1], *rj = &S.r[3 * b2], *vi = &S.v[3 * b1], *vj = &S.v[3 * b2];
         const double xr = ri[0] - rj[0], yr = ri[1] - rj[1], zr = ri[2] - rj[2];
         const double vxr = vi[0] - vj[0], vyr = vi[1] - vj[1], vzr = vi[2] - vj[2];
-        const double Gmtot = isp ? S.gm[b1] + S.gm[b2] : S.gm[b1];
         const double rlim = isp ? S.rad[b1] + S.rad[b2] : S.rad[b1];
+        if (d_collision_far(xr, yr, zr, vxr, vyr, vzr, rlim, dt, S.elv[k] != 0)) continue;
+        const double Gmtot = isp ? S.gm[b1] + S.gm[b2] : S.gm[b1];
         if (d_collision_one(xr, yr, zr, vxr, vyr, vzr, Gmtot, rlim, dt, S.elv[k] != 0)) {
             S.est[k] = ST_COLLIDED;
             *s_coll = 1;
@@ -1320,12 +1354,14 @@ static __device__ void blk_symba_recursion_t(const RecArgs &a, void *stage) {
     // shell-radius powers, formed once per launch with the per-call algorithms (same bits):
     // s_pw[m] = d_powi(RSHELL, m) (the kick's shell radii), s_rs[k] = RSHELL^k by repeated
     // products (d_renc, the list check's encounter radii)
-    __shared__ double s_pw[2 * MAXLEV + 2], s_rs[MAXLEV + 1];
+    // s_ik[k] = RSHELL^-k / (1 - RSHELL) (the mixed path's shell polynomial)
+    __shared__ double s_pw[2 * MAXLEV + 2], s_rs[MAXLEV + 1], s_ik[MAXLEV + 1];
     // each level's step dt / 3^k and the underflow test of symba_step.f90:196-201, formed
     // once per launch as the loop would form them (the FP64 divides are long on GB300)
     __shared__ double s_dtl[MAXLEV];
     __shared__ unsigned char s_under[MAXLEV];
     for (int m = threadIdx.x; m < 2 * MAXLEV + 2; m += blockDim.x) s_pw[m] = d_powi(RSHELL, m);
+    for (int k = threadIdx.x; k <= MAXLEV; k += blockDim.x) s_ik[k] = xdiv(1.0 / (1.0 - RSHELL), d_powi(RSHELL, k));
     for (int k = threadIdx.x; k < MAXLEV; k += blockDim.x) {
         double p3 = 1.0;
         for (int q = 0; q < k; q++) p3 *= 3.0;
@@ -1406,11 +1442,11 @@ static __device__ void blk_symba_recursion_t(const RecArgs &a, void *stage) {
             __syncthreads();
             if constexpr (STAGED) {
                 stg_list_check(a, S, irecp, dtl, &s_any, s_rs);
-                stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
+                stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
                 stg_drift(a, S, nbpl, nbtp, ireci, dtl, inv_gm);
             } else {
                 blk_list_check(a, irecp, dtl, &s_any, s_rs);
-                blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
+                blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
                 blk_drift(a, nbpl, nbtp, ireci, dtl, inv_gm);
             }
             const int any = s_any;
@@ -1431,9 +1467,9 @@ static __device__ void blk_symba_recursion_t(const RecArgs &a, void *stage) {
         }
         // after the deeper levels (or none) for loop j of level ireci
         if constexpr (STAGED)
-            stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
+            stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
         else
-            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
+            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
         if (a.lclose) {
             if (threadIdx.x == 0) s_any = 0;
             __syncthreads();
