@@ -38,14 +38,14 @@ __host__ __device__ inline double hd_pot_term(const double *ri, const double *rj
 // quotient and square root: on the device outside the FP64 pipe (fp64_exact.cuh, the same bits)
 __host__ __device__ inline double hd_div(double a, double b) {
 #ifdef __CUDA_ARCH__
-    return xdiv(a, b);
+    return xdiv_call(a, b);
 #else
     return a / b;
 #endif
 }
 __host__ __device__ inline double hd_sqrt(double x) {
 #ifdef __CUDA_ARCH__
-    return xsqrt(x);
+    return xsqrt_call(x);
 #else
     return sqrt(x);
 #endif

@@ -19,11 +19,11 @@ constexpr int NLAG2 = 40;
 __device__ __forceinline__ bool less_than_4(double x) { return (__double2hiint(x) & 0x7fffffff) < 0x40100000; }
 
 __device__ __forceinline__ void d_scget(double angle, double &sx, double &cx) {
-    const int nper = (int)xdiv(angle, TWOPI);
+    const int nper = (int)xdiv_call(angle, TWOPI);
     double x = angle - nper * TWOPI;
     if (x < 0.0) x = x + TWOPI;
     sx = sin(x);
-    cx = xsqrt(1.0 - sx * sx);
+    cx = xsqrt_call(1.0 - sx * sx);
     if ((x > PIBY2) && (x < PI3BY2)) cx = -cx;
 }
 
@@ -40,11 +40,11 @@ __device__ __forceinline__ void d_stumpff(double x, double &c0, double &c1, doub
     c2 = c3 = 1.0;
 #pragma unroll 1
     for (int k = 0; k < 6; k++) {
-        c2 = 1.0 - xdiv(x * c2, STUMPFF_Q2[k]);
-        c3 = 1.0 - xdiv(x * c3, STUMPFF_Q3[k]);
+        c2 = 1.0 - xdiv_call(x * c2, STUMPFF_Q2[k]);
+        c3 = 1.0 - xdiv_call(x * c3, STUMPFF_Q3[k]);
     }
     c2 = c2 / 2.0;
-    c3 = xdiv(c3, 6.0);
+    c3 = xdiv_call(c3, 6.0);
     c1 = 1.0 - x * c3;
     c0 = 1.0 - x * c2;
     for (int i = n; i >= 1; i--) {
@@ -64,7 +64,7 @@ __device__ inline void d_kepmd(xd dm, xd es, xd ec, xd &x, xd &s, xd &c) {
     xd xx = q * (one - xd(x_half(fac1.v)) * q * (es - q * fac2));
     xd y = xx * xx;
     xd ss = xx * (a0 - y * (a1 - y * (a2 - y * (a3 - y * (a4 - y))))) / a0;
-    xd cc = xsqrt((one - ss * ss).v);
+    xd cc = root(one - ss * ss);
     const xd ecs = ec * ss, ecc = ec * cc, ess = es * ss, esc = es * cc;
     const xd f = xx - ecs + es * (one - cc) - dm;
     const xd fp = one - ecc + ess;
@@ -76,7 +76,7 @@ __device__ inline void d_kepmd(xd dm, xd es, xd ec, xd &x, xd &s, xd &c) {
     xx = xx + dx;
     y = xx * xx;
     ss = xx * (a0 - y * (a1 - y * (a2 - y * (a3 - y * (a4 - y))))) / a0;
-    cc = xsqrt((one - ss * ss).v);
+    cc = root(one - ss * ss);
     x = xx;
     s = ss;
     c = cc;
@@ -112,21 +112,21 @@ __device__ inline void d_p3solve(double dt, double r0, double mu, double alpha, 
 __device__ inline void d_kepu_guess(double dt, double r0, double mu, double alpha, double u, double &s) {
     const double thresh = 0.4, danbyk = 0.85;
     if (alpha > 0.0) {
-        const double dr = xdiv(dt, r0);
+        const double dr = xdiv_call(dt, r0);
         if (dr <= thresh) {
-            s = dr - xdiv(dt * dt * u, 2.0 * r0 * r0 * r0);
+            s = dr - xdiv_call(dt * dt * u, 2.0 * r0 * r0 * r0);
         } else {
-            const double a = xdiv(mu, alpha);
-            const double en = xsqrt(xdiv(mu, a * a * a));
-            const double ec = 1.0 - xdiv(r0, a);
-            const double es = xdiv(u, en * a * a);
-            const double e = xsqrt(ec * ec + es * es);
+            const double a = xdiv_call(mu, alpha);
+            const double en = xsqrt_call(xdiv_call(mu, a * a * a));
+            const double ec = 1.0 - xdiv_call(r0, a);
+            const double es = xdiv_call(u, en * a * a);
+            const double e = xsqrt_call(ec * ec + es * es);
             const double y = en * dt - es;
             double sy, cy;
             d_scget(y, sy, cy);
             const double sigma = copysign(1.0, es * cy + ec * sy);
             const double x = y + sigma * danbyk * e;
-            s = xdiv(x, xsqrt(alpha));
+            s = xdiv_call(x, xsqrt_call(alpha));
         }
     } else {
         int iflag;
@@ -158,11 +158,11 @@ __device__ inline void d_kepu_new(double &s, double dt, double r0, double mu, do
         fp = r0 * c0 + u * c1 + mu * c2;
         const double fpp = (-(r0 * alpha) + mu) * c1 + u * c0;
         const double fppp = (-(r0 * alpha) + mu) * c0 - u * alpha * c1;
-        double ds = -xdiv(f, fp);
-        ds = -xdiv(f, fp + ds * fpp / 2.0);
-        ds = -xdiv(f, fp + ds * fpp / 2.0 + xdiv(ds * ds * fppp, 6.0));
+        double ds = -xdiv_call(f, fp);
+        ds = -xdiv_call(f, fp + ds * fpp / 2.0);
+        ds = -xdiv_call(f, fp + ds * fpp / 2.0 + xdiv_call(ds * ds * fppp, 6.0));
         s = s + ds;
-        const double fdt = xdiv(f, dt);
+        const double fdt = xdiv_call(f, dt);
         if (fdt * fdt < DANBYB * DANBYB) {
             iflag = 0;
             return;
@@ -187,9 +187,9 @@ __device__ inline void d_kepu_lag(double &s, double dt, double r0, double mu, do
         const double fpp = (-(r0 * alpha) + mu) * c1 + u * c0;
         const double lnm1 = (double)ln - 1.0;
         const double disc = fabs(lnm1 * lnm1 * fp * fp - lnm1 * (double)ln * f * fpp);
-        const double ds = -xdiv((double)ln * f, fp + copysign(1.0, fp) * xsqrt(disc));
+        const double ds = -xdiv_call((double)ln * f, fp + copysign(1.0, fp) * xsqrt_call(disc));
         s = s + ds;
-        const double fdt = xdiv(f, dt);
+        const double fdt = xdiv_call(f, dt);
         if (fdt * fdt < DANBYB * DANBYB) {
             iflag = 0;
             return;
@@ -220,10 +220,10 @@ static __device__ __noinline__ void d_drift_kepu(double mu, double &rx0, double 
     double fp, c1, c2, c3;
     d_kepu(dt, r0, mu, alpha, u, fp, c1, c2, c3, iflag);
     if (iflag == 0) {
-        const double f = 1.0 - xdiv(mu, r0) * c2;
+        const double f = 1.0 - xdiv_call(mu, r0) * c2;
         const double g = dt - mu * c3;
-        const double fdot = -(xdiv(mu, fp * r0) * c1);
-        const double gdot = 1.0 - xdiv(mu, fp) * c2;
+        const double fdot = -(xdiv_call(mu, fp * r0) * c1);
+        const double gdot = 1.0 - xdiv_call(mu, fp) * c2;
         const double rx = rx0 * f + vx0 * g;
         const double ry = ry0 * f + vy0 * g;
         const double rz = rz0 * f + vz0 * g;
@@ -245,20 +245,20 @@ __device__ inline void d_drift_dan(double mu, double &rx0, double &ry0, double &
     double dt = dt0;
     iflag = 0;
     const xd X = rx0, Y = ry0, Z = rz0, U = vx0, V = vy0, W = vz0, one = 1.0;
-    const double r0 = xsqrt((X * X + Y * Y + Z * Z).v);
+    const double r0 = root(X * X + Y * Y + Z * Z).v;
     const xd v0s = U * U + V * V + W * W;
     const double u = (X * U + Y * V + Z * W).v;
     const double alpha = (xd(2.0 * mu) / r0 - v0s).v;
     if (x_greater(alpha, 0.0)) {
-        const xd a = xdiv(mu, alpha);
+        const xd a = xd(mu) / alpha;
         const xd asq = a * a;
-        const xd en = xsqrt((xd(mu) / (a * asq)).v);
+        const xd en = root(xd(mu) / (a * asq));
         const xd ec = one - xd(r0) / a;
         const xd es = xd(u) / (en * asq);
         const xd esq = ec * ec + es * es;
         const xd den = xd(dt) * en;
         // dt en - int(dt en / 2 pi) 2 pi, whose integer is zero below 4
-        const xd dm = less_than_4(den.v) ? den.v : den.v - (double)(int)xdiv(den.v, TWOPI) * TWOPI;
+        const xd dm = less_than_4(den.v) ? den.v : den.v - (double)(int)xdiv_call(den.v, TWOPI) * TWOPI;
         const xd dm2 = dm * dm;
         dt = (dm / en).v;
         if (x_less(esq.v, E2MAX) && x_less(dm2.v, DM2MAX) && x_less((esq * dm2).v, E2DM2MAX)) {

@@ -377,9 +377,9 @@ __device__ __forceinline__ void d_enc_one(double xr, double yr, double zr, doubl
             if (v2 <= VSMALL) {
                 r2min = r2;
             } else {
-                const double tmin = xdiv(-vdotr, v2);
+                const double tmin = xdiv_call(-vdotr, v2);
                 if (tmin < dt)
-                    r2min = r2 - xdiv(vdotr * vdotr, v2);
+                    r2min = r2 - xdiv_call(vdotr * vdotr, v2);
                 else
                     r2min = r2 + 2.0 * vdotr * dt + v2 * (dt * dt);
             }
@@ -409,7 +409,7 @@ __device__ __forceinline__ void d_enc_one_fast(double xr, double yr, double zr, 
             if (v2 <= VSMALL) {
                 r2min = r2;
             } else {
-                const double iv2 = xdiv(1.0, v2);
+                const double iv2 = xdiv_call(1.0, v2);
                 const double tmin = -vdotr * iv2;
                 if (tmin < dt)
                     r2min = fma(-(vdotr * vdotr), iv2, r2);
@@ -433,7 +433,7 @@ __device__ __forceinline__ void d_enc_one_fast(double xr, double yr, double zr, 
 __device__ __forceinline__ double pow_m1p5(double x, double s, double p, double y0) {
     if (!(x > 0.0) || isinf(x)) return pow(x, -1.5);
     const double rs = fma(-s, s, x);
-    const double ds = xdiv(rs, 2.0 * s);
+    const double ds = xdiv_call(rs, 2.0 * s);
     const double ep = fma(x, s, -p);
     const double ql = ep + x * ds;
     const double err = fma(-y0, p, 1.0) - y0 * ql;
@@ -448,7 +448,7 @@ __device__ __forceinline__ double d_powi(double x, int m) {
         x = x * x;
         if (n % 2) y = y * x;
     }
-    return m < 0 ? xdiv(1.0, y) : y;
+    return m < 0 ? xdiv_call(1.0, y) : y;
 }
 
 // Encounter lists live in one int32 allocation per kind: [i1 | i2 | lvdotr | status | level],
@@ -574,7 +574,7 @@ __device__ __forceinline__ KickFac d_kick_factors(bool fast, bool both, double b
         const bool out_p = !x_less(r2, ri_p);
         k.km = both && out_p;
         if (!k.kp) return k;
-        const double y = x_rsqrt(r2), r = r2 * y, ir3 = (y * y) * y;
+        const double y = x_rsqrt_call(r2), r = r2 * y, ir3 = (y * y) * y;
         auto shell = [&](double q) {  // rr = (1 - r / sqrt(ri)) / (1 - RSHELL); 1 - 3 rr^2 + 2 rr^3 as 1 + rr^2 (2 rr - 3)
             const double rr = fma(-r, q, 1.0 / (1.0 - RSHELL));
             return ir3 * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
@@ -589,12 +589,12 @@ __device__ __forceinline__ KickFac d_kick_factors(bool fast, bool both, double b
     k.km = both && !x_less(r2, ri_m * R2);
     if (!k.kp && !k.km) return k;
     const bool shp = k.kp && x_less(r2, ri_p), shm = k.km && x_less(r2, ri_m);
-    const double r = xsqrt(r2), r3 = r2 * r, ir3 = xdiv(1.0, r3);
+    const double r = xsqrt_call(r2), r3 = r2 * r, ir3 = xdiv_call(1.0, r3);
     k.fp = k.fm = ir3;
     if (shp || shm) {
         const double p = pow_m1p5(r2, r, r3, ir3);
         auto shell = [&](double ri) {
-            const double s = xsqrt(ri), rr = xdiv(s - r, s * (1.0 - RSHELL));
+            const double s = xsqrt_call(ri), rr = xdiv_call(s - r, s * (1.0 - RSHELL));
             return p * (1.0 - 3.0 * (rr * rr) + 2.0 * (rr * rr * rr));
         };
         if (shp) k.fp = shell(ri_p);
@@ -1361,7 +1361,7 @@ static __device__ void blk_symba_recursion_t(const RecArgs &a, void *stage) {
     __shared__ double s_dtl[MAXLEV];
     __shared__ unsigned char s_under[MAXLEV];
     for (int m = threadIdx.x; m < 2 * MAXLEV + 2; m += blockDim.x) s_pw[m] = d_powi(RSHELL, m);
-    for (int k = threadIdx.x; k <= MAXLEV; k += blockDim.x) s_ik[k] = xdiv(1.0 / (1.0 - RSHELL), d_powi(RSHELL, k));
+    for (int k = threadIdx.x; k <= MAXLEV; k += blockDim.x) s_ik[k] = xdiv_call(1.0 / (1.0 - RSHELL), d_powi(RSHELL, k));
     for (int k = threadIdx.x; k < MAXLEV; k += blockDim.x) {
         double p3 = 1.0;
         for (int q = 0; q < k; q++) p3 *= 3.0;
