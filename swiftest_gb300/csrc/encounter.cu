@@ -628,6 +628,11 @@ int shift_index2(swg_ctx *c, long long from, long long to, int32_t *i2, int shif
 
 namespace swg {
 
+// From this many pair tests on, a TRIANGULAR check of one list, or of massive bodies against test
+// particles, goes over radius-sorted tiles, which test a few percent of a disk's pairs but take
+// three launches and about 50 us; the all-pairs kernel tests 4.2e5 pairs per us.
+constexpr int64_t SORTED_PAIRS = 20000000;
+
 int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1, const double *r1,
                          const double *v1, const double *renc1, int32_t n2, const double *r2, const double *v2,
                          const double *renc2, double dt, int64_t *n_out, int32_t **o1, int32_t **o2,
@@ -639,14 +644,18 @@ int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1,
         w.rawcap = 1024;
         SWG_TRY(ensure(c, w.raw, (size_t)w.rawcap * 3 * sizeof(int32_t)));
     }
-    const int ntot = (kind == 0 ? n1 : n1 + n2);
-    SWG_TRY(ensure(c, w.sort, encounter_scratch_bytes(mode, n1, kind == 0 ? n1 : n2)));
-    (void)ntot;
+    const int64_t pairs = kind == 0 ? (int64_t)n1 * n1 / 2 : (int64_t)n1 * n2;
+    const bool sorted = mode == SWG_ENC_TRIANGULAR && kind != 1 && pairs >= SORTED_PAIRS;
+    SWG_TRY(ensure(c, w.sort, sorted ? encounter_sorted_one_bytes(n1, kind == 0 ? 0 : n2)
+                                     : encounter_scratch_bytes(mode, n1, kind == 0 ? n1 : n2)));
     unsigned long long h_count = 0;
     for (int attempt = 0; attempt < 8; attempt++) {
         int32_t *i1 = (int32_t *)w.raw.ptr, *i2 = i1 + w.rawcap, *lv = i2 + w.rawcap;
         SWG_TRY(cuda_status(c, cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), c->stream), "memset"));
-        if (kind == 0) {
+        if (sorted) {
+            SWG_TRY(encounter_sorted_one(c, n1, r1, v1, renc1, kind == 0 ? 0 : n2, r2, v2, dt, w.rawcap, i1, i2, lv,
+                                         d_count, w.sort.ptr));
+        } else if (kind == 0) {
             SWG_TRY(encounter_launch(c, mode, n1, r1, v1, renc1, n1, r1, v1, renc1, 1, 0, dt, w.rawcap, i1, i2, lv,
                                      d_count, w.sort.ptr));
         } else if (kind == 1) {
@@ -675,17 +684,15 @@ int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1,
     *o2 = i2;
     *olv = lv;
     if (h_count == 0) return SWG_OK;
-    const bool need_unique = (mode == SWG_ENC_SORTSWEEP);
-    (void)need_unique;
-    // sort by (index1, index2) and drop repeats (sweep duplicates); the sort scratch
-    // is separate from the sweep scratch only in size, the sweep is finished.
+    // sort by (index1, index2) and drop repeats; only the sweep repeats pairs, so only its count
+    // is read again
     const size_t need = sort_pairs_scratch_bytes((int64_t)h_count);
-    if (mode == SWG_ENC_SORTSWEEP) {
-        if (w.sort.bytes < need) SWG_TRY(ensure(c, w.sort, need));
-    } else {
-        SWG_TRY(ensure(c, w.sort, need));
-    }
+    if (w.sort.bytes < need) SWG_TRY(ensure(c, w.sort, need));
     SWG_TRY(sort_pairs_unique(c, (int64_t)h_count, i1, i2, lv, w.sort.ptr, d_count + 1));
+    if (mode == SWG_ENC_TRIANGULAR) {
+        *n_out = (int64_t)h_count;
+        return SWG_OK;
+    }
     unsigned long long h_unique = 0;
     SWG_TRY(cuda_status(c, cudaMemcpyAsync(&h_unique, d_count + 1, sizeof(h_unique), cudaMemcpyDeviceToHost, c->stream),
                         "count"));

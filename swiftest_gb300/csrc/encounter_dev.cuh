@@ -86,7 +86,7 @@ __device__ __forceinline__ BodyF load_body(const double *r, const double *v, con
 //     r^2 (1 - 4e-6) > (R (1 + 1e-5) + V |dt| + e_x)^2,
 // where the relative margins cover float rounding of r^2, R and |x| (< 1e-6) and
 // e_x, V's extra term cover the hi/lo position split and the float rounding of the
-// velocities.  NaN or inf inputs make the comparison false: such pairs go to the FP64 test.
+// velocities.  R = |renc_p + renc_q|: the test squares it.  NaN or inf inputs make the comparison false: such pairs go to the FP64 test.
 __device__ __forceinline__ bool prefilter_reject(const BodyF &p, const BodyF &q, float dtf) {
     const float dx = (p.a.x - q.a.x) + (p.b.x - q.b.x);
     const float dy = (p.a.y - q.a.y) + (p.b.y - q.b.y);
@@ -94,7 +94,7 @@ __device__ __forceinline__ bool prefilter_reject(const BodyF &p, const BodyF &q,
     const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
     const float vl1 = fabsf(p.v.x - q.v.x) + fabsf(p.v.y - q.v.y) + fabsf(p.v.z - q.v.z);
     const float vhi = fmaf(vl1, 1.0f + 2e-6f, 2e-7f * (p.v.w + q.v.w));
-    const float reff = fmaf(p.a.w + q.a.w, 1.0f + 1e-5f, fmaf(vhi, dtf, 1e-13f * (p.b.w + q.b.w)));
+    const float reff = fmaf(fabsf(p.a.w + q.a.w), 1.0f + 1e-5f, fmaf(vhi, dtf, 1e-13f * (p.b.w + q.b.w)));
     return r2 * (1.0f - 4e-6f) > reff * reff;
 }
 

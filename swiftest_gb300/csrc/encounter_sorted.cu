@@ -48,15 +48,14 @@ static_assert(SQ == ENC_SORTED_TILE && SB == ENC_BOUND_TILE, "tile sizes of the 
 // a contiguous segment of the bodies 32 at a time, ranks equal digits among its lanes with
 // __match_any_sync, and counts per (digit, warp); an exclusive scan over the counts in
 // (digit, warp) order gives every warp's first slot per digit, so each pass keeps the
-// previous order among equal digits and the result is ordered by (key, index).
+// previous order among equal digits and the result is ordered by (key, index).  bits: 24, or 16
+// for short runs (two passes; the key then resolves 0.4% of the radius).
 constexpr int RS_T = 512;                 // threads of k_radial_sort
 constexpr int RS_W = RS_T / 32;           // warps of k_radial_sort
 constexpr int RS_HIST = 256 * RS_W;       // (digit, warp) counts
-__global__ void __launch_bounds__(RS_T) k_radial_sort(const int32_t *__restrict__ poff, const int32_t *__restrict__ npl,
-                                                      const double *__restrict__ r, int32_t *__restrict__ perm) {
+__device__ __forceinline__ void blk_radial_sort(int n, int o, const double *__restrict__ r, int32_t *__restrict__ perm,
+                                                int bits) {
     extern __shared__ unsigned char smem[];
-    const int s = blockIdx.x;
-    const int n = npl[s], o = poff[s];
     if (n > SORT_MAX) {
         for (int t = threadIdx.x; t < n; t += blockDim.x) perm[o + t] = o + t;
         return;
@@ -69,14 +68,14 @@ __global__ void __launch_bounds__(RS_T) k_radial_sort(const int32_t *__restrict_
         const float x0 = (float)x[0], x1 = (float)x[1], x2 = (float)x[2];
         float k = sqrtf(fmaf(x2, x2, fmaf(x1, x1, x0 * x0)));
         if (!(k >= 0.f)) k = __int_as_float(0x7f800000);
-        key[0][t] = (uint32_t)__float_as_int(k) >> 7;
+        key[0][t] = (uint32_t)__float_as_int(k) >> (31 - bits);
         idx[0][t] = (uint16_t)t;
     }
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int seg = (n + RS_W - 1) / RS_W, b0 = min(n, w * seg), b1 = min(n, b0 + seg);
     const unsigned lt = (1u << lane) - 1u;
     int in = 0;
-    for (int shift = 0; shift < 24; shift += 8, in ^= 1) {
+    for (int shift = 0; shift < bits; shift += 8, in ^= 1) {
         for (int t = threadIdx.x; t < RS_HIST; t += blockDim.x) hist[t] = 0;
         __syncthreads();  // keys of this pass written, counts cleared
         for (int b = b0; b < b1; b += 32) {  // counts of this warp's segment
@@ -133,19 +132,19 @@ __global__ void __launch_bounds__(RS_T) k_radial_sort(const int32_t *__restrict_
     }
     for (int t = threadIdx.x; t < n; t += blockDim.x) perm[o + t] = o + (int32_t)idx[in][t];
 }
+__global__ void __launch_bounds__(RS_T) k_radial_sort(const int32_t *__restrict__ poff, const int32_t *__restrict__ npl,
+                                                      const double *__restrict__ r, int32_t *__restrict__ perm) {
+    blk_radial_sort(npl[blockIdx.x], poff[blockIdx.x], r, perm, 24);
+}
 
 // One block of SB threads per bound tile (sys, first sorted position): the prefilter's
 // float copies in sorted order and the bounds (min lo, max hi, max renc), rounded outward,
 // of each 32-body half u of the tile (bounds[2 t + u]; a half without bodies gets
 // (+inf, -inf, 0), which is apart from everything).
-__global__ void __launch_bounds__(SB) k_sorted_prep(const int2 *__restrict__ tiles, const int32_t *__restrict__ poff,
-                                                    const int32_t *__restrict__ npl, const int32_t *__restrict__ perm,
-                                                    const double *__restrict__ r, const double *__restrict__ v,
-                                                    const double *__restrict__ renc, float adt, float4 *A, float4 *B,
-                                                    float4 *V, float4 *bounds) {
-    const int2 tl = tiles[blockIdx.x];
-    const int p = poff[tl.x] + tl.y + threadIdx.x;
-    const bool in = tl.y + (int)threadIdx.x < npl[tl.x];
+__device__ __forceinline__ void blk_sorted_prep(int tile, int p, bool in, const int32_t *__restrict__ perm,
+                                                const double *__restrict__ r, const double *__restrict__ v,
+                                                const double *__restrict__ renc, float adt, float4 *A, float4 *B,
+                                                float4 *V, float4 *bounds) {
     float lo = __int_as_float(0x7f800000), hi = -__int_as_float(0x7f800000), Rm = 0.f;
     if (in) {
         const int g = perm[p];
@@ -164,14 +163,27 @@ __global__ void __launch_bounds__(SB) k_sorted_prep(const int2 *__restrict__ til
         const float T = adt;
         lo = sqrtf(fmaxf(x2 * (1.0f - 1e-5f) - 2.0f * xv * T * (1.0f + 1e-5f), 0.0f)) * (1.0f - 1e-5f);
         hi = sqrtf((x2 + 2.0f * xv * T + v2 * T * T) * (1.0f + 1e-5f)) * (1.0f + 1e-5f);
-        Rm = o.a.w * (1.0f + 1e-5f);
+        Rm = fabsf(o.a.w) * (1.0f + 1e-5f);  // (R_i + R_j)^2 decides, whatever the signs
+        if (!(hi < __int_as_float(0x7f800000))) {  // NaN or infinite position or velocity: never apart
+            lo = 0.f;
+            hi = __int_as_float(0x7f800000);
+        }
     }
     for (int off = 16; off > 0; off >>= 1) {
         lo = fminf(lo, __shfl_down_sync(0xffffffffu, lo, off));
         hi = fmaxf(hi, __shfl_down_sync(0xffffffffu, hi, off));
         Rm = fmaxf(Rm, __shfl_down_sync(0xffffffffu, Rm, off));
     }
-    if ((threadIdx.x & 31) == 0) bounds[(SB / 32) * blockIdx.x + (threadIdx.x >> 5)] = make_float4(lo, hi, Rm, 0.f);
+    if ((threadIdx.x & 31) == 0) bounds[(SB / 32) * tile + (threadIdx.x >> 5)] = make_float4(lo, hi, Rm, 0.f);
+}
+__global__ void __launch_bounds__(SB) k_sorted_prep(const int2 *__restrict__ tiles, const int32_t *__restrict__ poff,
+                                                    const int32_t *__restrict__ npl, const int32_t *__restrict__ perm,
+                                                    const double *__restrict__ r, const double *__restrict__ v,
+                                                    const double *__restrict__ renc, float adt, float4 *A, float4 *B,
+                                                    float4 *V, float4 *bounds) {
+    const int2 tl = tiles[blockIdx.x];
+    blk_sorted_prep(blockIdx.x, poff[tl.x] + tl.y + threadIdx.x, tl.y + (int)threadIdx.x < npl[tl.x], perm, r, v, renc,
+                    adt, A, B, V, bounds);
 }
 
 // True when no pair across tiles P and Q can pass the FP64 test (see the file comment).
@@ -439,6 +451,134 @@ int encounter_plpl_sorted_batched(swg_ctx *c, int nsys, int nmax, const int32_t 
                                                      v, renc, dt, cap, o1, o2, olv, count, nplm);
     c->launches++;
     return launch_status(c, "encounter_sorted");
+}
+
+// ---- one pair of lists (the C entry points encounter_check_all_plpl / _pltp, TRIANGULAR)
+// The radial order only steers the cull, so a long list is ordered in segments of SEG bodies,
+// one block each, instead of one block for all: a segment's sub-tiles are wider by its share of
+// the list, the list found is the same.  4096 pl x 40,001 tp: the check's kernel 23 us with segments
+// of 2048 or 4096 (98 us with 1024), the order 14 and 23 us; the whole call 480 -> 98 us.
+constexpr int SEG = 2048, SEG_BITS = 16;
+static_assert(SEG % SB == 0, "segments are whole bound tiles");
+
+// The two lists of one check (n2 == 0: one list); per list its order, float copies and bounds.
+struct OneLists {
+    int n1, n2, seg1, nt1;
+    const double *r1, *v1, *renc1, *r2, *v2;
+    int32_t *perm1, *perm2;
+    float4 *F1, *F2, *b1, *b2;
+    int32_t *meta;  // 0, n1, n2
+    int4 *items;
+};
+
+// Blocks below seg1: segments of list 1, then of list 2.
+__global__ void __launch_bounds__(RS_T) k_one_order(OneLists l) {
+    const bool first = (int)blockIdx.x < l.seg1;
+    const int o = ((int)blockIdx.x - (first ? 0 : l.seg1)) * SEG, n = first ? l.n1 : l.n2;
+    blk_radial_sort(min(SEG, n - o), o, first ? l.r1 : l.r2, first ? l.perm1 : l.perm2, SEG_BITS);
+}
+// Blocks below nt1: bound tiles of list 1, then of list 2; and the items (receivers of list 2 by
+// chunks of list 1's sub-tiles; one list: its own receivers), one per thread of the grid.
+__global__ void __launch_bounds__(SB) k_one_prep(OneLists l, float adt, int nitems, int nchunk) {
+    const bool first = (int)blockIdx.x < l.nt1;
+    const int tile = (int)blockIdx.x - (first ? 0 : l.nt1), n = first ? l.n1 : l.n2, p = tile * SB + (int)threadIdx.x;
+    float4 *F = first ? l.F1 : l.F2;
+    blk_sorted_prep(tile, p, p < n, first ? l.perm1 : l.perm2, first ? l.r1 : l.r2, first ? l.v1 : l.v2,
+                    first ? l.renc1 : nullptr, adt, F, F + n, F + 2 * (size_t)n, first ? l.b1 : l.b2);
+    const int nr = l.n2 ? l.n2 : l.n1;
+    for (int i = blockIdx.x * SB + threadIdx.x; i < nitems; i += gridDim.x * SB) {
+        const int q0 = i / nchunk * SQ;
+        l.items[i] = make_int4(0, q0, min(SQ, nr - q0), i % nchunk);
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 3) l.meta[threadIdx.x] = threadIdx.x == 0 ? 0 : threadIdx.x == 1 ? l.n1 : l.n2;
+}
+
+namespace {
+struct OnePlan {
+    OneLists l;
+    int seg2, nt2, nitems, nchunk, pchunk;
+    size_t bytes;
+};
+OnePlan one_plan(int n1, int n2, char *base) {
+    OnePlan p;
+    auto up = [](int64_t a, int64_t b) { return (int)((a + b - 1) / b); };
+    p.l.n1 = n1;
+    p.l.n2 = n2;
+    p.l.seg1 = up(n1, SEG);
+    p.seg2 = up(n2, SEG);
+    p.l.nt1 = up(n1, SB);
+    p.nt2 = up(n2, SB);
+    // about 1024 blocks, so that the check fills the GPU
+    const int nq = up(n2 ? n2 : n1, SQ), nsub = up(n1, 32);
+    p.nchunk = n2 ? std::max(1, std::min(nsub, 1024 / std::max(nq, 1))) : 1;
+    p.pchunk = n2 ? up(nsub, p.nchunk) : 0;
+    if (n2) p.nchunk = up(nsub, p.pchunk);
+    p.nitems = nq * p.nchunk;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char *q = base + at;
+        at += (bytes + 15) & ~(size_t)15;
+        return (void *)q;
+    };
+    p.l.F1 = (float4 *)take(sizeof(float4) * 3 * (size_t)n1);
+    p.l.F2 = (float4 *)take(sizeof(float4) * 3 * (size_t)n2);
+    p.l.b1 = (float4 *)take(sizeof(float4) * 2 * (size_t)p.l.nt1);
+    p.l.b2 = (float4 *)take(sizeof(float4) * 2 * (size_t)p.nt2);
+    p.l.items = (int4 *)take(sizeof(int4) * (size_t)p.nitems);
+    p.l.meta = (int32_t *)take(16);
+    p.l.perm1 = (int32_t *)take(4 * (size_t)n1);
+    p.l.perm2 = (int32_t *)take(4 * (size_t)n2);
+    p.bytes = at;
+    return p;
+}
+}  // namespace
+
+size_t encounter_sorted_one_bytes(int n1, int n2) { return one_plan(n1, n2, nullptr).bytes; }
+
+int encounter_sorted_one(swg_ctx *c, int n1, const double *r1, const double *v1, const double *renc1, int n2,
+                         const double *r2, const double *v2, double dt, long long cap, int32_t *o1, int32_t *o2,
+                         int32_t *olv, unsigned long long *count, void *scratch) {
+    OnePlan p = one_plan(n1, n2, (char *)scratch);
+    OneLists &l = p.l;
+    l.r1 = r1;
+    l.v1 = v1;
+    l.renc1 = renc1;
+    l.r2 = r2;
+    l.v2 = v2;
+    const size_t smem = 4 * (size_t)RS_HIST + 12 * (size_t)SEG;
+    static_assert(4 * RS_HIST + 12 * SEG <= 48 * 1024, "a segment fits the default shared memory");
+    k_one_order<<<l.seg1 + p.seg2, RS_T, smem, c->stream>>>(l);
+    const float adt = (float)fabs(dt) * (1.0f + 1e-6f);  // |dt| rounded to float, then up
+    k_one_prep<<<l.nt1 + p.nt2, SB, 0, c->stream>>>(l, adt, p.nitems, p.nchunk);
+    c->launches += 2;
+    SWG_TRY(launch_status(c, "one_prep"));
+    if (n2 == 0) {
+        k_encounter_sorted<<<p.nitems, SQ, 0, c->stream>>>(l.items, l.meta, l.meta, l.perm1, l.F1, l.F1 + n1,
+                                                           l.F1 + 2 * (size_t)n1, l.b1, r1, v1, renc1, dt, cap, o1, o2,
+                                                           olv, count, nullptr);
+        c->launches++;
+        return launch_status(c, "encounter_sorted");
+    }
+    SortedSet a, b;
+    a.off = a.tbase = b.off = b.tbase = l.meta;
+    a.n = l.meta + 1;
+    b.n = l.meta + 2;
+    a.r = r1;
+    a.v = v1;
+    a.renc = renc1;
+    a.perm = l.perm1;
+    a.F = l.F1;
+    a.N = n1;
+    a.ntiles = l.nt1;
+    a.bounds = l.b1;
+    b.r = r2;
+    b.v = v2;
+    b.perm = l.perm2;
+    b.F = l.F2;
+    b.N = n2;
+    b.bounds = l.b2;
+    return pltp_sorted_batched(c, false, a, b, nullptr, p.nitems, l.items, dt, cap, o1, o2, olv, count, nullptr,
+                               p.pchunk);
 }
 
 }  // namespace swg

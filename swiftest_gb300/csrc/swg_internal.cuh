@@ -336,6 +336,14 @@ int pltp_sorted_batched(swg_ctx *c, bool discard, const SortedSet &pl, const Sor
                         int nitems, const int4 *items, double dt, long long cap, int32_t *o1, int32_t *o2,
                         int32_t *olv, unsigned long long *count, int32_t *flag, int pchunk = 0);
 
+// One TRIANGULAR check over radius-sorted tiles (encounter_sorted.cu): list 1 against itself
+// (n2 == 0, index1 < index2) or against list 2 (zero encounter radii), 1-based pairs in any order;
+// scratch of encounter_sorted_one_bytes(n1, n2).
+size_t encounter_sorted_one_bytes(int n1, int n2);
+int encounter_sorted_one(swg_ctx *c, int n1, const double *r1, const double *v1, const double *renc1, int n2,
+                         const double *r2, const double *v2, double dt, long long cap, int32_t *o1, int32_t *o2,
+                         int32_t *olv, unsigned long long *count, void *scratch);
+
 // Full check of one kind (0 plpl, 1 plplm, 2 pltp): sorted unique pairs in the
 // workspace's raw buffers; *n_out gets the count (host).  Synchronizes.
 int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1, const double *r1,
