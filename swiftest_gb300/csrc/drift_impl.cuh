@@ -326,21 +326,21 @@ __device__ inline int d_drift_one(double mu, double &rx, double &ry, double &rz,
 // reference's degree-11 sine polynomial, cos from sqrt(1 - sin^2)) and carried to the
 // polished root by their Taylor expansion to second order in dx.
 //
-// WIDE: the form for kernels that fill the GPU, which the FP64 pipe bounds: products
-// (other than those of a fused multiply-add) and square roots by integer instructions, as in
-// xd<true> (547,900 bodies: 145 -> 69 us).  Otherwise (the recursion, which waits for each
-// result) the shortest chains.
+// Divisions, the square root, conversions and compares take no FP64 instructions (fp64_exact.cuh,
+// the same bits).  WIDE: the form for kernels that fill the GPU, which the FP64 pipe bounds: the
+// products (other than those of a fused multiply-add) by integer instructions too, as in
+// xd<true> (547,900 bodies: 145 -> 77 us).
 template <bool WIDE>
 __device__ __forceinline__ double d_mul(double a, double b) {
     return WIDE ? xmul(a, b) : a * b;
 }
 
 template <bool WIDE>
-__device__ inline void d_kepmd_fast(double dm, double es, double ec, float dmf, float esf, float ecf, double &x,
-                                    double &s, double &c) {
+__device__ inline void d_kepmd_fast(double dm, double es, double ec, double &x, double &s, double &c) {
     const double a0 = 39916800.0, a1 = 6652800.0, a2 = 332640.0, a3 = 7920.0, a4 = 110.0;
     const double inv_a0 = 1.0 / 39916800.0;
     // FP32 root: sin x as its Taylor series to x^11 in nested form
+    const float dmf = x_to_float_rn(dm), esf = x_to_float_rn(es), ecf = x_to_float_rn(ec);
     const float fac1 = 1.0f / (1.0f - ecf);
     const float q = fac1 * dmf;
     const float fac2 = fmaf(esf * esf, fac1, -ecf * (1.0f / 3.0f));
@@ -384,36 +384,27 @@ __device__ inline void d_drift_dan_fast(double mu, double &rx0, double &ry0, dou
                                         double &vz0, double dt0, int &iflag, double inv_mu0 = 0.0) {
     iflag = 0;
     const double r2 = fma(rz0, rz0, fma(ry0, ry0, d_mul<WIDE>(rx0, rx0)));
-    double r0, inv_r0;
-    if (WIDE) {
-        r0 = xsqrt(r2);
-        inv_r0 = xdiv(1.0, r0);
-    } else {
-        inv_r0 = x_rsqrt(r2);
-        r0 = r2 * inv_r0;
-    }
+    const double inv_r0 = rsqrt(r2);
     const double v0s = fma(vz0, vz0, fma(vy0, vy0, d_mul<WIDE>(vx0, vx0)));
     const double u = fma(rz0, vz0, fma(ry0, vy0, d_mul<WIDE>(rx0, vx0)));
     const double alpha = fma(2.0 * mu, inv_r0, -v0s);
     if (x_greater(alpha, 0.0)) {
         const double inv_mu = inv_mu0 != 0.0 ? inv_mu0 : xdiv(1.0, mu);
-        const double rsa = WIDE ? xdiv(1.0, xsqrt(alpha)) : x_rsqrt(alpha);
-        const double rsa2 = d_mul<WIDE>(rsa, rsa);
-        const double a = d_mul<WIDE>(mu, rsa2);                   // mu / alpha
-        const double ia = d_mul<WIDE>(alpha, inv_mu);             // 1 / a
-        const double en = d_mul<WIDE>(d_mul<WIDE>(alpha, rsa), ia);  // sqrt(mu / a^3)
-        const double inv_en = d_mul<WIDE>(a, rsa);
-        const double ec = fma(-r0, ia, 1.0);
-        const double es = d_mul<WIDE>(d_mul<WIDE>(u, rsa), ia);   // u / (en a^2)
+        const double rsa = rsqrt(alpha);
+        const double a = d_mul<WIDE>(d_mul<WIDE>(mu, rsa), rsa);                                // mu / alpha
+        const double ia = d_mul<WIDE>(alpha, inv_mu);                                           // 1 / a
+        const double en = d_mul<WIDE>(d_mul<WIDE>(alpha, d_mul<WIDE>(alpha, rsa)), inv_mu);     // sqrt(mu / a^3)
+        const double inv_en = d_mul<WIDE>(mu, d_mul<WIDE>(d_mul<WIDE>(rsa, rsa), rsa));
+        const double ec = fma(-d_mul<WIDE>(r2, inv_r0), ia, 1.0);
+        const double es = d_mul<WIDE>(d_mul<WIDE>(d_mul<WIDE>(u, inv_en), ia), ia);
+        const double esq = fma(ec, ec, d_mul<WIDE>(es, es));
         const double den = d_mul<WIDE>(dt0, en);
         const double dm = less_than_4(den) ? den : fma(-(double)(int)(den * (1.0 / TWOPI)), TWOPI, den);
-        // the branch limits in FP32: either side of them both branches are valid
-        const float dmf = x_to_float(dm), esf = x_to_float(es), ecf = x_to_float(ec);
-        const float esq = fmaf(ecf, ecf, esf * esf), dm2 = dmf * dmf;
-        if (esq < (float)E2MAX && dm2 < (float)DM2MAX && esq * dm2 < (float)E2DM2MAX) {
+        const double dm2 = d_mul<WIDE>(dm, dm);
+        if (x_less(esq, E2MAX) && x_less(dm2, DM2MAX) && x_less(d_mul<WIDE>(esq, dm2), E2DM2MAX)) {
             const double dt = d_mul<WIDE>(dm, inv_en);
             double xkep, s, c;
-            d_kepmd_fast<WIDE>(dm, es, ec, dmf, esf, ecf, xkep, s, c);
+            d_kepmd_fast<WIDE>(dm, es, ec, xkep, s, c);
             const double c1 = xsub(c, 1.0);
             const double fchk = xsub(fma(-es, c1, fma(-ec, s, xkep)), dm);
             if (x_greater(x_abs(fchk), DANBYB)) {
@@ -425,7 +416,7 @@ __device__ inline void d_drift_dan_fast(double mu, double &rx0, double &ry0, dou
             const double ar = d_mul<WIDE>(a, inv_r0);
             const double f = fma(ar, c1, 1.0);
             const double g = fma(xsub(s, xkep), inv_en, dt);
-            const double fdot = d_mul<WIDE>(-d_mul<WIDE>(d_mul<WIDE>(ar, en), s), inv_fp);
+            const double fdot = -d_mul<WIDE>(d_mul<WIDE>(d_mul<WIDE>(ar, inv_fp), en), s);
             const double gdot = fma(c1, inv_fp, 1.0);
             const double rx = fma(rx0, f, d_mul<WIDE>(vx0, g)), ry = fma(ry0, f, d_mul<WIDE>(vy0, g)),
                          rz = fma(rz0, f, d_mul<WIDE>(vz0, g));

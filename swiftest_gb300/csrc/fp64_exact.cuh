@@ -162,7 +162,7 @@ __device__ __forceinline__ double x_div(const XNum &g, double p, bool &bad) {
 }
 
 // Conversions by integer instructions (the conversion instructions take the FP64 pipe): a
-// double cut to its leading 24 bits, and a normal (or zero) float as a double.
+// double cut to its leading 24 bits, a float as a double, and the rounded float of a double.
 __device__ __forceinline__ float x_to_float(double x) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
     if (!x_ok(hi & 0x7fffffff)) return ((hi & 0x7fffffff) | lo) == 0 ? 0.0f : (float)x;
@@ -170,7 +170,16 @@ __device__ __forceinline__ float x_to_float(double x) {
 }
 __device__ __forceinline__ double x_to_double(float f) {
     const int b = __float_as_int(f), m = b & 0x7fffffff;
+    if (m < 0x800000 && m != 0) return (double)f;  // subnormal
     return __hiloint2double((b & 0x80000000) | (m == 0 ? 0 : (m >> 3) + ((1023 - 127) << 20)), b << 29);
+}
+// (float)x, rounded to nearest even
+__device__ __forceinline__ float x_to_float_rn(double x) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    if (!x_ok(hi & 0x7fffffff)) return (float)x;
+    const unsigned f = __funnelshift_l(lo, (hi & 0x7fffffff) - ((1023 - 127) << 20), 3);
+    const unsigned up = ((lo & 0x1fffffffu) + 0x0fffffffu + (f & 1u)) >> 29;
+    return __int_as_float((int)((f + up) | (hi & 0x80000000)));
 }
 
 __device__ __forceinline__ double x_half(double a) {
