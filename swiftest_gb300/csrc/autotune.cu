@@ -46,7 +46,7 @@ void load_locked() {
     char key[512];
     int v = 0;
     while (std::fscanf(f, "%511s %d", key, &v) == 2)
-        if (v >= 0 && v < 16) g_tune[key] = v;  // callers check the range of their own keys
+        if (v >= 0 && v < 512) g_tune[key] = v;  // packed shapes; callers check the range of their own keys
     std::fclose(f);
 }
 
