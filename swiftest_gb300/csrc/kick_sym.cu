@@ -574,46 +574,91 @@ __global__ void k_kick_sym_item_flags(int nitems, const int4 *__restrict__ items
 // kernel.  grp: tiles per row group (1: one-row items, whose pair slot (g, K) is
 // pair_slot(g, K, nt)); a group g holds nt - g grp - 1 pair slots and one item per strip
 // of its tiles J >= g grp, each item grp receiver slots.
-__global__ void k_kick_sym_reduce(int64_t n, const int32_t *__restrict__ psys, const int32_t *__restrict__ poff,
-                                  const int32_t *__restrict__ npl, const int32_t *__restrict__ sbase,
-                                  const float *__restrict__ rpart, const float *__restrict__ ppart,
-                                  double *__restrict__ acc, int acc_is_zero, const int32_t *__restrict__ sys_flag,
-                                  int phase, int strip, int ts, int grp) {
+// One thread per body and component (blockIdx.y), the slots' loads batched ahead of their
+// additions: both keep the additions' order.  A thread per body with its three components in
+// turn waited for each slot (65,536 bodies: 323 us for 300 MB, now 84 us).
+constexpr int RED_B = 8;  // slots per batch of loads
+// Items of the row groups before group gK: sum over g < gK of ceil((nt - g grp) / strip), grp and
+// strip powers of two.
+__device__ __forceinline__ int rows_before(int nt, int gK, int strip_log2, int grp_log2) {
+    if (strip_log2 < grp_log2)  // ceil(nt / strip) - g grp / strip
+        return gK * ((nt + (1 << strip_log2) - 1) >> strip_log2) - ((gK * (gK - 1) / 2) << (grp_log2 - strip_log2));
+    // ceil((m - g) / S) with m = ceil(nt / grp), S = strip / grp: F(m) - F(m - gK), F(x) the sum over 1 .. x
+    const int sl = strip_log2 - grp_log2, m = (nt + (1 << grp_log2) - 1) >> grp_log2;
+    auto F = [&](int x) {
+        const int q = x >> sl, r = x - (q << sl);
+        return ((q * (q + 1) / 2) << sl) + r * (q + 1);
+    };
+    return F(m) - F(m - gK);
+}
+__global__ void __launch_bounds__(256, 6) k_kick_sym_reduce(int64_t n, const int32_t *__restrict__ psys,
+                                                         const int32_t *__restrict__ poff,
+                                                         const int32_t *__restrict__ npl,
+                                                         const int32_t *__restrict__ sbase,
+                                                         const float *__restrict__ rpart,
+                                                         const float *__restrict__ ppart, double *__restrict__ acc,
+                                                         int acc_is_zero, const int32_t *__restrict__ sys_flag,
+                                                         int phase, int strip_log2, int ts_log2, int grp_log2) {
     const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int c = blockIdx.y;
     if (b >= n) return;
     const int s = psys ? psys[b] : 0;
     if (sys_flag && sys_flag[s] != phase) return;
     const int i = (int)(b - poff[s]);
-    const int nt = (npl[s] + ts - 1) / ts, K = i / ts, l = i % ts, gK = K / grp;
-    FF fx{0.f, 0.f}, fy{0.f, 0.f}, fz{0.f, 0.f};
-    float lx = 0.f, ly = 0.f, lz = 0.f;
-    int pslot = sbase[2 * s + 1];  // first pair slot of group g
-    int row = 0;                   // items of the groups before gK
-    for (int g = 0; g <= gK; g++) {
-        const int I0 = g * grp;
-        if (I0 < K) {
-            const float *o = ppart + (size_t)(pslot + K - I0 - 1) * 3 * ts;
-            ff_add3(fx, fy, fz, o[l], o[ts + l], o[2 * ts + l]);
+    const int ts = 1 << ts_log2, grp = 1 << grp_log2, strip = 1 << strip_log2;  // powers of two
+    const int nt = (npl[s] + ts - 1) >> ts_log2, K = i >> ts_log2, l = i & (ts - 1), gK = K >> grp_log2;
+    FF f{0.f, 0.f};
+    float lo = 0.f;
+    // pair slots (g, K) of the groups with I0 = g grp < K: group g's are nt - I0 - 1 - grp slots
+    // on from group g - 1's
+    const int np = (K + grp - 1) >> grp_log2;
+    const float *o = ppart + ((size_t)(sbase[2 * s + 1] + K - 1) * 3 + c) * ts + l;
+    ptrdiff_t step = (ptrdiff_t)(nt - 1 - grp) * 3 * ts;
+    const int dstep = 3 * ts << grp_log2;
+    int g = 0;
+    for (; g + RED_B <= np; g += RED_B) {
+        float v[RED_B];
+#pragma unroll
+        for (int u = 0; u < RED_B; u++) {
+            v[u] = *o;
+            o += step;
+            step -= dstep;
         }
-        if (g < gK) {
-            pslot += nt - I0 - 1;
-            row += (nt - I0 + strip - 1) / strip;
+#pragma unroll
+        for (int u = 0; u < RED_B; u++) ff_add(f, v[u]);
+    }
+    for (; g < np; g++) {
+        ff_add(f, *o);
+        o += step;
+        step -= dstep;
+    }
+    const int row = rows_before(nt, gK, strip_log2, grp_log2);
+    const int nm = (nt - gK * grp + strip - 1) >> strip_log2;
+    const size_t rstep = (size_t)grp * 6 * ts;
+    o = rpart + ((size_t)(sbase[2 * s] + row * grp + K - gK * grp) * 6 + 2 * c) * ts + l;
+    int m = 0;
+    for (; m + RED_B / 2 <= nm; m += RED_B / 2) {
+        float v[RED_B / 2], w[RED_B / 2];
+#pragma unroll
+        for (int u = 0; u < RED_B / 2; u++) {
+            v[u] = o[0];
+            w[u] = o[ts];
+            o += rstep;
+        }
+#pragma unroll
+        for (int u = 0; u < RED_B / 2; u++) {
+            ff_add(f, v[u]);
+            lo += w[u];
         }
     }
-    for (int m = 0; m < (nt - gK * grp + strip - 1) / strip; m++) {
-        const float *o = rpart + ((size_t)(sbase[2 * s] + (row + m) * grp + K - gK * grp)) * 6 * ts;
-        ff_add3(fx, fy, fz, o[l], o[2 * ts + l], o[4 * ts + l]);
-        lx += o[ts + l];
-        ly += o[3 * ts + l];
-        lz += o[5 * ts + l];
+    for (; m < nm; m++) {
+        ff_add(f, o[0]);
+        lo += o[ts];
+        o += rstep;
     }
-    const double sx = (double)fx.hi + ((double)fx.lo + (double)lx);
-    const double sy = (double)fy.hi + ((double)fy.lo + (double)ly);
-    const double sz = (double)fz.hi + ((double)fz.lo + (double)lz);
-    double *a = acc + 3 * b;
-    a[0] = (acc_is_zero ? 0.0 : a[0]) + sx;
-    a[1] = (acc_is_zero ? 0.0 : a[1]) + sy;
-    a[2] = (acc_is_zero ? 0.0 : a[2]) + sz;
+    const double sum = (double)f.hi + ((double)f.lo + (double)lo);
+    double *a = acc + 3 * b + c;
+    *a = (acc_is_zero ? 0.0 : *a) + sum;
 }
 
 }  // namespace
@@ -752,8 +797,13 @@ int kick_mixed_sym_reduce(swg_ctx *c, int strip, int64_t n, const int32_t *psys,
                           const int32_t *npl, const int32_t *sbase, const float *rpart, const float *ppart,
                           double *acc, int acc_is_zero, const int32_t *sys_flag, int phase, int tile, int group) {
     if (n <= 0) return SWG_OK;
-    k_kick_sym_reduce<<<(int)((n + 255) / 256), 256, 0, c->stream>>>(n, psys, poff, npl, sbase, rpart, ppart, acc,
-                                                                      acc_is_zero, sys_flag, phase, strip, tile, group);
+    auto log2i = [](int v) {
+        int l = 0;
+        while ((1 << l) < v) l++;
+        return l;
+    };
+    k_kick_sym_reduce<<<dim3((unsigned)((n + 255) / 256), 3), 256, 0, c->stream>>>(
+        n, psys, poff, npl, sbase, rpart, ppart, acc, acc_is_zero, sys_flag, phase, log2i(strip), log2i(tile), log2i(group));
     c->launches++;
     return launch_status(c, "kick_sym_reduce");
 }
