@@ -1889,7 +1889,8 @@ int whm_kick_vh_pl(swg_ensemble *e, double dt, int lbeg) {
 // system at rp, plus the pl-tp pair kick
 int whm_accel_tp(swg_ensemble *e, int lbeg, unsigned *head = nullptr) {
     swg_ctx *c = e->c;
-    const double *rp = lbeg ? e->rbeg : e->rend;
+    // the end positions: rend, or (the same values) rh before the pl's closing kick copies it there
+    const double *rp = lbeg ? e->rbeg : exact(e) ? e->rh : e->rend;
     if (!head) head = e->head;
     k_ens_whm_ah0<<<e->nsys, 256, 0, c->stream>>>(e->poff, e->npl, e->Gmass, rp, e->whm_ah0, exact(e));
     SWG_TRY(L(c, "ens_whm_ah0"));
@@ -1921,6 +1922,7 @@ int whm_ens_step(swg_ensemble *e, double dt) {
     // stream beside the pl half-steps; the closing accelerations (at the pl end positions
     // and their partner split) wait for the pl.  Each body's arithmetic is unchanged.
     const bool split = !first_tp && !e->prof.on && e->NPL > 0 && e->NTP > 0;
+    bool early = false;  // the closing tp accelerations start before the pl's
     unsigned *head_tp = e->head + 1;
     if (split) {
         SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_fork, c->stream), "fork"));
@@ -1943,10 +1945,15 @@ int whm_ens_step(swg_ensemble *e, double dt) {
                                                                              e->whm_fail);
         SWG_TRY(L(c, "ens_whm_drift_status"));
         SWG_TRY(whm_coord(e, WHM_J2H));
+        // FP64 path: the test particles' closing accelerations read only the pl positions, which
+        // are final here, so they start beside the pl accelerations (whose running sums
+        // leave most of the GPU idle); the mixed path's also read the pl kick's partner split
+        early = split && exact(e);
+        if (early) SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_drift, c->stream), "pl done"));
         SWG_TRY(whm_kick_vh_pl(e, dth, 0));
     }
     if (split) {
-        SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_drift, c->stream), "pl done"));
+        if (!early) SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_drift, c->stream), "pl done"));
         SWG_TRY(cuda_status(c, cudaStreamWaitEvent(e->side, e->ev_drift, 0), "pl done"));
         SWG_TRY(on_stream(c, e->side, [&] { return whm_kick_vh_tp(e, dth, 0, false, head_tp); }));
         SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_join, e->side), "join"));

@@ -1711,10 +1711,11 @@ static __device__ __forceinline__ void whm_running(WhmScratch &sh, int m, int cn
     if (exact) {
         if (threadIdx.x < m) {
             const int c = threadIdx.x;
-            double s = sh.run[c];
+            double s = sh.run[c], *v = sh.t[c];
+#pragma unroll 8
             for (int q = 0; q < cnt; q++) {
-                s = s + sh.t[c][q];
-                sh.t[c][q] = s;
+                s = s + v[q];
+                v[q] = s;
             }
             sh.run[c] = s;
         }
@@ -1748,8 +1749,8 @@ static __device__ void blk_whm_h2j(int n, const double *Gm, const double *eta, c
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             const int i = c0 + q;
             for (int d = 0; d < 3; d++) {
-                const double cap = sh.t[d][q] / eta[i - 1];
-                const double capv = sh.t[3 + d][q] / eta[i - 1];
+                const double cap = xdiv(sh.t[d][q], eta[i - 1]);
+                const double capv = xdiv(sh.t[3 + d][q], eta[i - 1]);
                 xj[3 * i + d] = rh[3 * i + d] - cap;
                 vj[3 * i + d] = vh[3 * i + d] - capv;
             }
@@ -1771,8 +1772,8 @@ static __device__ void blk_whm_j2h(int n, const double *Gm, const double *eta, c
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             const int k = c0 + q - 1;
             for (int d = 0; d < 3; d++) {
-                sh.t[d][q] = Gm[k] * xj[3 * k + d] / eta[k];
-                sh.t[3 + d][q] = Gm[k] * vj[3 * k + d] / eta[k];
+                sh.t[d][q] = xdiv(Gm[k] * xj[3 * k + d], eta[k]);
+                sh.t[3 + d][q] = xdiv(Gm[k] * vj[3 * k + d], eta[k]);
             }
         }
         whm_running(sh, 6, cnt, exact);
@@ -1802,7 +1803,7 @@ static __device__ void blk_whm_vh2vj(int n, const double *Gm, const double *eta,
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             const int i = c0 + q;
             for (int d = 0; d < 3; d++) {
-                const double capv = sh.t[d][q] / eta[i - 1];
+                const double capv = xdiv(sh.t[d][q], eta[i - 1]);
                 vj[3 * i + d] = vh[3 * i + d] - capv;
             }
         }
@@ -1810,41 +1811,130 @@ static __device__ void blk_whm_vh2vj(int n, const double *Gm, const double *eta,
 }
 // whm_kick_getacch_ah0 (whm_kick.f90:125-149): ah0 = -sum mu_i rhp_i / |rhp_i|^3 in index
 // order, into out[3] (shared or global), visible to the block on return
+static __device__ __forceinline__ void whm_ah0_term(const double *mu, const double *rhp, int i, double *t) {
+    const double r2 = rhp[3 * i] * rhp[3 * i] + rhp[3 * i + 1] * rhp[3 * i + 1] + rhp[3 * i + 2] * rhp[3 * i + 2];
+    const double ir3h = xdiv(1.0, r2 * xsqrt(r2));
+    const double fac = mu[i] * ir3h;
+    for (int d = 0; d < 3; d++) t[d] = -(fac * rhp[3 * i + d]);  // a - b == a + (-b)
+}
 static __device__ void blk_whm_ah0(const double *mu, const double *rhp, int n, double *out, WhmScratch &sh,
                                    bool exact) {
+    if (exact) {
+        static_assert(sizeof(SumScratch) <= sizeof(WhmScratch), "the serial sums' workspace fits");
+        SumScratch &ss = *reinterpret_cast<SumScratch *>(&sh);
+        blk_serial_sums<3>(n, false, [&](int i, double *t) { whm_ah0_term(mu, rhp, i, t); return true; }, ss);
+        if (threadIdx.x < 3) out[threadIdx.x] = ss.sum[threadIdx.x];
+        __syncthreads();
+        return;
+    }
     if (threadIdx.x < 3) sh.run[threadIdx.x] = 0.0;
     for (int c0 = 0; c0 < n; c0 += WCH) {
         const int cnt = min(WCH, n - c0);
         __syncthreads();
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-            const int i = c0 + q;
-            const double r2 =
-                rhp[3 * i] * rhp[3 * i] + rhp[3 * i + 1] * rhp[3 * i + 1] + rhp[3 * i + 2] * rhp[3 * i + 2];
-            const double ir3h = 1.0 / (r2 * sqrt(r2));
-            const double fac = mu[i] * ir3h;
-            for (int d = 0; d < 3; d++) sh.t[d][q] = -(fac * rhp[3 * i + d]);  // a - b == a + (-b)
+            double t[3];
+            whm_ah0_term(mu, rhp, c0 + q, t);
+            for (int d = 0; d < 3; d++) sh.t[d][q] = t[d];
         }
-        whm_running(sh, 3, cnt, exact);
+        whm_running(sh, 3, cnt, false);
     }
     __syncthreads();
     if (threadIdx.x < 3) out[threadIdx.x] = sh.run[threadIdx.x];
     __syncthreads();
 }
+
+// set_ir3j of body i (whm_util.f90:117-140)
+static __device__ __forceinline__ void whm_ir3(const double *x, double &ir3) {
+    const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+    const double ir = xdiv(1.0, xsqrt(r2));
+    ir3 = xdiv(ir, r2);
+}
+
+// blk_whm_accel_pl of the FP64 path.  The three running sums (ah0; etaj = GMcb + the masked
+// Gm[i-1]; ah2, whose terms need etaj) go through the bodies together, ah2 one chunk behind: seven
+// lanes of one warp add in the same instruction, so a body costs one addition's latency (64
+// cycles) instead of three.  A masked-out body's terms are -0.0, which leaves the sums as they are.
+static __device__ void blk_whm_accel_exact(int n, const double *Gm, double GMcb, const double *rh, const double *xj,
+                                           const int32_t *lmask, double *ir3h, double *ir3j, double *ah,
+                                           WhmScratch &sh) {
+    constexpr int W = WCH / 2;  // bodies per chunk; chunk k sits in half k & 1 of the arrays
+    const int chunks = (n - 1 + W - 1) / W, lane = threadIdx.x;
+    double s = lane == 3 ? GMcb : 0.0;  // lanes 0-2 ah0, 3 etaj, 4-6 ah2
+    if (threadIdx.x == 0) {
+        whm_ir3(rh, ir3h[0]);
+        whm_ir3(xj, ir3j[0]);
+    }
+    for (int k = 0; k <= chunks; k++) {
+        const int at = (k & 1) * W, bt = W - at;  // halves of chunks k and k - 1
+        for (int q = threadIdx.x; q < W; q += blockDim.x) {
+            const int i = 1 + k * W + q;
+            if (i < n) {
+                whm_ir3(&rh[3 * i], ir3h[i]);
+                whm_ir3(&xj[3 * i], ir3j[i]);
+                double t[3];
+                whm_ah0_term(Gm, rh, i, t);
+                for (int d = 0; d < 3; d++) sh.t[d][at + q] = t[d];
+                sh.e[at + q] = lmask[i] ? Gm[i - 1] : -0.0;
+            }
+            const int j = i - W;
+            if (k > 0 && j < n) {
+                const bool on = lmask[j] != 0;
+                const double fac = on ? xdiv(Gm[j] * GMcb * ir3j[j], sh.e[bt + q]) : 0.0;
+                for (int d = 0; d < 3; d++) sh.t[3 + d][q] = on ? fac * xj[3 * j + d] : -0.0;
+            }
+        }
+        __syncthreads();
+        if (lane < 7) {
+            const int first = 1 + (lane < 4 ? k : k - 1) * W, cnt = first < 1 ? 0 : max(0, min(W, n - first));
+            double *v = lane < 3 ? &sh.t[lane][at] : lane == 3 ? &sh.e[at] : &sh.t[lane - 1][0];
+#pragma unroll 8
+            for (int q = 0; q < cnt; q++) {
+                s = s + v[q];
+                if (lane >= 3) v[q] = s;
+            }
+        }
+        __syncthreads();
+        if (k > 0)  // ah2 of chunk k - 1, kept in ah until ah0 is known
+            for (int q = threadIdx.x; q < W; q += blockDim.x) {
+                const int j = 1 + (k - 1) * W + q;
+                if (j < n)
+                    for (int d = 0; d < 3; d++) ah[3 * j + d] = sh.t[3 + d][q];
+            }
+        __syncthreads();
+    }
+    if (lane < 3) sh.run[lane] = s;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const bool on = i >= 1 && lmask[i];
+        for (int d = 0; d < 3; d++) {
+            double a = 0.0 + sh.run[d];
+            if (on) {
+                const double ah1j = xj[3 * i + d] * ir3j[i];
+                const double ah1h = rh[3 * i + d] * ir3h[i];
+                a = a + GMcb * (ah1j - ah1h);
+                a = a + ah[3 * i + d];
+            }
+            ah[3 * i + d] = a;
+        }
+    }
+    __syncthreads();
+}
+
 // whm_kick_getacch_pl (whm_kick.f90:14-67) up to accel_int, with set_ir3j (whm_util.f90:117-140),
-// ah1 (:152-179) and ah2 (:182-215), whole block
+// ah1 (:152-179) and ah2 (:182-215), whole block; ah is zero at entry
 static __device__ void blk_whm_accel_pl(int n, const double *Gm, double GMcb, const double *rh, const double *xj,
                                         const int32_t *lmask, double *ir3h, double *ir3j, double *ah,
                                         WhmScratch &sh, bool exact) {
+    if (exact) {
+        blk_whm_accel_exact(n, Gm, GMcb, rh, xj, lmask, ir3h, ir3j, ah, sh);
+        return;
+    }
     __shared__ double s_ah0[3];
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double r2 = rh[3 * i] * rh[3 * i] + rh[3 * i + 1] * rh[3 * i + 1] + rh[3 * i + 2] * rh[3 * i + 2];
-        double ir = 1.0 / sqrt(r2);
-        ir3h[i] = ir / r2;
-        r2 = xj[3 * i] * xj[3 * i] + xj[3 * i + 1] * xj[3 * i + 1] + xj[3 * i + 2] * xj[3 * i + 2];
-        ir = 1.0 / sqrt(r2);
-        ir3j[i] = ir / r2;
+        whm_ir3(&rh[3 * i], ir3h[i]);
+        whm_ir3(&xj[3 * i], ir3j[i]);
     }
-    blk_whm_ah0(Gm + 1, rh + 3, n - 1, s_ah0, sh, exact);
+    blk_whm_ah0(Gm + 1, rh + 3, n - 1, s_ah0, sh, false);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         for (int d = 0; d < 3; d++) ah[3 * i + d] = ah[3 * i + d] + s_ah0[d];
         if (i >= 1 && lmask[i])
@@ -1865,22 +1955,11 @@ static __device__ void blk_whm_accel_pl(int n, const double *Gm, double GMcb, co
             sh.e[q] = Gm[c0 + q - 1];
         }
         __syncthreads();
-        if (exact) {
-            if (threadIdx.x == 0) {
-                double etaj = sh.run[3];
-                for (int q = 0; q < cnt; q++) {
-                    if (!sh.m[q]) continue;
-                    etaj = etaj + sh.e[q];
-                    sh.e[q] = etaj;
-                }
-                sh.run[3] = etaj;
-            }
-        } else {  // unmasked bodies add zero; their running values are not used
-            for (int q = threadIdx.x; q < cnt; q += blockDim.x)
-                if (!sh.m[q]) sh.e[q] = 0.0;
-            __syncthreads();
-            if (threadIdx.x < 32) warp_seg_scan(sh.e, cnt, sh.run[3]);
-        }
+        // unmasked bodies add zero; their running values are not used
+        for (int q = threadIdx.x; q < cnt; q += blockDim.x)
+            if (!sh.m[q]) sh.e[q] = 0.0;
+        __syncthreads();
+        if (threadIdx.x < 32) warp_seg_scan(sh.e, cnt, sh.run[3]);
         __syncthreads();
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             if (!sh.m[q]) {
@@ -1888,22 +1967,11 @@ static __device__ void blk_whm_accel_pl(int n, const double *Gm, double GMcb, co
                 continue;
             }
             const int i = c0 + q;
-            const double fac = Gm[i] * GMcb * ir3j[i] / sh.e[q];
+            const double fac = xdiv(Gm[i] * GMcb * ir3j[i], sh.e[q]);
             for (int d = 0; d < 3; d++) sh.t[d][q] = fac * xj[3 * i + d];
         }
         __syncthreads();
-        if (exact) {
-            if (threadIdx.x < 3) {
-                const int d = threadIdx.x;
-                double a2 = sh.run[d];
-                for (int q = 0; q < cnt; q++) {
-                    if (!sh.m[q]) continue;
-                    a2 = a2 + sh.t[d][q];
-                    sh.t[d][q] = a2;
-                }
-                sh.run[d] = a2;
-            }
-        } else if (threadIdx.x < 96) {
+        if (threadIdx.x < 96) {
             const int d = threadIdx.x >> 5;
             warp_seg_scan(sh.t[d], cnt, sh.run[d]);
         }
