@@ -72,8 +72,15 @@ __device__ void blk_serial_sums(int n, bool reverse, TermFn term_fn, SumScratch 
         } else if (c < NC) {
             const double *t = sh.t[k & 1][c];
             const int cnt = min(SCH, n - k * SCH);
-#pragma unroll 16
-            for (int q = 0; q < cnt; q++) s = s + t[q];
+            int q = 0;
+            for (; q + 16 <= cnt; q += 16) {  // loads ahead of the chain of additions
+                double x[16];
+#pragma unroll
+                for (int u = 0; u < 16; u++) x[u] = t[q + u];
+#pragma unroll
+                for (int u = 0; u < 16; u++) s = s + x[u];
+            }
+            for (; q < cnt; q++) s = s + t[q];
         }
     }
     if (w == 0 && c < NC) sh.sum[c] = s;
@@ -1703,25 +1710,75 @@ static __device__ __forceinline__ void warp_seg_scan(double *v, int cnt, double 
     if (lane == 0) run = base + total;
 }
 
-// t[c][q] <- run[c] + t[c][0] + ... + t[c][q] for c < m.  exact: one thread per component
-// adds in index order (the reference's operands and order); otherwise one warp per
-// component runs warp_seg_scan (blockDim >= 32 m).
-static __device__ __forceinline__ void whm_running(WhmScratch &sh, int m, int cnt, bool exact) {
+// t[c][q] <- run[c] + t[c][0] + ... + t[c][q] for c < m (mixed path): one warp per component runs
+// warp_seg_scan (blockDim >= 32 m).
+static __device__ __forceinline__ void whm_running(WhmScratch &sh, int m, int cnt) {
     __syncthreads();
-    if (exact) {
-        if (threadIdx.x < m) {
-            const int c = threadIdx.x;
-            double s = sh.run[c], *v = sh.t[c];
-#pragma unroll 8
-            for (int q = 0; q < cnt; q++) {
-                s = s + v[q];
-                v[q] = s;
-            }
-            sh.run[c] = s;
-        }
-    } else if ((int)(threadIdx.x >> 5) < m) {
+    if ((int)(threadIdx.x >> 5) < m) {
         const int c = threadIdx.x >> 5;
         warp_seg_scan(sh.t[c], cnt, sh.run[c]);
+    }
+    __syncthreads();
+}
+
+// v[q] <- s + v[0] + ... + v[q] in order (store; else only the sum), by one lane: batches of eight
+// loads ahead of their additions, so that the chain is the additions' alone.
+static __device__ __forceinline__ double serial_running(double *v, int cnt, double s, bool store) {
+    int q = 0;
+    for (; q + 8 <= cnt; q += 8) {
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = v[q + u];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            s = s + x[u];
+            x[u] = s;
+        }
+        if (store) {
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[q + u] = x[u];
+        }
+    }
+    for (; q < cnt; q++) {
+        s = s + v[q];
+        if (store) v[q] = s;
+    }
+    return s;
+}
+
+// Running sums of the FP64 path's coordinate conversions: form(i, t) writes body i's M terms (i =
+// 1 .. n-1), which are added in index order from zero, and use(i, run) gets the sums including
+// body i's.  Lane c of warp 0 adds component c of chunk k (64 cycles a body) while the other warps
+// form chunk k + 1 and use chunk k - 1; three buffers, one barrier per chunk.
+template <int M, class Form, class Use>
+static __device__ __forceinline__ void whm_exact_running(int n, Form form, Use use, WhmScratch &sh) {
+    constexpr int W = 160;
+    static_assert(3 * W <= WCH && M <= 6, "three chunks fit");
+    const int chunks = (n - 1 + W - 1) / W, others = blockDim.x - 32;
+    double s = 0.0;
+    for (int k = -1; k <= chunks; k++) {
+        __syncthreads();
+        if (threadIdx.x >= 32) {
+            const int a = (k + 1) % 3 * W, b = (k + 2) % 3 * W;  // buffers of chunks k + 1 and k - 1
+            for (int q = threadIdx.x - 32; q < W; q += others) {
+                const int i = 1 + (k + 1) * W + q, j = i - 2 * W;
+                double t[M];
+                if (i < n) {
+                    form(i, t);
+#pragma unroll
+                    for (int c = 0; c < M; c++) sh.t[c][a + q] = t[c];
+                }
+                if (k > 0 && j < n) {
+#pragma unroll
+                    for (int c = 0; c < M; c++) t[c] = sh.t[c][b + q];
+                    use(j, t);
+                }
+            }
+        } else if (k >= 0 && threadIdx.x < M) {
+            double *v = &sh.t[threadIdx.x][k % 3 * W];
+            const int cnt = min(W, n - 1 - k * W);
+            s = serial_running(v, cnt, s, true);
+        }
     }
     __syncthreads();
 }
@@ -1734,6 +1791,24 @@ static __device__ void blk_whm_h2j(int n, const double *Gm, const double *eta, c
         xj[threadIdx.x] = rh[threadIdx.x];
         vj[threadIdx.x] = vh[threadIdx.x];
     }
+    if (exact) {
+        whm_exact_running<6>(
+            n,
+            [&](int i, double *t) {
+                for (int d = 0; d < 3; d++) {
+                    t[d] = Gm[i - 1] * rh[3 * (i - 1) + d];
+                    t[3 + d] = Gm[i - 1] * vh[3 * (i - 1) + d];
+                }
+            },
+            [&](int i, const double *run) {
+                for (int d = 0; d < 3; d++) {
+                    xj[3 * i + d] = rh[3 * i + d] - xdiv(run[d], eta[i - 1]);
+                    vj[3 * i + d] = vh[3 * i + d] - xdiv(run[3 + d], eta[i - 1]);
+                }
+            },
+            sh);
+        return;
+    }
     if (threadIdx.x < 6) sh.run[threadIdx.x] = 0.0;
     for (int c0 = 1; c0 < n; c0 += WCH) {
         const int cnt = min(WCH, n - c0);
@@ -1745,7 +1820,7 @@ static __device__ void blk_whm_h2j(int n, const double *Gm, const double *eta, c
                 sh.t[3 + d][q] = Gm[k] * vh[3 * k + d];
             }
         }
-        whm_running(sh, 6, cnt, exact);
+        whm_running(sh, 6, cnt);
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             const int i = c0 + q;
             for (int d = 0; d < 3; d++) {
@@ -1765,6 +1840,24 @@ static __device__ void blk_whm_j2h(int n, const double *Gm, const double *eta, c
         rh[threadIdx.x] = xj[threadIdx.x];
         vh[threadIdx.x] = vj[threadIdx.x];
     }
+    if (exact) {
+        whm_exact_running<6>(
+            n,
+            [&](int i, double *t) {
+                for (int d = 0; d < 3; d++) {
+                    t[d] = xdiv(Gm[i - 1] * xj[3 * (i - 1) + d], eta[i - 1]);
+                    t[3 + d] = xdiv(Gm[i - 1] * vj[3 * (i - 1) + d], eta[i - 1]);
+                }
+            },
+            [&](int i, const double *run) {
+                for (int d = 0; d < 3; d++) {
+                    rh[3 * i + d] = xj[3 * i + d] + run[d];
+                    vh[3 * i + d] = vj[3 * i + d] + run[3 + d];
+                }
+            },
+            sh);
+        return;
+    }
     if (threadIdx.x < 6) sh.run[threadIdx.x] = 0.0;
     for (int c0 = 1; c0 < n; c0 += WCH) {
         const int cnt = min(WCH, n - c0);
@@ -1776,7 +1869,7 @@ static __device__ void blk_whm_j2h(int n, const double *Gm, const double *eta, c
                 sh.t[3 + d][q] = xdiv(Gm[k] * vj[3 * k + d], eta[k]);
             }
         }
-        whm_running(sh, 6, cnt, exact);
+        whm_running(sh, 6, cnt);
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             const int i = c0 + q;
             for (int d = 0; d < 3; d++) {
@@ -1791,6 +1884,18 @@ static __device__ void blk_whm_vh2vj(int n, const double *Gm, const double *eta,
                                      WhmScratch &sh, bool exact) {
     if (n <= 0) return;
     if (threadIdx.x < 3) vj[threadIdx.x] = vh[threadIdx.x];
+    if (exact) {
+        whm_exact_running<3>(
+            n,
+            [&](int i, double *t) {
+                for (int d = 0; d < 3; d++) t[d] = Gm[i - 1] * vh[3 * (i - 1) + d];
+            },
+            [&](int i, const double *run) {
+                for (int d = 0; d < 3; d++) vj[3 * i + d] = vh[3 * i + d] - xdiv(run[d], eta[i - 1]);
+            },
+            sh);
+        return;
+    }
     if (threadIdx.x < 3) sh.run[threadIdx.x] = 0.0;
     for (int c0 = 1; c0 < n; c0 += WCH) {
         const int cnt = min(WCH, n - c0);
@@ -1799,7 +1904,7 @@ static __device__ void blk_whm_vh2vj(int n, const double *Gm, const double *eta,
             const int k = c0 + q - 1;
             for (int d = 0; d < 3; d++) sh.t[d][q] = Gm[k] * vh[3 * k + d];
         }
-        whm_running(sh, 3, cnt, exact);
+        whm_running(sh, 3, cnt);
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             const int i = c0 + q;
             for (int d = 0; d < 3; d++) {
@@ -1836,7 +1941,7 @@ static __device__ void blk_whm_ah0(const double *mu, const double *rhp, int n, d
             whm_ah0_term(mu, rhp, c0 + q, t);
             for (int d = 0; d < 3; d++) sh.t[d][q] = t[d];
         }
-        whm_running(sh, 3, cnt, false);
+        whm_running(sh, 3, cnt);
     }
     __syncthreads();
     if (threadIdx.x < 3) out[threadIdx.x] = sh.run[threadIdx.x];
@@ -1887,11 +1992,7 @@ static __device__ void blk_whm_accel_exact(int n, const double *Gm, double GMcb,
         if (lane < 7) {
             const int first = 1 + (lane < 4 ? k : k - 1) * W, cnt = first < 1 ? 0 : max(0, min(W, n - first));
             double *v = lane < 3 ? &sh.t[lane][at] : lane == 3 ? &sh.e[at] : &sh.t[lane - 1][0];
-#pragma unroll 8
-            for (int q = 0; q < cnt; q++) {
-                s = s + v[q];
-                if (lane >= 3) v[q] = s;
-            }
+            s = serial_running(v, cnt, s, lane >= 3);
         }
         __syncthreads();
         if (k > 0)  // ah2 of chunk k - 1, kept in ah until ah0 is known
