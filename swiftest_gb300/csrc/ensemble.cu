@@ -248,6 +248,20 @@ __global__ void __launch_bounds__(ENS_SUM_T) k_ens_vb2vh(const int32_t *__restri
     blk_vb2vh_pl(npl[s], Gm + o, vb + 3 * o, status + o, vh + 3 * o, GMcb[s], dcb + CB_N * s, exact, sh);
 }
 
+// closing linear drift and vb2vh of the FP64 path
+__global__ void __launch_bounds__(ENS_SUM_T) k_ens_close(const int32_t *__restrict__ poff, const int32_t *__restrict__ npl,
+                                                  const double *__restrict__ Gm, const double *__restrict__ vb,
+                                                  const int32_t *__restrict__ lmask, const int32_t *__restrict__ status,
+                                                  const double *__restrict__ GMcb, double *rh, double *vh, double dt,
+                                                  double *dcb) {
+    const int s = blockIdx.x;
+    if (npl[s] == 0) return;
+    __shared__ SumScratch sh;
+    const size_t o = poff[s];
+    blk_close_pl(npl[s], Gm + o, vb + 3 * o, lmask + o, status + o, GMcb[s], rh + 3 * o, vh + 3 * o, dt, dcb + CB_N * s,
+                 sh);
+}
+
 // Test-particle coordinate updates with their own system's central-body record (modes
 // as k_tp_misc of system.cu: 2 linear drift, 3 linear drift then vb2vh, 4 vh2vb then
 // linear drift, 5 vb = vh + the central body's vb).  mode_first >= 0 replaces mode
@@ -1159,8 +1173,13 @@ int close_pl(swg_ensemble *e, double dth, bool have_acc = false) {
     swg_ctx *c = e->c;
     if (exact(e) || e->NPL == 0 || e->nchunks == 0) {
         SWG_TRY(kick_vb_pl(e, dth, 0, have_acc));
-        SWG_TRY(lindrift_pl(e, dth, CB_PTEND));
-        return vb2vh_pl(e);
+        if (!exact(e) || e->NPL == 0) {
+            SWG_TRY(lindrift_pl(e, dth, CB_PTEND));
+            return vb2vh_pl(e);
+        }
+        k_ens_close<<<e->nsys, ENS_SUM_T, 0, e->c->stream>>>(e->poff, e->npl, e->Gmass, e->vb, e->lmask, e->status,
+                                                            e->GMcb, e->rh, e->vh, dth, e->dcb);
+        return L(e->c, "ens_close");
     }
     SWG_TRY(kick_vb_pl(e, dth, 0, have_acc, false));
     SWG_TRY(ensure(c, e->close_part, sizeof(double) * 6 * (size_t)e->nchunks));

@@ -103,6 +103,14 @@ __device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int npl
     constexpr bool plpl = MODE != KICK_TP;
     const int jmax = plpl && i0 >= nplm ? nplm : npart;  // partners of the block's receivers
     const int rounds = (jmax + PT - 1) / PT;
+    if (!plpl) {  // a block without an active receiver
+        const int i = i0 + (int)threadIdx.x;
+        if (!__syncthreads_or((int)threadIdx.x < RT && i < nrecv && lmask[i] != 0)) {
+            if (acc_is_zero)
+                for (int k = threadIdx.x; k < 3 * min(RT, nrecv - i0); k += nth) acc[3 * i0 + k] = 0.0;
+            return;
+        }
+    }
     if (w >= 0) {  // term warps: warp w + 1 of the block
         // a term that leaves the sum as it is, signed zeros included
         const double neutral = plpl ? -0.0 : 0.0;

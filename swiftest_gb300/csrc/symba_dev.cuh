@@ -36,13 +36,13 @@ struct Sum3 {
 constexpr int SCH = 256;  // terms per chunk of the serial sums
 // shared-memory workspace of the ordered sums (one per kernel)
 struct SumScratch {
-    double t[2][4][SCH + 1];  // two chunks of up to four components (offset: conflict-free columns)
+    double t[2][6][SCH + 1];  // two chunks of up to six components (offset: conflict-free columns)
     double rx[RB / 32], ry[RB / 32], rz[RB / 32];
-    double sum[4];
+    double sum[6];
     Sum3 acc;
 };
 
-// Sums of NC components (up to four) over i = 0 .. n-1 (reverse: n-1 .. 0), one addition at a
+// Sums of NC components (up to six) over i = 0 .. n-1 (reverse: n-1 .. 0), one addition at a
 // time in that order, whole block; the sums are left in sh.sum.  term_fn(i, t) writes the NC
 // terms of index i and returns whether they count; one that does not is added as -0.0, which
 // leaves every sum as it is.  Lane c of warp 0 adds component c, so one FP64 addition (64 cycles,
@@ -237,9 +237,9 @@ static __device__ void blk_vb2vh_pl(int npl, const double *__restrict__ Gm,
     const double inv = 1.0 / GMcb;
     auto term = [&](int i, double &x, double &y, double &z) -> unsigned char {
         if (exact) {
-            x = Gm[i] * vb[3 * i + 0] / GMcb;
-            y = Gm[i] * vb[3 * i + 1] / GMcb;
-            z = Gm[i] * vb[3 * i + 2] / GMcb;
+            x = xdiv(Gm[i] * vb[3 * i + 0], GMcb);
+            y = xdiv(Gm[i] * vb[3 * i + 1], GMcb);
+            z = xdiv(Gm[i] * vb[3 * i + 2], GMcb);
         } else {
             const double g = Gm[i] * inv;
             x = g * vb[3 * i + 0];
@@ -258,6 +258,46 @@ static __device__ void blk_vb2vh_pl(int npl, const double *__restrict__ Gm,
         vh[3 * i + 0] = vb[3 * i + 0] - s.x;
         vh[3 * i + 1] = vb[3 * i + 1] - s.y;
         vh[3 * i + 2] = vb[3 * i + 2] - s.z;
+    }
+}
+
+// The end of a step in the FP64 path: helio_drift_linear_pl, then swiftest_util_coord_vb2vh_pl.  The
+// linear drift leaves vb as it is, so both sums (one forward, one in reverse order) run
+// together, six lanes in one addition.
+static __device__ void blk_close_pl(int npl, const double *__restrict__ Gm, const double *__restrict__ vb,
+                                    const int32_t *__restrict__ lmask, const int32_t *__restrict__ status,
+                                    double GMcb, double *rh, double *vh, double dt, double *dcb, SumScratch &sh) {
+    blk_serial_sums<6>(
+        npl, false,
+        [&](int i, double *t) {
+            const int j = npl - 1 - i;
+            const bool on = lmask[i] != 0, act = status[j] != ST_INACTIVE;
+            for (int d = 0; d < 3; d++) {
+                t[d] = on ? Gm[i] * vb[3 * i + d] : -0.0;
+                t[3 + d] = act ? -xdiv(Gm[j] * vb[3 * j + d], GMcb) : -0.0;
+            }
+            return true;
+        },
+        sh);
+    const Sum3 c = {sh.sum[3], sh.sum[4], sh.sum[5]};
+    const Sum3 pt = blk_quotient({sh.sum[0], sh.sum[1], sh.sum[2]}, GMcb, sh);
+    if (threadIdx.x == 0) {
+        dcb[CB_PTEND + 0] = pt.x;
+        dcb[CB_PTEND + 1] = pt.y;
+        dcb[CB_PTEND + 2] = pt.z;
+        dcb[CB_VB + 0] = c.x;
+        dcb[CB_VB + 1] = c.y;
+        dcb[CB_VB + 2] = c.z;
+    }
+    for (int i = threadIdx.x; i < npl; i += blockDim.x) {
+        if (lmask[i]) {
+            rh[3 * i + 0] = rh[3 * i + 0] + pt.x * dt;
+            rh[3 * i + 1] = rh[3 * i + 1] + pt.y * dt;
+            rh[3 * i + 2] = rh[3 * i + 2] + pt.z * dt;
+        }
+        vh[3 * i + 0] = vb[3 * i + 0] - c.x;
+        vh[3 * i + 1] = vb[3 * i + 1] - c.y;
+        vh[3 * i + 2] = vb[3 * i + 2] - c.z;
     }
 }
 

@@ -74,9 +74,11 @@ struct swg_system {
     DevBuf kick_scratch, kick_scratch_tp, pair_scratch, flags, red;
     // SyMBA: the level-0 checks and the test particles' half-steps run on a second stream
     // beside the massive bodies' (events: 0 opening ready, 1 tp opening done, 2 closing
-    // ready, 3 central-body drift ready, 4 tp closing done, 5 level-0 lists ready)
+    // ready, 3 central-body drift ready, 4 tp closing done, 5 level-0 lists ready, 6 recursion
+    // about to start)
     cudaStream_t side = nullptr, side2 = nullptr;  // side2: the pl-tp check beside the pl-pl one on side
-    cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    DevBuf tmask;  // masks of the listed and the other test particles
     DevBuf snap;  // the start-of-step rh, vb, trh, tvb that the overlapped level-0 checks read
     int32_t *h_flags = nullptr;  // pinned: [0] lencounter, [1] nfail, [2] recursion status, [3] deepest level,
                                  // [4] collision pending
@@ -130,6 +132,14 @@ __global__ void __launch_bounds__(RB) k_vb2vh_pl(int npl, const double *__restri
                                                  double *vh, double GMcb, double *dcb, int exact) {
     __shared__ SumScratch sh;
     blk_vb2vh_pl(npl, Gm, vb, status, vh, GMcb, dcb, exact, sh);
+}
+
+__global__ void __launch_bounds__(RB) k_close_pl(int npl, const double *__restrict__ Gm,
+                                                 const double *__restrict__ vb, const int32_t *__restrict__ lmask,
+                                                 const int32_t *__restrict__ status, double GMcb, double *rh,
+                                                 double *vh, double dt, double *dcb) {
+    __shared__ SumScratch sh;
+    blk_close_pl(npl, Gm, vb, lmask, status, GMcb, rh, vh, dt, dcb, sh);
 }
 
 // test particles: mode 0 vh2vb(vbcb=-pt) ; 1 vb2vh(vbcb=-pt) ; 2 lindrift rh += pt*dt ;
@@ -215,6 +225,16 @@ __global__ void __launch_bounds__(ADDBACK_SMALL) k_pltp_addback_small(int n, con
     tah[3 * j + 0] = x;
     tah[3 * j + 1] = y;
     tah[3 * j + 2] = z;
+}
+
+// the kicked test particles in an encounter list (level 0) and the others
+__global__ void k_listed_masks(int ntp, const int32_t *__restrict__ tlmask, const int32_t *__restrict__ tlevelg,
+                               int32_t *listed, int32_t *others) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ntp) return;
+    const bool on = tlmask[i] != 0, in = tlevelg[i] >= 0;
+    listed[i] = on && in;
+    others[i] = on && !in;
 }
 
 // The whole SyMBA recursion of one step, one block (blk_symba_recursion).
@@ -340,24 +360,27 @@ int kick_vb_pl(swg_system *s, double dt, int lbeg, bool copy_r = true, bool have
 }
 
 // helio_kick_vb_tp (helio_kick.f90:135-169) with symba_kick_getacch_tp (symba_kick.f90:79-123)
-int kick_vb_tp(swg_system *s, double dt, int lbeg) {
+// mask (optional): the test particles to kick instead of all; addback: add the pl-tp encounter
+// terms back (they concern the listed test particles alone)
+int kick_vb_tp(swg_system *s, double dt, int lbeg, const int32_t *mask = nullptr, bool addback = true) {
     swg_ctx *c = s->c;
     if (s->ntp == 0) return SWG_OK;
+    if (!mask) mask = s->tlmask;
     const double *rp = lbeg ? s->rbeg : s->rend;
     if (s->npl > 0) {
         ProfScope ps(s->prof, s->c->stream, PROF_KICK_TP);
         if (s->precision == SWG_MIXED) {
             const int nch = kick_mixed_chunks(c, s->ntp, s->npl);
             SWG_TRY(ensure_kick_scratch(c, s->kick_scratch_tp, kick_mixed_scratch_bytes(s->ntp, s->npl, nch)));
-            SWG_TRY(kick_mixed_launch(c, true, s->ntp, s->npl, 0, s->trh, rp, s->Gmass, nullptr, s->tlmask, s->tah,
+            SWG_TRY(kick_mixed_launch(c, true, s->ntp, s->npl, 0, s->trh, rp, s->Gmass, nullptr, mask, s->tah,
                                       1, nch, s->kick_scratch_tp.ptr));
         } else {
-            SWG_TRY(kick_tp_fp64(c, s->ntp, s->npl, s->trh, rp, s->Gmass, s->tlmask, s->tah, 1));
+            SWG_TRY(kick_tp_fp64(c, s->ntp, s->npl, s->trh, rp, s->Gmass, mask, s->tah, 1));
         }
     } else {
         SWG_TRY(cuda_status(c, cudaMemsetAsync(s->tah, 0, sizeof(double) * 3 * s->ntp, c->stream), "memset"));
     }
-    if (s->integrator == SWG_SYMBA && s->pltp_n > 0) {
+    if (addback && s->integrator == SWG_SYMBA && s->pltp_n > 0) {
         if (s->pltp_n <= ADDBACK_SMALL)
             k_pltp_addback_small<<<1, ADDBACK_SMALL, 0, c->stream>>>((int)s->pltp_n, s->pltp_l,
                                                                       s->pltp_l + s->pltp_cap, s->tlmask, s->trh, rp,
@@ -367,7 +390,7 @@ int kick_vb_tp(swg_system *s, double dt, int lbeg) {
                                                     s->trh, rp, s->Gmass, s->tah);
         SWG_TRY(L(c, "pltp_addback"));
     }
-    k_kick_update<<<grid_for(s->ntp, 128), 128, 0, c->stream>>>(s->ntp, s->tvb, s->tah, s->tlmask, dt, nullptr,
+    k_kick_update<<<grid_for(s->ntp, 128), 128, 0, c->stream>>>(s->ntp, s->tvb, s->tah, mask, dt, nullptr,
                                                                  nullptr);
     return L(c, "kick_update_tp");
 }
@@ -429,6 +452,17 @@ int vb2vh_pl(swg_system *s) {
     k_vb2vh_pl<<<1, RB, 0, s->c->stream>>>(s->npl, s->Gmass, s->vb, s->status, s->vh, s->GMcb, s->dcb, exact(s));
     return L(s->c, "vb2vh_pl");
 }
+// the closing linear drift and vb2vh (one launch in the FP64 path)
+int close_pl(swg_system *s, double dt) {
+    if (s->npl == 0) return SWG_OK;
+    if (!exact(s)) {
+        SWG_TRY(lindrift_pl(s, dt, 0));
+        return vb2vh_pl(s);
+    }
+    k_close_pl<<<1, RB, 0, s->c->stream>>>(s->npl, s->Gmass, s->vb, s->lmask, s->status, s->GMcb, s->rh, s->vh, dt,
+                                            s->dcb);
+    return L(s->c, "close_pl");
+}
 // drift with the SyMBA level mask (levelg == irec) or the plain status mask
 int drift_pl(swg_system *s, double dt) {
     if (s->npl == 0) return SWG_OK;
@@ -446,11 +480,78 @@ int drift_tp(swg_system *s, double dt) {
                         !exact(s));
 }
 
+// Runs f with the context's stream temporarily replaced (single host thread).
+template <class F>
+int on_stream(swg_ctx *c, cudaStream_t st, F f) {
+    const cudaStream_t saved = c->stream;
+    c->stream = st;
+    const int rc = f();
+    c->stream = saved;
+    return rc;
+}
+
+int ensure_side(swg_system *s) {
+    if (s->side) return SWG_OK;
+    SWG_TRY(cuda_status(s->c, cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking), "side stream"));
+    SWG_TRY(cuda_status(s->c, cudaStreamCreateWithFlags(&s->side2, cudaStreamNonBlocking), "side stream"));
+    for (cudaEvent_t &e : s->ev) SWG_TRY(cuda_status(s->c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event"));
+    return SWG_OK;
+}
+// stream b waits for the work queued so far on stream a (event e)
+int join(swg_ctx *c, cudaStream_t a, cudaStream_t b, cudaEvent_t e) {
+    SWG_TRY(cuda_status(c, cudaEventRecord(e, a), "event"));
+    return cuda_status(c, cudaStreamWaitEvent(b, e, 0), "event");
+}
+
+// the massive bodies' positions into rbeg or rend, on the context's stream
+int copy_positions(swg_system *s, double *to) {
+    return cuda_status(s->c, cudaMemcpyAsync(to, s->rh, 24 * (size_t)s->npl, cudaMemcpyDeviceToDevice, s->c->stream),
+                       "positions");
+}
+// The closing half of a step whose test particles are on the side stream (their closing kick
+// queued): the massive bodies' closing kick and sums here, the test particles' closing linear
+// drift once the central-body record is there, then both joined.
+int close_half(swg_system *s, double dth) {
+    swg_ctx *c = s->c;
+    SWG_TRY(kick_vb_pl(s, dth, 0, false));
+    if (exact(s)) SWG_TRY(close_pl(s, dth));
+    else SWG_TRY(lindrift_pl(s, dth, 0));
+    SWG_TRY(join(c, c->stream, s->side, s->ev[3]));
+    SWG_TRY(on_stream(c, s->side, [&] { return tp_misc(s, CB_PTEND, dth, 3); }));
+    if (!exact(s)) SWG_TRY(vb2vh_pl(s));
+    return join(c, s->side, c->stream, s->ev[4]);
+}
+
 // helio_step_pl / _tp (helio_step.f90:37-119) via whm_step_system (whm_step.f90:14-35)
 // opened: the opening sums and the pl-pl accelerations already ran (symba_step)
+// With test particles their half-steps run on a second stream beside the massive bodies'
+// (reading the positions recorded in rbeg / rend and the central-body record), as in
+// symba_interp; each kernel's arithmetic is unchanged.
 int helio_step(swg_system *s, double dt, bool opened = false) {
+    swg_ctx *c = s->c;
     const double dth = 0.5 * dt;
     s->lfirst_tp = s->lfirst_pl;
+    const bool fork = s->ntp > 0 && s->npl > 0 && !s->prof.on;
+    const int first_mode = s->lfirst_tp ? 4 : 2;
+    if (fork) {
+        SWG_TRY(ensure_side(s));
+        if (s->lfirst_pl && !opened) SWG_TRY(vh2vb_pl(s));
+        s->lfirst_pl = s->lfirst_tp = 0;
+        if (!opened) SWG_TRY(lindrift_pl(s, dth, 1));
+        SWG_TRY(copy_positions(s, s->rbeg));
+        SWG_TRY(join(c, c->stream, s->side, s->ev[0]));
+        SWG_TRY(on_stream(c, s->side, [&] {
+            SWG_TRY(tp_misc(s, CB_PTBEG, dth, first_mode));
+            SWG_TRY(kick_vb_tp(s, dth, 1));
+            return drift_tp(s, dt);
+        }));
+        SWG_TRY(kick_vb_pl(s, dth, 1, false, opened));
+        SWG_TRY(drift_pl(s, dt));
+        SWG_TRY(copy_positions(s, s->rend));
+        SWG_TRY(join(c, c->stream, s->side, s->ev[2]));
+        SWG_TRY(on_stream(c, s->side, [&] { return kick_vb_tp(s, dth, 0); }));
+        return close_half(s, dth);
+    }
     if (s->npl > 0) {
         if (s->lfirst_pl) {
             if (!opened) SWG_TRY(vh2vb_pl(s));
@@ -460,8 +561,7 @@ int helio_step(swg_system *s, double dt, bool opened = false) {
         SWG_TRY(kick_vb_pl(s, dth, 1, true, opened));
         SWG_TRY(drift_pl(s, dt));
         SWG_TRY(kick_vb_pl(s, dth, 0));
-        SWG_TRY(lindrift_pl(s, dth, 0));
-        SWG_TRY(vb2vh_pl(s));
+        SWG_TRY(close_pl(s, dth));
     }
     if (s->ntp > 0) {
         if (s->lfirst_tp) {
@@ -566,29 +666,6 @@ int whm_step(swg_system *s, double dt) {
 }
 
 // ---- SyMBA
-// Runs f with the context's stream temporarily replaced (single host thread).
-template <class F>
-int on_stream(swg_ctx *c, cudaStream_t st, F f) {
-    const cudaStream_t saved = c->stream;
-    c->stream = st;
-    const int rc = f();
-    c->stream = saved;
-    return rc;
-}
-
-int ensure_side(swg_system *s) {
-    if (s->side) return SWG_OK;
-    SWG_TRY(cuda_status(s->c, cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking), "side stream"));
-    SWG_TRY(cuda_status(s->c, cudaStreamCreateWithFlags(&s->side2, cudaStreamNonBlocking), "side stream"));
-    for (cudaEvent_t &e : s->ev) SWG_TRY(cuda_status(s->c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event"));
-    return SWG_OK;
-}
-// stream b waits for the work queued so far on stream a (event e)
-int join(swg_ctx *c, cudaStream_t a, cudaStream_t b, cudaEvent_t e) {
-    SWG_TRY(cuda_status(c, cudaEventRecord(e, a), "event"));
-    return cuda_status(c, cudaStreamWaitEvent(b, e, 0), "event");
-}
-
 int ensure_list(swg_system *s, int32_t **l, int64_t *cap, int64_t need) {
     if (need <= *cap) return SWG_OK;
     const int64_t ncap = std::max<int64_t>(need + need / 2, 256);
@@ -909,9 +986,13 @@ int resolve_collisions(swg_system *s) {
     return cuda_status(c, cudaStreamSynchronize(c->stream), "collision");
 }
 
+// beside (optional): queues work that runs beside the recursion, after event 6 (recorded just
+// before the kernel): work queued earlier would hold every SM, and the recursion's one block
+// needs most of one.
 // Launch the whole SyMBA recursion of one step (symba_step_recur_system from level 0)
 // as one single-block kernel; no host round trip until the next step's checks.
-int symba_recursion(swg_system *s, double dt) {
+template <class F>
+int symba_recursion(swg_system *s, double dt, bool have_beside, F beside) {
     swg_ctx *c = s->c;
     s->rec_dt = dt;
     const int64_t n = s->plpl_n + s->pltp_n;
@@ -977,8 +1058,11 @@ int symba_recursion(swg_system *s, double dt) {
     for (;;) {
         if (s->lclose)
             SWG_TRY(cuda_status(c, cudaMemsetAsync(a.pend, 0, sizeof(int32_t), c->stream), "memset"));
+        if (have_beside) SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[6], c->stream), "event"));
         k_symba_recursion<<<1, RECT, smem, c->stream>>>(a);
         SWG_TRY(L(c, "symba_recursion"));
+        if (have_beside) SWG_TRY(beside());
+        have_beside = false;
         if (!s->lclose) break;
         // a collision pauses the recursion: resolve it on the host, then resume
         SWG_TRY(cuda_status(c, cudaMemcpyAsync(s->h_flags + 4, a.pend, sizeof(int32_t), cudaMemcpyDeviceToHost,
@@ -986,6 +1070,7 @@ int symba_recursion(swg_system *s, double dt) {
                             "pending"));
         SWG_TRY(cuda_status(c, cudaStreamSynchronize(c->stream), "recursion"));
         if (s->h_flags[4] == 0) break;
+        if (s->side) SWG_TRY(cuda_status(c, cudaStreamSynchronize(s->side), "test particles"));  // it copies all of them
         SWG_TRY(resolve_collisions(s));
     }
     // status word read back at the next host synchronization
@@ -1006,48 +1091,60 @@ int symba_interp(swg_system *s, double dt, bool opened = false) {
     const double dth = 0.5 * dt;
     s->irec = -1;
     const bool fork = s->ntp > 0 && s->npl > 0;
+    // FP64 path: the recursion moves only the listed test particles, so it waits for their
+    // opening kick alone and the others' kick and drift run beside it (10,000 tp against 2000
+    // pl: 0.42 ms beside a recursion of 0.1 to 2 ms)
+    const bool listed_first = fork && exact(s);
     if (fork) SWG_TRY(ensure_side(s));
+    if (listed_first) SWG_TRY(ensure(c, s->tmask, sizeof(int32_t) * 2 * (size_t)s->ntp));
     if (!opened) {
         if (s->lfirst_pl) SWG_TRY(vh2vb_pl(s));
         SWG_TRY(lindrift_pl(s, dth, 1));
     }
     if (fork) {
-        SWG_TRY(cuda_status(c, cudaMemcpyAsync(s->rbeg, s->rh, 24 * (size_t)s->npl, cudaMemcpyDeviceToDevice, c->stream),
-                            "rbeg"));
+        SWG_TRY(copy_positions(s, s->rbeg));
         SWG_TRY(join(c, c->stream, s->side, s->ev[0]));
         SWG_TRY(on_stream(c, s->side, [&] {
             SWG_TRY(tp_misc(s, CB_PTBEG, dth, s->lfirst_tp ? 4 : 2));
-            SWG_TRY(kick_vb_tp(s, dth, 1));
-            return drift_tp(s, dt);
+            if (!listed_first) {
+                SWG_TRY(kick_vb_tp(s, dth, 1));
+                SWG_TRY(drift_tp(s, dt));
+                return cuda_status(c, cudaEventRecord(s->ev[1], s->side), "event");
+            }
+            int32_t *listed = (int32_t *)s->tmask.ptr;
+            k_listed_masks<<<grid_for(s->ntp, 256), 256, 0, c->stream>>>(s->ntp, s->tlmask, s->tlevelg, listed,
+                                                                          listed + s->ntp);
+            SWG_TRY(L(c, "listed_masks"));
+            if (s->pltp_n > 0) SWG_TRY(kick_vb_tp(s, dth, 1, listed));
+            return cuda_status(c, cudaEventRecord(s->ev[1], s->side), "event");
         }));
     }
     SWG_TRY(kick_vb_pl(s, dth, 1, !fork, opened));
     SWG_TRY(drift_pl(s, dt));
     if (fork) {
-        SWG_TRY(join(c, s->side, c->stream, s->ev[1]));
+        SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[1], 0), "event"));
     } else if (s->ntp > 0) {
         SWG_TRY(tp_misc(s, CB_PTBEG, dth, s->lfirst_tp ? 4 : 2));
         SWG_TRY(kick_vb_tp(s, dth, 1));
         SWG_TRY(drift_tp(s, dt));
     }
-    SWG_TRY(symba_recursion(s, dt));
+    SWG_TRY(symba_recursion(s, dt, listed_first, [&] {
+        SWG_TRY(cuda_status(c, cudaStreamWaitEvent(s->side, s->ev[6], 0), "event"));
+        return on_stream(c, s->side, [&] {
+            SWG_TRY(kick_vb_tp(s, dth, 1, (int32_t *)s->tmask.ptr + s->ntp, false));
+            return drift_tp(s, dt);  // the listed ones drift in the recursion
+        });
+    }));
     s->irec = -1;
     if (fork) {
-        SWG_TRY(cuda_status(c, cudaMemcpyAsync(s->rend, s->rh, 24 * (size_t)s->npl, cudaMemcpyDeviceToDevice, c->stream),
-                            "rend"));
+        SWG_TRY(copy_positions(s, s->rend));
         SWG_TRY(join(c, c->stream, s->side, s->ev[2]));
         SWG_TRY(on_stream(c, s->side, [&] { return kick_vb_tp(s, dth, 0); }));
+        return close_half(s, dth);
     }
-    SWG_TRY(kick_vb_pl(s, dth, 0, !fork));
-    SWG_TRY(lindrift_pl(s, dth, 0));
-    if (fork) {  // the test particles' closing linear drift needs the central-body record
-        SWG_TRY(join(c, c->stream, s->side, s->ev[3]));
-        SWG_TRY(on_stream(c, s->side, [&] { return tp_misc(s, CB_PTEND, dth, 3); }));
-    }
-    SWG_TRY(vb2vh_pl(s));
-    if (fork) {
-        SWG_TRY(join(c, s->side, c->stream, s->ev[4]));
-    } else if (s->ntp > 0) {
+    SWG_TRY(kick_vb_pl(s, dth, 0));
+    SWG_TRY(close_pl(s, dth));
+    if (s->ntp > 0) {
         SWG_TRY(kick_vb_tp(s, dth, 0));
         SWG_TRY(tp_misc(s, CB_PTEND, dth, 3));
     }
@@ -1201,7 +1298,7 @@ int swg_system_destroy(swg_system *s) {
                     s->enc.sort.ptr, s->enc.counters.ptr, s->enc2.raw.ptr, s->enc2.sort.ptr, s->enc2.counters.ptr, s->kick_scratch.ptr, s->pair_scratch.ptr, s->flags.ptr,
                     s->red.ptr, s->mark_pl, s->mark_tp, s->rec_out, s->rec_resume, s->rec_scratch.ptr,
                     s->discard_scratch.ptr, s->tflag, s->ndiscard, s->chunk_buf.ptr, s->kick_scratch_tp.ptr,
-                    s->snap.ptr};
+                    s->snap.ptr,       s->tmask.ptr};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (s->h_flags) cudaFreeHost(s->h_flags);
