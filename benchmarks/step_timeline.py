@@ -158,15 +158,13 @@ def _patch_system(s: str) -> str:
     rep("    SWG_TRY(kick_vb_pl(s, dth, 1, !fork, opened));\n    SWG_TRY(drift_pl(s, dt));\n",
         "    SWG_TRY(kick_vb_pl(s, dth, 1, !fork, opened));\n    swg_tr(c->stream, 22);\n    SWG_TRY(drift_pl(s, dt));\n"
         "    swg_tr(c->stream, 23);\n")
-    rep("            return drift_tp(s, dt);\n        }));\n",
-        "            SWG_TRY(drift_tp(s, dt));\n            swg_tr(c->stream, 24);\n            return SWG_OK;\n        }));\n")
-    rep("    SWG_TRY(symba_recursion(s, dt));\n    s->irec = -1;\n",
-        "    SWG_TRY(symba_recursion(s, dt));\n    swg_tr(c->stream, 25);\n    s->irec = -1;\n")
-    rep("        SWG_TRY(on_stream(c, s->side, [&] { return kick_vb_tp(s, dth, 0); }));\n",
-        "        SWG_TRY(on_stream(c, s->side, [&] { SWG_TRY(kick_vb_tp(s, dth, 0)); swg_tr(c->stream, 27); "
-        "return SWG_OK; }));\n")
-    rep("    SWG_TRY(kick_vb_pl(s, dth, 0, !fork));\n    SWG_TRY(lindrift_pl(s, dth, 0));\n",
-        "    SWG_TRY(kick_vb_pl(s, dth, 0, !fork));\n    swg_tr(c->stream, 26);\n    SWG_TRY(lindrift_pl(s, dth, 0));\n")
+    rep("                SWG_TRY(drift_tp(s, dt));\n                return cuda_status(c, cudaEventRecord(s->ev[1], s->side)",
+        "                SWG_TRY(drift_tp(s, dt));\n                swg_tr(c->stream, 24);\n"
+        "                return cuda_status(c, cudaEventRecord(s->ev[1], s->side)")
+    rep("    }));\n    s->irec = -1;\n    if (fork) {\n", "    }));\n    swg_tr(c->stream, 25);\n    s->irec = -1;\n    if (fork) {\n")
+    rep("    SWG_TRY(kick_vb_pl(s, dth, 0, false));\n", "    SWG_TRY(kick_vb_pl(s, dth, 0, false));\n    swg_tr(c->stream, 26);\n")
+    rep("    SWG_TRY(join(c, c->stream, s->side, s->ev[3]));\n",
+        "    swg_tr(s->side, 27);\n    SWG_TRY(join(c, c->stream, s->side, s->ev[3]));\n")
     rep("    s->lfirst_tp = s->lfirstkick;\n    s->lfirst_pl = s->lfirstkick;\n    int lany = 0;\n",
         "    swg_tr(c->stream, 20);\n    s->lfirst_tp = s->lfirstkick;\n    s->lfirst_pl = s->lfirstkick;\n"
         "    int lany = 0;\n")
