@@ -15,8 +15,8 @@
 // are issued as DFMA with a factor of one: the same rounding).  The square root, the
 // quotient and the products are formed outside that pipe (fp64_exact.cuh, the same bits), which
 // leaves five additions per pair and 3.2 for the fold: 8.2 instructions, 131 cycles, per 32
-// pairs and SM against ~40 before.  65,537 tp x 2047 pl: 10.3 -> 2.6 ms (16,384 pl: 22.6 -> 5.4 ms),
-// FP64 pipe 72%, ALU pipe 66%, issue slots 63% busy (ncu); four blocks of 40 registers per SM
+// pairs and SM against ~40 before.  65,537 tp x 2047 pl: 10.3 -> 2.6 ms (16,384 pl: 22.6 -> 5.3 ms),
+// FP64 pipe 74%, ALU pipe 60%, issue slots 64% busy (ncu); four blocks of 40 registers per SM
 // (three of 56: 2.8 ms, two: 3.9 ms): the long chains of dependent instructions want warps.
 //
 #include <cuda_runtime.h>
@@ -70,23 +70,24 @@ __device__ __forceinline__ float radius_bound(double R) {
     return __fmul_ru(2.0f, __fmul_ru(f, f));
 }
 
-// Product of a factor f (x_ok unless bad) and a displacement: x_mul where both operands are in
-// range, the zero itself for a zero displacement; elsewhere bad.
-__device__ __forceinline__ double mul_disp(double f, double d, bool &bad) {
-    const int h = __double2hiint(d) & 0x7fffffff;
-    const bool zero = (h | __double2loint(d)) == 0;
-    bad |= !x_ok(h) && !zero;
-    const double p = x_mul(f, d);
-    return zero ? d : p;
-}
-
-// Square of a displacement: zero for a zero one, bad out of range.
-__device__ __forceinline__ double sqr_disp(double d, bool &bad) {
-    const int h = __double2hiint(d) & 0x7fffffff;
-    const bool zero = (h | __double2loint(d)) == 0;
-    bad |= !x_ok(h) && !zero;
-    const double p = x_sqr(d);
-    return zero ? 0.0 : p;
+// Displacements outside the exact products' range, found by one test of the smallest and one of
+// the largest exponent (a test per component: kick_pl_fp64's 16,384 bodies 5.47 ms, this 5.29).
+// A zero component is replaced by 2^-300, whose square leaves every other square and r^2 as they
+// are, and marked (bit c of the result); what else is out of range sets bad.
+__device__ __forceinline__ int odd_disp(double &dx, double &dy, double &dz, bool &bad) {
+    constexpr int LOW = (1023 - XR_EXP) << 20, HIGH = ((1023 + XR_EXP + 1) << 20) - 1;
+    auto one = [&](double &d, int bit) {
+        const int h = __double2hiint(d) & 0x7fffffff;
+        if (h >= LOW) return 0;
+        bad |= (h | __double2loint(d)) != 0;
+        d = __hiloint2double((1023 - 300) << 20, 0);
+        return bit;
+    };
+    const int hx = __double2hiint(dx) & 0x7fffffff, hy = __double2hiint(dy) & 0x7fffffff,
+              hz = __double2hiint(dz) & 0x7fffffff;
+    bad |= max(hx, max(hy, hz)) > HIGH;
+    if (min(hx, min(hy, hz)) >= LOW) return 0;
+    return one(dx, 1) | one(dy, 2) | one(dz, 4);
 }
 
 // Receivers [i0, i0 + RT) (those below nrecv) of one system against all its partners, whole
@@ -132,11 +133,12 @@ __device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int npl
             if (j < jend && (!plpl || j != i)) {
                 const double g = Gm[j];
                 const double xj = rp[3 * j + 0], yj = rp[3 * j + 1], zj = rp[3 * j + 2];
-                const double dx = plpl ? sub1(xj, xi) : sub1(xi, xj);
-                const double dy = plpl ? sub1(yj, yi) : sub1(yi, yj);
-                const double dz = plpl ? sub1(zj, zi) : sub1(zi, zj);
+                double dx = plpl ? sub1(xj, xi) : sub1(xi, xj);
+                double dy = plpl ? sub1(yj, yi) : sub1(yi, yj);
+                double dz = plpl ? sub1(zj, zi) : sub1(zi, zj);
                 bool bad = false, near = false;
-                const double r2 = add1(add1(sqr_disp(dx, bad), sqr_disp(dy, bad)), sqr_disp(dz, bad));
+                const int zero = odd_disp(dx, dy, dz, bad);
+                const double r2 = add1(add1(x_sqr(dx), x_sqr(dy)), x_sqr(dz));
                 const int h = __double2hiint(r2);
                 bad |= !x_ok(h) || !x_ok(__double2hiint(g));
                 if (RAD) near = !(__int_as_float((h - ((1023 - 127) << 20)) << 3) > __fadd_ru(rbi, radius_bound(R[j])));
@@ -149,10 +151,18 @@ __device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int npl
                 } else {
                     fac = x_div(x_num(g), p, bad);
                 }
-                fx = mul_disp(fac, dx, bad);
-                fy = mul_disp(fac, dy, bad);
-                fz = mul_disp(fac, dz, bad);
+                fx = x_mul(fac, dx);
+                fy = x_mul(fac, dy);
+                fz = x_mul(fac, dz);
+                if (zero) {  // the products of zero displacements, with their signs
+                    if (zero & 1) fx = plpl ? sub1(xj, xi) : sub1(xi, xj);
+                    if (zero & 2) fy = plpl ? sub1(yj, yi) : sub1(yi, yj);
+                    if (zero & 4) fz = plpl ? sub1(zj, zi) : sub1(zi, zj);
+                }
                 if (bad || near) {  // rare: native operations
+                    dx = plpl ? sub1(xj, xi) : sub1(xi, xj);
+                    dy = plpl ? sub1(yj, yi) : sub1(yi, yj);
+                    dz = plpl ? sub1(zj, zi) : sub1(zi, zj);
                     const double q2 = dx * dx + dy * dy + dz * dz;
                     const double q = q2 * sqrt(q2);
                     fac = MODE == KICK_SPLIT ? g * (1.0 / q) : g / q;

@@ -30,12 +30,20 @@ def _inputs(kind, n):
         r *= 2.0 ** rng.choice([-70, -55, -45, 0, 0, 45, 55, 70], n)[:, None]
         g *= 2.0 ** rng.choice([-120, 0, 60, 110], n)
         R = np.where(rng.random(n) < 0.3, 0.0, R * 2.0 ** rng.choice([-130, 0, 0, 8, 12], n))
+    elif kind == "huge":  # squares beyond the doubles' range, exponents that wrap around
+        r *= 2.0 ** rng.choice([0, 0, 60, 103, 510, 513, 600], n)[:, None]
+        r[::4, 1:] = 0.0
+    elif kind == "ties":  # x: zero; y^2: half a unit in the last place of z^2
+        r[:] = 0.0
+        r[1:, 1] = 2.0 ** -76
+        r[1:, 2] = 2.0 ** -49.5 * (1.0 + rng.uniform(0.01, 0.4, n - 1))
+        g = rng.uniform(1.0, 2.0, n) * 2.0 ** -90
     elif kind == "close":  # near and overlapping pairs
         r[1::2] = r[: 2 * (n // 2) : 2] * (1.0 + 2.0 ** -rng.integers(8, 45, n // 2))[:, None]
     return r, g, R
 
 
-@pytest.mark.parametrize("kind", ["disk", "coplanar", "grid", "scales", "close"])
+@pytest.mark.parametrize("kind", ["disk", "coplanar", "grid", "scales", "close", "huge", "ties"])
 @pytest.mark.parametrize("n", [3, 10, 11, 31, 32, 33, 65, 321])
 def test_kick_pl_bits(ctx, kind, n):
     r, g, R = _inputs(kind, n)
@@ -45,7 +53,7 @@ def test_kick_pl_bits(ctx, kind, n):
             assert np.array_equal(_bits(a), _bits(O.kick_tri_pl(r, g, rad, nplm=nplm)))
 
 
-@pytest.mark.parametrize("kind", ["disk", "coplanar", "grid", "scales"])
+@pytest.mark.parametrize("kind", ["disk", "coplanar", "grid", "scales", "huge", "ties"])
 @pytest.mark.parametrize("ntp,npl", [(1, 33), (10, 32), (11, 64), (331, 97), (3001, 5)])
 def test_kick_tp_bits(ctx, kind, ntp, npl):
     r, g, _ = _inputs(kind, ntp + npl)
