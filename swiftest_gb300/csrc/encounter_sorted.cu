@@ -180,8 +180,15 @@ __global__ void __launch_bounds__(SB) k_sorted_prep(const int2 *__restrict__ til
                                                     const int32_t *__restrict__ npl, const int32_t *__restrict__ perm,
                                                     const double *__restrict__ r, const double *__restrict__ v,
                                                     const double *__restrict__ renc, float adt, float4 *A, float4 *B,
-                                                    float4 *V, float4 *bounds) {
+                                                    float4 *V, float4 *bounds, double *rcopy, double *vcopy) {
     const int2 tl = tiles[blockIdx.x];
+    if (rcopy && tl.y + (int)threadIdx.x < npl[tl.x]) {  // the state as it is now, in the bodies' own order
+        const size_t g = 3 * (size_t)(poff[tl.x] + tl.y + threadIdx.x);
+        for (int d = 0; d < 3; d++) {
+            rcopy[g + d] = r[g + d];
+            vcopy[g + d] = v[g + d];
+        }
+    }
     blk_sorted_prep(blockIdx.x, poff[tl.x] + tl.y + threadIdx.x, tl.y + (int)threadIdx.x < npl[tl.x], perm, r, v, renc,
                     adt, A, B, V, bounds);
 }
@@ -412,7 +419,7 @@ int sorted_set_prep(swg_ctx *c, const SortedSet &x, int nsys, bool resort, doubl
     if (resort) SWG_TRY(radial_sort_launch(c, nsys, x.nmax, x.off, x.n, x.r, x.perm));
     const float adt = (float)fabs(dt) * (1.0f + 1e-6f);
     k_sorted_prep<<<x.ntiles, SB, 0, c->stream>>>(x.tiles, x.off, x.n, x.perm, x.r, x.v, x.renc, adt, x.F, x.F + x.N,
-                                                  x.F + 2 * x.N, x.bounds);
+                                                  x.F + 2 * x.N, x.bounds, x.rcopy, x.vcopy);
     c->launches++;
     return launch_status(c, "sorted_prep");
 }
@@ -444,7 +451,7 @@ int encounter_plpl_sorted_batched(swg_ctx *c, int nsys, int nmax, const int32_t 
     if (resort) SWG_TRY(radial_sort_launch(c, nsys, nmax, poff, npl, r, perm));
     const float adt = (float)fabs(dt) * (1.0f + 1e-6f);  // |dt| rounded to float, then up
     k_sorted_prep<<<ntiles, SB, 0, c->stream>>>(tiles, poff, npl, perm, r, v, renc, adt, F, F + NPL, F + 2 * NPL,
-                                                bounds);
+                                                bounds, nullptr, nullptr);
     c->launches++;
     SWG_TRY(launch_status(c, "sorted_prep"));
     k_encounter_sorted<<<nitems, SQ, 0, c->stream>>>(items, poff, tbase, perm, F, F + NPL, F + 2 * NPL, bounds, r,

@@ -91,14 +91,15 @@ __device__ __forceinline__ int odd_disp(double &dx, double &dy, double &dz, bool
 }
 
 // Receivers [i0, i0 + RT) (those below nrecv) of one system against all its partners, whole
-// block of fp64_threads(RT) threads; sh: fp64_shared(RT) bytes.  MODE: KICK_DIRECT and
+// block of fp64_threads(RT) threads; sh: fp64_shared(RT) bytes.  kv: the velocities that the
+// finished accelerations kick (KickVel; a launch of their own took 3 us).  MODE: KICK_DIRECT and
 // KICK_SPLIT (pl-pl), KICK_TP (swiftest_kick.f90:374-415: acc -= Gm_j / (r^2 sqrt r^2)
 // (r_tp - r_j), masked).
 template <bool RAD, int MODE>
 __device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int nplm, const double *__restrict__ rr,
                                            const double *__restrict__ rp, const double *__restrict__ Gm,
                                            const double *__restrict__ R, const int32_t *__restrict__ lmask,
-                                           double *__restrict__ acc, int acc_is_zero, int i0, double *sh) {
+                                           double *__restrict__ acc, int acc_is_zero, int i0, double *sh, const KickVel &kv = KickVel()) {
     const int nth = fp64_threads(RT), ts = term_stride(RT);
     const int w = (int)(threadIdx.x >> 5) - 1, lane = threadIdx.x & 31;
     constexpr bool plpl = MODE != KICK_TP;
@@ -214,28 +215,30 @@ __device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int npl
             vb = v;
             v = 0.0;
         }
-        acc[3 * ia + d] = (acc_is_zero ? 0.0 : acc[3 * ia + d]) + v + vb;
+        v = (acc_is_zero ? 0.0 : acc[3 * ia + d]) + v + vb;
+        acc[3 * ia + d] = v;
     } else if (fold) {
         acc[3 * ia + d] = v;
     } else if (acc_is_zero) {
         acc[3 * ia + d] = 0.0;
     }
+    if (kv.v && (plpl ? kv.mask[ia] != 0 : fold)) kv.v[3 * ia + d] = kv.v[3 * ia + d] + v * kv.dt;
 }
 
 template <bool RAD, int MODE>
 __global__ void __launch_bounds__(fp64_threads(FP64_RTMAX), 4)
     k_kick_plpl_fp64(int RT, int npl, int nplm, const double *__restrict__ r, const double *__restrict__ Gm,
-                     const double *__restrict__ R, double *__restrict__ acc, int acc_is_zero) {
+                     const double *__restrict__ R, double *__restrict__ acc, int acc_is_zero, KickVel kv) {
     extern __shared__ double sh[];
-    fp64_group<RAD, MODE>(RT, npl, npl, nplm, r, r, Gm, R, nullptr, acc, acc_is_zero, blockIdx.x * RT, sh);
+    fp64_group<RAD, MODE>(RT, npl, npl, nplm, r, r, Gm, R, nullptr, acc, acc_is_zero, blockIdx.x * RT, sh, kv);
 }
 
 __global__ void __launch_bounds__(fp64_threads(FP64_RTMAX), 4)
     k_kick_tp_fp64(int RT, int ntp, int npl, const double *__restrict__ rtp, const double *__restrict__ rpl,
                    const double *__restrict__ Gm, const int32_t *__restrict__ lmask, double *__restrict__ acc,
-                   int acc_is_zero) {
+                   int acc_is_zero, KickVel kv) {
     extern __shared__ double sh[];
-    fp64_group<false, KICK_TP>(RT, ntp, npl, 0, rtp, rpl, Gm, nullptr, lmask, acc, acc_is_zero, blockIdx.x * RT, sh);
+    fp64_group<false, KICK_TP>(RT, ntp, npl, 0, rtp, rpl, Gm, nullptr, lmask, acc, acc_is_zero, blockIdx.x * RT, sh, kv);
 }
 
 // Batched (ensemble) forms: block b takes item b = (system s, first receiver r0) of a
@@ -301,31 +304,31 @@ static int fp64_rt(int num_sms, int n) {
 }
 
 int kick_plpl_fp64(swg_ctx *c, int32_t npl, int32_t nplm, const double *r, const double *Gm, const double *R,
-                   double *acc, int mode, int acc_is_zero) {
+                   double *acc, int mode, int acc_is_zero, const KickVel &kv) {
     if (npl <= 0) return SWG_OK;
     const int rt = fp64_rt(c->num_sms, npl), grid = div_up_i(npl, rt), th = fp64_threads(rt);
     const cudaStream_t st = c->stream;
     if (mode == KICK_DIRECT) {
         if (R)
-            k_kick_plpl_fp64<true, KICK_DIRECT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<true, KICK_DIRECT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero, kv);
         else
-            k_kick_plpl_fp64<false, KICK_DIRECT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<false, KICK_DIRECT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero, kv);
     } else {
         if (R)
-            k_kick_plpl_fp64<true, KICK_SPLIT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<true, KICK_SPLIT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero, kv);
         else
-            k_kick_plpl_fp64<false, KICK_SPLIT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero);
+            k_kick_plpl_fp64<false, KICK_SPLIT><<<grid, th, fp64_shared(rt), st>>>(rt, npl, nplm, r, Gm, R, acc, acc_is_zero, kv);
     }
     c->launches++;
     return launch_status(c, "kick_plpl_fp64");
 }
 
 int kick_tp_fp64(swg_ctx *c, int32_t ntp, int32_t npl, const double *rtp, const double *rpl, const double *Gm,
-                 const int32_t *lmask, double *acc, int acc_is_zero) {
+                 const int32_t *lmask, double *acc, int acc_is_zero, const KickVel &kv) {
     if (ntp <= 0) return SWG_OK;
     const int rt = fp64_rt(c->num_sms, ntp);
     k_kick_tp_fp64<<<div_up_i(ntp, rt), fp64_threads(rt), fp64_shared(rt), c->stream>>>(rt, ntp, npl, rtp, rpl, Gm, lmask, acc,
-                                                                          acc_is_zero);
+                                                                          acc_is_zero, kv);
     c->launches++;
     return launch_status(c, "kick_tp_fp64");
 }

@@ -134,10 +134,17 @@ int ensure_kick_scratch(swg_ctx *c, DevBuf &buf, size_t bytes);
 
 // kick.cu -- pair kick
 enum KickMode { KICK_DIRECT = 0, KICK_SPLIT = 1 };
+// v += acc dt for the receivers with mask (pl-pl; the test particles' kick uses its own mask), in the
+// kick's launch once acc is final; v == nullptr: no velocities
+struct KickVel {
+    double *v = nullptr;
+    const int32_t *mask = nullptr;
+    double dt = 0;
+};
 int kick_plpl_fp64(swg_ctx *c, int32_t npl, int32_t nplm, const double *r, const double *Gm, const double *R,
-                   double *acc, int mode, int acc_is_zero);
+                   double *acc, int mode, int acc_is_zero, const KickVel &kv = KickVel());
 int kick_tp_fp64(swg_ctx *c, int32_t ntp, int32_t npl, const double *rtp, const double *rpl, const double *Gm,
-                 const int32_t *lmask, double *acc, int acc_is_zero);
+                 const int32_t *lmask, double *acc, int acc_is_zero, const KickVel &kv = KickVel());
 size_t kick_mixed_scratch_bytes(int nrecv, int npart, int nchunk);
 int kick_mixed_nchunk(int num_sms, int nrecv, int npart);
 int kick_mixed_chunks(swg_ctx *c, int nrecv, int npart);
@@ -324,6 +331,7 @@ struct SortedSet {
     const int32_t *tbase = nullptr;
     float4 *bounds = nullptr;
     int nmax = 0;
+    double *rcopy = nullptr, *vcopy = nullptr;  // with both, the preparation copies r and v there
 };
 // resort: refresh the order; then the float copies and bounds from the current state
 int sorted_set_prep(swg_ctx *c, const SortedSet &x, int nsys, bool resort, double dt);

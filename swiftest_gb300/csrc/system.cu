@@ -75,11 +75,14 @@ struct swg_system {
     // SyMBA: the level-0 checks and the test particles' half-steps run on a second stream
     // beside the massive bodies' (events: 0 opening ready, 1 tp opening done, 2 closing
     // ready, 3 central-body drift ready, 4 tp closing done, 5 level-0 lists ready, 6 recursion
-    // about to start)
+    // about to start; HELIO steps in a row: 7 shared records read by the test particles, 8 discard
+    // scan done)
     cudaStream_t side = nullptr, side2 = nullptr;  // side2: the pl-tp check beside the pl-pl one on side
-    cudaEvent_t ev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev[9] = {};
+    bool behind = false;  // within swg_system_step: the last step's discard scan is still on side
     DevBuf tmask;  // masks of the listed and the other test particles
-    DevBuf snap;  // the start-of-step rh, vb, trh, tvb that the overlapped level-0 checks read
+    DevBuf snap;  // SyMBA: the start-of-step rh, vb, trh, tvb that the overlapped level-0 checks
+                  // read; HELIO: the end-of-step rh, vh that the discard scan reads
     int32_t *h_flags = nullptr;  // pinned: [0] lencounter, [1] nfail, [2] recursion status, [3] deepest level,
                                  // [4] collision pending
     int32_t *mark_pl = nullptr, *mark_tp = nullptr, *rec_out = nullptr, *rec_resume = nullptr;
@@ -319,7 +322,8 @@ int pair_scratch(swg_system *s, double **p) {
 }
 
 // pl-pl interaction accelerations (swiftest_kick.f90:12-43 / symba_kick.f90:14-33), acc starts at zero
-int accel_int_pl(swg_system *s, int acc_is_zero) {
+// kv: velocities to kick in the same launch (FP64 path)
+int accel_int_pl(swg_system *s, int acc_is_zero, const KickVel &kv = KickVel()) {
     swg_ctx *c = s->c;
     const bool symba = s->integrator == SWG_SYMBA;
     const double *rad = (symba || s->lclose) ? s->radius : nullptr;
@@ -334,7 +338,7 @@ int accel_int_pl(swg_system *s, int acc_is_zero) {
     }
     // flat, or triangular with GMTINY bodies dominating -> symmetric (split) sums
     const int mode = (s->loop_mode == 1 || (s->npl - nplm) > nplm) ? KICK_SPLIT : KICK_DIRECT;
-    return kick_plpl_fp64(c, s->npl, nplm, s->rh, s->Gmass, rad, s->ah, mode, acc_is_zero);
+    return kick_plpl_fp64(c, s->npl, nplm, s->rh, s->Gmass, rad, s->ah, mode, acc_is_zero, kv);
 }
 
 // helio_kick_vb_pl (helio_kick.f90:91-132) with symba_kick_getacch_pl (symba_kick.f90:36-76);
@@ -344,10 +348,14 @@ int accel_int_pl(swg_system *s, int acc_is_zero) {
 int kick_vb_pl(swg_system *s, double dt, int lbeg, bool copy_r = true, bool have_acc = false) {
     swg_ctx *c = s->c;
     if (s->npl == 0) return SWG_OK;
+    copy_r = copy_r && s->ntp > 0;
+    // without encounter pairs to subtract the accelerations are final in the kick's launch
+    const bool fused = exact(s) && !have_acc && !copy_r && !(s->integrator == SWG_SYMBA && s->plpl_n > 0);
     if (!have_acc) {
         ProfScope ps(s->prof, s->c->stream, PROF_KICK_PL);
-        SWG_TRY(accel_int_pl(s, 1));
+        SWG_TRY(accel_int_pl(s, 1, fused ? KickVel{s->vb, s->lmask, dt} : KickVel()));
     }
+    if (fused) return SWG_OK;
     if (s->integrator == SWG_SYMBA && s->plpl_n > 0) {
         double *scr;
         SWG_TRY(pair_scratch(s, &scr));
@@ -367,6 +375,8 @@ int kick_vb_tp(swg_system *s, double dt, int lbeg, const int32_t *mask = nullptr
     if (s->ntp == 0) return SWG_OK;
     if (!mask) mask = s->tlmask;
     const double *rp = lbeg ? s->rbeg : s->rend;
+    const bool back = addback && s->integrator == SWG_SYMBA && s->pltp_n > 0;
+    const bool fused = exact(s) && s->npl > 0 && !back;
     if (s->npl > 0) {
         ProfScope ps(s->prof, s->c->stream, PROF_KICK_TP);
         if (s->precision == SWG_MIXED) {
@@ -375,12 +385,14 @@ int kick_vb_tp(swg_system *s, double dt, int lbeg, const int32_t *mask = nullptr
             SWG_TRY(kick_mixed_launch(c, true, s->ntp, s->npl, 0, s->trh, rp, s->Gmass, nullptr, mask, s->tah,
                                       1, nch, s->kick_scratch_tp.ptr));
         } else {
-            SWG_TRY(kick_tp_fp64(c, s->ntp, s->npl, s->trh, rp, s->Gmass, mask, s->tah, 1));
+            SWG_TRY(kick_tp_fp64(c, s->ntp, s->npl, s->trh, rp, s->Gmass, mask, s->tah, 1,
+                                 fused ? KickVel{s->tvb, mask, dt} : KickVel()));
         }
     } else {
         SWG_TRY(cuda_status(c, cudaMemsetAsync(s->tah, 0, sizeof(double) * 3 * s->ntp, c->stream), "memset"));
     }
-    if (addback && s->integrator == SWG_SYMBA && s->pltp_n > 0) {
+    if (fused) return SWG_OK;
+    if (back) {
         if (s->pltp_n <= ADDBACK_SMALL)
             k_pltp_addback_small<<<1, ADDBACK_SMALL, 0, c->stream>>>((int)s->pltp_n, s->pltp_l,
                                                                       s->pltp_l + s->pltp_cap, s->tlmask, s->trh, rp,
@@ -510,16 +522,18 @@ int copy_positions(swg_system *s, double *to) {
 }
 // The closing half of a step whose test particles are on the side stream (their closing kick
 // queued): the massive bodies' closing kick and sums here, the test particles' closing linear
-// drift once the central-body record is there, then both joined.
-int close_half(swg_system *s, double dth) {
+// drift once the central-body record is there, then both joined (aside: left apart, event 7
+// marks the test particles' last read of the shared records).
+int close_half(swg_system *s, double dth, bool aside = false) {
     swg_ctx *c = s->c;
     SWG_TRY(kick_vb_pl(s, dth, 0, false));
     if (exact(s)) SWG_TRY(close_pl(s, dth));
     else SWG_TRY(lindrift_pl(s, dth, 0));
     SWG_TRY(join(c, c->stream, s->side, s->ev[3]));
     SWG_TRY(on_stream(c, s->side, [&] { return tp_misc(s, CB_PTEND, dth, 3); }));
+    if (aside) SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[7], s->side), "event"));
     if (!exact(s)) SWG_TRY(vb2vh_pl(s));
-    return join(c, s->side, c->stream, s->ev[4]);
+    return aside ? SWG_OK : join(c, s->side, c->stream, s->ev[4]);
 }
 
 // helio_step_pl / _tp (helio_step.f90:37-119) via whm_step_system (whm_step.f90:14-35)
@@ -527,14 +541,17 @@ int close_half(swg_system *s, double dth) {
 // With test particles their half-steps run on a second stream beside the massive bodies'
 // (reading the positions recorded in rbeg / rend and the central-body record), as in
 // symba_interp; each kernel's arithmetic is unchanged.
-int helio_step(swg_system *s, double dt, bool opened = false) {
+// aside: the streams stay apart at the end (discard_aside and join_aside follow)
+bool helio_fork(const swg_system *s) { return s->ntp > 0 && s->npl > 0 && !s->prof.on; }
+int helio_step(swg_system *s, double dt, bool opened = false, bool aside = false) {
     swg_ctx *c = s->c;
     const double dth = 0.5 * dt;
     s->lfirst_tp = s->lfirst_pl;
-    const bool fork = s->ntp > 0 && s->npl > 0 && !s->prof.on;
     const int first_mode = s->lfirst_tp ? 4 : 2;
-    if (fork) {
+    if (helio_fork(s)) {
         SWG_TRY(ensure_side(s));
+        // the last step's test particles have read rbeg, rend and the central-body record
+        if (s->behind) SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[7], 0), "event"));
         if (s->lfirst_pl && !opened) SWG_TRY(vh2vb_pl(s));
         s->lfirst_pl = s->lfirst_tp = 0;
         if (!opened) SWG_TRY(lindrift_pl(s, dth, 1));
@@ -550,7 +567,7 @@ int helio_step(swg_system *s, double dt, bool opened = false) {
         SWG_TRY(copy_positions(s, s->rend));
         SWG_TRY(join(c, c->stream, s->side, s->ev[2]));
         SWG_TRY(on_stream(c, s->side, [&] { return kick_vb_tp(s, dth, 0); }));
-        return close_half(s, dth);
+        return close_half(s, dth, aside);
     }
     if (s->npl > 0) {
         if (s->lfirst_pl) {
@@ -1151,6 +1168,16 @@ int symba_interp(swg_system *s, double dt, bool opened = false) {
     return SWG_OK;
 }
 
+// the close-approach scan over the two sets and its outcome, on the context's stream
+int discard_scan(swg_system *s, const SortedSet &pl, const SortedSet &tp) {
+    swg_ctx *c = s->c;
+    SWG_TRY(pltp_sorted_batched(c, true, pl, tp, s->tstatus, s->srt->nitems, s->srt->items, s->dt, 0, nullptr, nullptr,
+                                nullptr, nullptr, s->tflag, s->srt->pchunk));
+    k_apply_discard<<<grid_for(s->ntp, 256), 256, 0, c->stream>>>(s->ntp, s->tflag, s->tstatus, s->tlmask, s->trh,
+                                                                  s->tvh, s->tvb, s->npl, nullptr, nullptr, nullptr,
+                                                                  s->ndiscard);
+    return L(c, "apply_discard");
+}
 // swiftest_discard_pl_tp (src/swiftest/swiftest_discard.f90:244-290), run after each step
 // when close encounters are checked (param%lclose), as the reference's main loop
 // (swiftest_driver) does after every step.
@@ -1163,12 +1190,39 @@ int discard_step(swg_system *s) {
     const SortedSet pl = sorted_pl(s, s->rh, s->vh, s->radius), tp = sorted_tp(s, s->trh, s->tvh);
     SWG_TRY(sorted_set_prep(c, pl, 1, s->srt->npl_prep++ % 8 == 0, s->dt));
     SWG_TRY(sorted_set_prep(c, tp, 1, s->srt->ntp_prep++ % 32 == 0, s->dt));
-    SWG_TRY(pltp_sorted_batched(c, true, pl, tp, s->tstatus, s->srt->nitems, s->srt->items, s->dt, 0, nullptr, nullptr,
-                                nullptr, nullptr, s->tflag, s->srt->pchunk));
-    k_apply_discard<<<grid_for(s->ntp, 256), 256, 0, c->stream>>>(s->ntp, s->tflag, s->tstatus, s->tlmask, s->trh,
-                                                                  s->tvh, s->tvb, s->npl, nullptr, nullptr, nullptr,
-                                                                  s->ndiscard);
-    return L(c, "apply_discard");
+    return discard_scan(s, pl, tp);
+}
+
+// discard_step after a HELIO step left apart: the massive bodies' sorted set here, with a copy of
+// their state for the exact tests, the rest on the test particles' stream, beside the massive
+// bodies' next step (which no test particle concerns): 100 pl x 1000 tp, 92 -> 70 us a step with
+// the velocity updates in the kicks' launches.  Event 8: the scan has read the set and the copy.
+int discard_aside(swg_system *s) {
+    swg_ctx *c = s->c;
+    const size_t n = s->npl;
+    SWG_TRY(ensure(c, s->snap, sizeof(double) * 6 * n));
+    SortedSet pl = sorted_pl(s, s->rh, s->vh, s->radius);
+    pl.rcopy = (double *)s->snap.ptr;
+    pl.vcopy = pl.rcopy + 3 * n;
+    if (s->behind) SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[8], 0), "event"));
+    SWG_TRY(sorted_set_prep(c, pl, 1, s->srt->npl_prep++ % 8 == 0, s->dt));
+    pl.r = pl.rcopy;
+    pl.v = pl.vcopy;
+    SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[4], c->stream), "event"));
+    s->behind = true;
+    return on_stream(c, s->side, [&] {
+        const SortedSet tp = sorted_tp(s, s->trh, s->tvh);
+        SWG_TRY(sorted_set_prep(c, tp, 1, s->srt->ntp_prep++ % 32 == 0, s->dt));
+        SWG_TRY(cuda_status(c, cudaStreamWaitEvent(s->side, s->ev[4], 0), "event"));
+        SWG_TRY(discard_scan(s, pl, tp));
+        return cuda_status(c, cudaEventRecord(s->ev[8], s->side), "event");
+    });
+}
+// what a step left on the side stream joins the context's stream
+int join_aside(swg_system *s) {
+    if (!s->behind) return SWG_OK;
+    s->behind = false;
+    return join(s->c, s->side, s->c->stream, s->ev[4]);
 }
 
 // symba_step_system (symba_step.f90:14-52); both level-0 checks are evaluated
@@ -1421,25 +1475,35 @@ int swg_system_initialize(swg_system *s) {
     return cuda_status(c, cudaStreamSynchronize(c->stream), "init");
 }
 
-int swg_system_step(swg_system *s, int32_t nsteps) {
-    if (!s || !s->initialized) return SWG_ERR_STATE;
-    s->h_flags[2] = 0;
+static int steps(swg_system *s, int32_t nsteps) {
+    // HELIO: the test particles' discard scan runs beside the massive bodies' next step
+    const bool aside = s->integrator == SWG_HELIO && s->lclose && helio_fork(s);
+    if (aside) SWG_TRY(ensure_sorted(s));
     for (int32_t k = 0; k < nsteps; k++) {
         int rc;
         if (s->integrator == SWG_WHM)
             rc = whm_step(s, s->dt);
         else if (s->integrator == SWG_HELIO)
-            rc = helio_step(s, s->dt);
+            rc = helio_step(s, s->dt, false, aside);
         else
             rc = symba_step(s, s->dt);
         if (rc != SWG_OK) return rc;
-        SWG_TRY(discard_step(s));
+        SWG_TRY(aside ? discard_aside(s) : discard_step(s));
         if (s->h_flags[2] != 0) {  // recursion status of an earlier step, seen at a sync point
             s->c->err = "SyMBA local time step too small";
             return s->h_flags[2];
         }
         s->t += s->dt;
     }
+    return SWG_OK;
+}
+
+int swg_system_step(swg_system *s, int32_t nsteps) {
+    if (!s || !s->initialized) return SWG_ERR_STATE;
+    s->h_flags[2] = 0;
+    const int rc = steps(s, nsteps), joined = join_aside(s);
+    if (rc != SWG_OK) return rc;
+    SWG_TRY(joined);
     if (s->integrator == SWG_SYMBA) {
         SWG_TRY(cuda_status(s->c, cudaStreamSynchronize(s->c->stream), "step"));
         if (s->h_flags[2] != 0) {
