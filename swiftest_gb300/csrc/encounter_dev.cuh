@@ -64,17 +64,19 @@ struct BodyF {
     float4 v;  // vx, vy, vz, |v|
 };
 
-__device__ __forceinline__ BodyF load_body(const double *r, const double *v, const double *renc, int i) {
+__device__ __forceinline__ BodyF make_body(double x, double y, double z, double u, double v, double w, float renc) {
     BodyF o;
-    const double x = r[3 * i], y = r[3 * i + 1], z = r[3 * i + 2];
     const float xh = __double2float_rn(x), yh = __double2float_rn(y), zh = __double2float_rn(z);
-    o.a = make_float4(xh, yh, zh, renc ? __double2float_rn(renc[i]) : 0.f);
+    o.a = make_float4(xh, yh, zh, renc);
     o.b = make_float4(__double2float_rn(x - (double)xh), __double2float_rn(y - (double)yh),
                       __double2float_rn(z - (double)zh), sqrtf(xh * xh + yh * yh + zh * zh));
-    const float vx = __double2float_rn(v[3 * i]), vy = __double2float_rn(v[3 * i + 1]),
-                vz = __double2float_rn(v[3 * i + 2]);
+    const float vx = __double2float_rn(u), vy = __double2float_rn(v), vz = __double2float_rn(w);
     o.v = make_float4(vx, vy, vz, sqrtf(vx * vx + vy * vy + vz * vz));
     return o;
+}
+__device__ __forceinline__ BodyF load_body(const double *r, const double *v, const double *renc, int i) {
+    return make_body(r[3 * i], r[3 * i + 1], r[3 * i + 2], v[3 * i], v[3 * i + 1], v[3 * i + 2],
+                     renc ? __double2float_rn(renc[i]) : 0.f);
 }
 
 // True when the pair certainly fails encounter_check_one.  The FP64 test accepts a

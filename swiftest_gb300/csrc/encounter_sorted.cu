@@ -141,14 +141,13 @@ __global__ void __launch_bounds__(RS_T) k_radial_sort(const int32_t *__restrict_
 // float copies in sorted order and the bounds (min lo, max hi, max renc), rounded outward,
 // of each 32-body half u of the tile (bounds[2 t + u]; a half without bodies gets
 // (+inf, -inf, 0), which is apart from everything).
-__device__ __forceinline__ void blk_sorted_prep(int tile, int p, bool in, const int32_t *__restrict__ perm,
-                                                const double *__restrict__ r, const double *__restrict__ v,
-                                                const double *__restrict__ renc, float adt, float4 *A, float4 *B,
-                                                float4 *V, float4 *bounds) {
+// load(g): body g's float copies.
+template <class F>
+__device__ __forceinline__ void blk_sorted_prep(int tile, int p, bool in, const int32_t *__restrict__ perm, F load,
+                                                float adt, float4 *A, float4 *B, float4 *V, float4 *bounds) {
     float lo = __int_as_float(0x7f800000), hi = -__int_as_float(0x7f800000), Rm = 0.f;
     if (in) {
-        const int g = perm[p];
-        const BodyF o = load_body(r, v, renc, g);
+        const BodyF o = load(perm[p]);
         A[p] = o.a;
         B[p] = o.b;
         V[p] = o.v;
@@ -180,16 +179,33 @@ __global__ void __launch_bounds__(SB) k_sorted_prep(const int2 *__restrict__ til
                                                     const int32_t *__restrict__ npl, const int32_t *__restrict__ perm,
                                                     const double *__restrict__ r, const double *__restrict__ v,
                                                     const double *__restrict__ renc, float adt, float4 *A, float4 *B,
-                                                    float4 *V, float4 *bounds, double *rcopy, double *vcopy) {
+                                                    float4 *V, float4 *bounds) {
     const int2 tl = tiles[blockIdx.x];
-    if (rcopy && tl.y + (int)threadIdx.x < npl[tl.x]) {  // the state as it is now, in the bodies' own order
-        const size_t g = 3 * (size_t)(poff[tl.x] + tl.y + threadIdx.x);
-        for (int d = 0; d < 3; d++) {
-            rcopy[g + d] = r[g + d];
-            vcopy[g + d] = v[g + d];
-        }
-    }
-    blk_sorted_prep(blockIdx.x, poff[tl.x] + tl.y + threadIdx.x, tl.y + (int)threadIdx.x < npl[tl.x], perm, r, v, renc,
+    blk_sorted_prep(blockIdx.x, poff[tl.x] + tl.y + threadIdx.x, tl.y + (int)threadIdx.x < npl[tl.x], perm,
+                    [&](int g) { return load_body(r, v, renc, g); }, adt, A, B, V, bounds);
+}
+// The same for the test particles of one system at the end of a step, whose closing linear drift
+// and heliocentric velocities are formed on the way (r and v change: no read-only loads).
+__global__ void __launch_bounds__(SB) k_sorted_prep_close(const int2 *__restrict__ tiles, int n,
+                                                          const int32_t *__restrict__ perm, TpClose c, double *r,
+                                                          double *v, float adt, float4 *A, float4 *B, float4 *V,
+                                                          float4 *bounds) {
+    const int p = tiles[blockIdx.x].y + (int)threadIdx.x;
+    blk_sorted_prep(blockIdx.x, p, p < n, perm,
+                    [&](int g) {
+                        double x[3], u[3];
+                        for (int d = 0; d < 3; d++) {
+                            x[d] = r[3 * g + d];
+                            u[d] = v[3 * g + d];
+                        }
+                        if (c.mask[g])
+                            for (int d = 0; d < 3; d++) {
+                                const double pt = c.pt[d], vbcb = -pt;
+                                r[3 * g + d] = x[d] = x[d] + pt * c.dt;
+                                v[3 * g + d] = u[d] = c.vb[3 * g + d] - vbcb;
+                            }
+                        return make_body(x[0], x[1], x[2], u[0], u[1], u[2], 0.f);
+                    },
                     adt, A, B, V, bounds);
 }
 
@@ -419,9 +435,18 @@ int sorted_set_prep(swg_ctx *c, const SortedSet &x, int nsys, bool resort, doubl
     if (resort) SWG_TRY(radial_sort_launch(c, nsys, x.nmax, x.off, x.n, x.r, x.perm));
     const float adt = (float)fabs(dt) * (1.0f + 1e-6f);
     k_sorted_prep<<<x.ntiles, SB, 0, c->stream>>>(x.tiles, x.off, x.n, x.perm, x.r, x.v, x.renc, adt, x.F, x.F + x.N,
-                                                  x.F + 2 * x.N, x.bounds, x.rcopy, x.vcopy);
+                                                  x.F + 2 * x.N, x.bounds);
     c->launches++;
     return launch_status(c, "sorted_prep");
+}
+
+int sorted_tp_close(swg_ctx *c, const SortedSet &x, const TpClose &k, double *r, double *v, double dt) {
+    if (x.ntiles <= 0) return SWG_OK;
+    const float adt = (float)fabs(dt) * (1.0f + 1e-6f);
+    k_sorted_prep_close<<<x.ntiles, SB, 0, c->stream>>>(x.tiles, (int)x.N, x.perm, k, r, v, adt, x.F, x.F + x.N,
+                                                        x.F + 2 * x.N, x.bounds);
+    c->launches++;
+    return launch_status(c, "sorted_prep_close");
 }
 
 int pltp_sorted_batched(swg_ctx *c, bool discard, const SortedSet &pl, const SortedSet &tp, const int32_t *tstatus,
@@ -451,7 +476,7 @@ int encounter_plpl_sorted_batched(swg_ctx *c, int nsys, int nmax, const int32_t 
     if (resort) SWG_TRY(radial_sort_launch(c, nsys, nmax, poff, npl, r, perm));
     const float adt = (float)fabs(dt) * (1.0f + 1e-6f);  // |dt| rounded to float, then up
     k_sorted_prep<<<ntiles, SB, 0, c->stream>>>(tiles, poff, npl, perm, r, v, renc, adt, F, F + NPL, F + 2 * NPL,
-                                                bounds, nullptr, nullptr);
+                                                bounds);
     c->launches++;
     SWG_TRY(launch_status(c, "sorted_prep"));
     k_encounter_sorted<<<nitems, SQ, 0, c->stream>>>(items, poff, tbase, perm, F, F + NPL, F + 2 * NPL, bounds, r,
@@ -490,8 +515,11 @@ __global__ void __launch_bounds__(SB) k_one_prep(OneLists l, float adt, int nite
     const bool first = (int)blockIdx.x < l.nt1;
     const int tile = (int)blockIdx.x - (first ? 0 : l.nt1), n = first ? l.n1 : l.n2, p = tile * SB + (int)threadIdx.x;
     float4 *F = first ? l.F1 : l.F2;
-    blk_sorted_prep(tile, p, p < n, first ? l.perm1 : l.perm2, first ? l.r1 : l.r2, first ? l.v1 : l.v2,
-                    first ? l.renc1 : nullptr, adt, F, F + n, F + 2 * (size_t)n, first ? l.b1 : l.b2);
+    blk_sorted_prep(tile, p, p < n, first ? l.perm1 : l.perm2,
+                    [&](int g) {
+                        return load_body(first ? l.r1 : l.r2, first ? l.v1 : l.v2, first ? l.renc1 : nullptr, g);
+                    },
+                    adt, F, F + n, F + 2 * (size_t)n, first ? l.b1 : l.b2);
     const int nr = l.n2 ? l.n2 : l.n1;
     for (int i = blockIdx.x * SB + threadIdx.x; i < nitems; i += gridDim.x * SB) {
         const int q0 = i / nchunk * SQ;

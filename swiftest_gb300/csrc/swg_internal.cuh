@@ -331,10 +331,17 @@ struct SortedSet {
     const int32_t *tbase = nullptr;
     float4 *bounds = nullptr;
     int nmax = 0;
-    double *rcopy = nullptr, *vcopy = nullptr;  // with both, the preparation copies r and v there
 };
 // resort: refresh the order; then the float copies and bounds from the current state
 int sorted_set_prep(swg_ctx *c, const SortedSet &x, int nsys, bool resort, double dt);
+// one system's test particles at the end of a step: with mask, r += pt dt and v = vb + pt
+// (k_tp_misc's closing form), then the preparation (the order as it is) over step dt
+struct TpClose {
+    const int32_t *mask;
+    const double *vb, *pt;
+    double dt;
+};
+int sorted_tp_close(swg_ctx *c, const SortedSet &x, const TpClose &k, double *r, double *v, double dt);
 // pl-tp over radius-sorted tiles (both sets prepared at the current state): the level-0
 // pl-tp check (pairs (pl, tp), global 1-based, into o1/o2/olv/count) or, discard, the
 // close-approach scan of swiftest_discard_pl_tp (flag[tp] = 1; tp renc = pl radius).

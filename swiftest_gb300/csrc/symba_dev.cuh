@@ -263,10 +263,13 @@ static __device__ void blk_vb2vh_pl(int npl, const double *__restrict__ Gm,
 
 // The end of a step in the FP64 path: helio_drift_linear_pl, then swiftest_util_coord_vb2vh_pl.  The
 // linear drift leaves vb as it is, so both sums (one forward, one in reverse order) run
-// together, six lanes in one addition.
+// together, six lanes in one addition.  rcopy, vcopy: copies of the resulting state.  rnext: the
+// opening linear drift of a step that follows at once, whose sum is the closing one's (vb, the
+// masses and the mask are as they were), and its positions there.
 static __device__ void blk_close_pl(int npl, const double *__restrict__ Gm, const double *__restrict__ vb,
                                     const int32_t *__restrict__ lmask, const int32_t *__restrict__ status,
-                                    double GMcb, double *rh, double *vh, double dt, double *dcb, SumScratch &sh) {
+                                    double GMcb, double *rh, double *vh, double dt, double *dcb, SumScratch &sh,
+                                    double *rcopy = nullptr, double *vcopy = nullptr, double *rnext = nullptr) {
     blk_serial_sums<6>(
         npl, false,
         [&](int i, double *t) {
@@ -288,16 +291,31 @@ static __device__ void blk_close_pl(int npl, const double *__restrict__ Gm, cons
         dcb[CB_VB + 0] = c.x;
         dcb[CB_VB + 1] = c.y;
         dcb[CB_VB + 2] = c.z;
-    }
-    for (int i = threadIdx.x; i < npl; i += blockDim.x) {
-        if (lmask[i]) {
-            rh[3 * i + 0] = rh[3 * i + 0] + pt.x * dt;
-            rh[3 * i + 1] = rh[3 * i + 1] + pt.y * dt;
-            rh[3 * i + 2] = rh[3 * i + 2] + pt.z * dt;
+        if (rnext) {
+            dcb[CB_PTBEG + 0] = pt.x;
+            dcb[CB_PTBEG + 1] = pt.y;
+            dcb[CB_PTBEG + 2] = pt.z;
         }
-        vh[3 * i + 0] = vb[3 * i + 0] - c.x;
-        vh[3 * i + 1] = vb[3 * i + 1] - c.y;
-        vh[3 * i + 2] = vb[3 * i + 2] - c.z;
+    }
+    const double p[3] = {pt.x, pt.y, pt.z}, cv[3] = {c.x, c.y, c.z};
+    for (int i = threadIdx.x; i < npl; i += blockDim.x) {
+        const bool on = lmask[i] != 0;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            double x = rh[3 * i + d];
+            const double v = vb[3 * i + d] - cv[d];
+            if (on) x = x + p[d] * dt;
+            vh[3 * i + d] = v;
+            if (rcopy) {
+                rcopy[3 * i + d] = x;
+                vcopy[3 * i + d] = v;
+            }
+            if (rnext) {
+                if (on) x = x + p[d] * dt;
+                rnext[3 * i + d] = x;
+            }
+            rh[3 * i + d] = x;
+        }
     }
 }
 
@@ -2171,12 +2189,20 @@ static __global__ void k_set_renc(int npl, const double *rhill, double rhscale, 
 // system: status INACTIVE, masked, parked with no velocity at 1e6 AU + (npl + local index)
 // (the reference spills them out of its arrays).  tsys/toff/npls (optional) give each
 // test particle's system in a CSR-packed ensemble; otherwise one system of npl bodies.
+// pt (one system): the others' opening linear drift of the step that follows (its
+// central-body drift).
 static __global__ void k_apply_discard(int64_t ntp, int32_t *flag, int32_t *tstatus, int32_t *tlmask, double *trh,
                                        double *tvh, double *tvb, int npl, const int32_t *__restrict__ tsys,
                                        const int32_t *__restrict__ toff, const int32_t *__restrict__ npls,
-                                       unsigned long long *count) {
+                                       unsigned long long *count, const double *__restrict__ pt = nullptr,
+                                       double dt = 0.0) {
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= ntp || !flag[j]) return;
+    if (j >= ntp) return;
+    if (!flag[j]) {
+        if (pt && tlmask[j])
+            for (int d = 0; d < 3; d++) trh[3 * j + d] = trh[3 * j + d] + pt[d] * dt;
+        return;
+    }
     flag[j] = 0;
     int64_t slot = npl + j;
     if (tsys) {

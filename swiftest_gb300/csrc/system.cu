@@ -75,14 +75,18 @@ struct swg_system {
     // SyMBA: the level-0 checks and the test particles' half-steps run on a second stream
     // beside the massive bodies' (events: 0 opening ready, 1 tp opening done, 2 closing
     // ready, 3 central-body drift ready, 4 tp closing done, 5 level-0 lists ready, 6 recursion
-    // about to start; HELIO steps in a row: 7 shared records read by the test particles, 8 discard
-    // scan done)
+    // about to start; HELIO steps in a row: 4 massive bodies' state ready for the
+    // scan, 5 their sorted set, 7 shared records read by the test particles, 8 discard scan done)
     cudaStream_t side = nullptr, side2 = nullptr;  // side2: the pl-tp check beside the pl-pl one on side
     cudaEvent_t ev[9] = {};
-    bool behind = false;  // within swg_system_step: the last step's discard scan is still on side
+    // within swg_system_step: the last step's discard scan is still on side; the next step's
+    // opening linear drifts are done
+    bool behind = false, ahead = false;
     DevBuf tmask;  // masks of the listed and the other test particles
     DevBuf snap;  // SyMBA: the start-of-step rh, vb, trh, tvb that the overlapped level-0 checks
                   // read; HELIO: the end-of-step rh, vh that the discard scan reads
+    double *rscan() const { return (double *)snap.ptr; }
+    double *vscan() const { return rscan() + 3 * (size_t)npl; }
     int32_t *h_flags = nullptr;  // pinned: [0] lencounter, [1] nfail, [2] recursion status, [3] deepest level,
                                  // [4] collision pending
     int32_t *mark_pl = nullptr, *mark_tp = nullptr, *rec_out = nullptr, *rec_resume = nullptr;
@@ -140,9 +144,10 @@ __global__ void __launch_bounds__(RB) k_vb2vh_pl(int npl, const double *__restri
 __global__ void __launch_bounds__(RB) k_close_pl(int npl, const double *__restrict__ Gm,
                                                  const double *__restrict__ vb, const int32_t *__restrict__ lmask,
                                                  const int32_t *__restrict__ status, double GMcb, double *rh,
-                                                 double *vh, double dt, double *dcb) {
+                                                 double *vh, double dt, double *dcb, double *rcopy, double *vcopy,
+                                                 double *rnext) {
     __shared__ SumScratch sh;
-    blk_close_pl(npl, Gm, vb, lmask, status, GMcb, rh, vh, dt, dcb, sh);
+    blk_close_pl(npl, Gm, vb, lmask, status, GMcb, rh, vh, dt, dcb, sh, rcopy, vcopy, rnext);
 }
 
 // test particles: mode 0 vh2vb(vbcb=-pt) ; 1 vb2vh(vbcb=-pt) ; 2 lindrift rh += pt*dt ;
@@ -464,15 +469,21 @@ int vb2vh_pl(swg_system *s) {
     k_vb2vh_pl<<<1, RB, 0, s->c->stream>>>(s->npl, s->Gmass, s->vb, s->status, s->vh, s->GMcb, s->dcb, exact(s));
     return L(s->c, "vb2vh_pl");
 }
+// Steps in a row whose discard scan runs beside the next step (discard_aside): the state that
+// the scan reads, and (FP64 path) the next step's opening linear drift in the closing kernel.
+struct Aside {
+    bool on = false, next = false;  // next: another step of the same length follows
+};
 // the closing linear drift and vb2vh (one launch in the FP64 path)
-int close_pl(swg_system *s, double dt) {
+int close_pl(swg_system *s, double dt, const Aside &aside = Aside()) {
     if (s->npl == 0) return SWG_OK;
     if (!exact(s)) {
         SWG_TRY(lindrift_pl(s, dt, 0));
         return vb2vh_pl(s);
     }
     k_close_pl<<<1, RB, 0, s->c->stream>>>(s->npl, s->Gmass, s->vb, s->lmask, s->status, s->GMcb, s->rh, s->vh, dt,
-                                            s->dcb);
+                                            s->dcb, aside.on ? s->rscan() : nullptr, aside.on ? s->vscan() : nullptr,
+                                            aside.next ? s->rbeg : nullptr);
     return L(s->c, "close_pl");
 }
 // drift with the SyMBA level mask (levelg == irec) or the plain status mask
@@ -522,18 +533,22 @@ int copy_positions(swg_system *s, double *to) {
 }
 // The closing half of a step whose test particles are on the side stream (their closing kick
 // queued): the massive bodies' closing kick and sums here, the test particles' closing linear
-// drift once the central-body record is there, then both joined (aside: left apart, event 7
-// marks the test particles' last read of the shared records).
-int close_half(swg_system *s, double dth, bool aside = false) {
+// drift once the central-body record is there, then both joined (aside: left apart, the test
+// particles' closing to discard_aside).
+int close_half(swg_system *s, double dth, const Aside &aside = Aside()) {
     swg_ctx *c = s->c;
     SWG_TRY(kick_vb_pl(s, dth, 0, false));
-    if (exact(s)) SWG_TRY(close_pl(s, dth));
+    if (exact(s) && aside.on) {
+        // the test particles' opening kick has read rbeg, the last scan its copies
+        SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[1], 0), "event"));
+        if (s->behind) SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[8], 0), "event"));
+    }
+    if (exact(s)) SWG_TRY(close_pl(s, dth, aside));
     else SWG_TRY(lindrift_pl(s, dth, 0));
     SWG_TRY(join(c, c->stream, s->side, s->ev[3]));
-    SWG_TRY(on_stream(c, s->side, [&] { return tp_misc(s, CB_PTEND, dth, 3); }));
-    if (aside) SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[7], s->side), "event"));
+    if (!aside.on) SWG_TRY(on_stream(c, s->side, [&] { return tp_misc(s, CB_PTEND, dth, 3); }));
     if (!exact(s)) SWG_TRY(vb2vh_pl(s));
-    return aside ? SWG_OK : join(c, s->side, c->stream, s->ev[4]);
+    return aside.on ? SWG_OK : join(c, s->side, c->stream, s->ev[4]);
 }
 
 // helio_step_pl / _tp (helio_step.f90:37-119) via whm_step_system (whm_step.f90:14-35)
@@ -541,29 +556,39 @@ int close_half(swg_system *s, double dth, bool aside = false) {
 // With test particles their half-steps run on a second stream beside the massive bodies'
 // (reading the positions recorded in rbeg / rend and the central-body record), as in
 // symba_interp; each kernel's arithmetic is unchanged.
-// aside: the streams stay apart at the end (discard_aside and join_aside follow)
+// aside: the streams stay apart at the end (discard_aside and join_aside follow); s->ahead: the
+// last step's closing kernels took this one's opening linear drifts.
 bool helio_fork(const swg_system *s) { return s->ntp > 0 && s->npl > 0 && !s->prof.on; }
-int helio_step(swg_system *s, double dt, bool opened = false, bool aside = false) {
+int helio_step(swg_system *s, double dt, bool opened = false, const Aside &aside = Aside()) {
     swg_ctx *c = s->c;
     const double dth = 0.5 * dt;
     s->lfirst_tp = s->lfirst_pl;
     const int first_mode = s->lfirst_tp ? 4 : 2;
     if (helio_fork(s)) {
         SWG_TRY(ensure_side(s));
-        // the last step's test particles have read rbeg, rend and the central-body record
-        if (s->behind) SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[7], 0), "event"));
-        if (s->lfirst_pl && !opened) SWG_TRY(vh2vb_pl(s));
+        // what the last step's test particles read: the central-body record, rbeg and rend
+        auto read = [&] {
+            return s->behind ? cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[7], 0), "event") : SWG_OK;
+        };
+        const bool ahead = s->ahead;
+        s->ahead = false;
+        if (!ahead) {
+            SWG_TRY(read());
+            if (s->lfirst_pl && !opened) SWG_TRY(vh2vb_pl(s));
+            if (!opened) SWG_TRY(lindrift_pl(s, dth, 1));
+            SWG_TRY(copy_positions(s, s->rbeg));
+            SWG_TRY(join(c, c->stream, s->side, s->ev[0]));
+        }
         s->lfirst_pl = s->lfirst_tp = 0;
-        if (!opened) SWG_TRY(lindrift_pl(s, dth, 1));
-        SWG_TRY(copy_positions(s, s->rbeg));
-        SWG_TRY(join(c, c->stream, s->side, s->ev[0]));
         SWG_TRY(on_stream(c, s->side, [&] {
-            SWG_TRY(tp_misc(s, CB_PTBEG, dth, first_mode));
+            if (!ahead) SWG_TRY(tp_misc(s, CB_PTBEG, dth, first_mode));
             SWG_TRY(kick_vb_tp(s, dth, 1));
+            SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[1], s->side), "event"));
             return drift_tp(s, dt);
         }));
         SWG_TRY(kick_vb_pl(s, dth, 1, false, opened));
         SWG_TRY(drift_pl(s, dt));
+        if (ahead) SWG_TRY(read());
         SWG_TRY(copy_positions(s, s->rend));
         SWG_TRY(join(c, c->stream, s->side, s->ev[2]));
         SWG_TRY(on_stream(c, s->side, [&] { return kick_vb_tp(s, dth, 0); }));
@@ -1168,14 +1193,16 @@ int symba_interp(swg_system *s, double dt, bool opened = false) {
     return SWG_OK;
 }
 
-// the close-approach scan over the two sets and its outcome, on the context's stream
-int discard_scan(swg_system *s, const SortedSet &pl, const SortedSet &tp) {
+// the close-approach scan over the two sets and its outcome, on the context's stream; open:
+// with the test particles' opening linear drift of the next step over dth
+int discard_scan(swg_system *s, const SortedSet &pl, const SortedSet &tp, bool open = false, double dth = 0.0) {
     swg_ctx *c = s->c;
     SWG_TRY(pltp_sorted_batched(c, true, pl, tp, s->tstatus, s->srt->nitems, s->srt->items, s->dt, 0, nullptr, nullptr,
                                 nullptr, nullptr, s->tflag, s->srt->pchunk));
     k_apply_discard<<<grid_for(s->ntp, 256), 256, 0, c->stream>>>(s->ntp, s->tflag, s->tstatus, s->tlmask, s->trh,
                                                                   s->tvh, s->tvb, s->npl, nullptr, nullptr, nullptr,
-                                                                  s->ndiscard);
+                                                                  s->ndiscard, open ? s->dcb + CB_PTBEG : nullptr,
+                                                                  dth);
     return L(c, "apply_discard");
 }
 // swiftest_discard_pl_tp (src/swiftest/swiftest_discard.f90:244-290), run after each step
@@ -1193,33 +1220,43 @@ int discard_step(swg_system *s) {
     return discard_scan(s, pl, tp);
 }
 
-// discard_step after a HELIO step left apart: the massive bodies' sorted set here, with a copy of
-// their state for the exact tests, the rest on the test particles' stream, beside the massive
-// bodies' next step (which no test particle concerns): 100 pl x 1000 tp, 92 -> 70 us a step with
-// the velocity updates in the kicks' launches.  Event 8: the scan has read the set and the copy.
-int discard_aside(swg_system *s) {
+// The end of a HELIO step left apart: the test particles' closing and discard_step on their
+// stream, beside the massive bodies' next step, which no test particle concerns; the scan reads
+// copies of the massive bodies' state, whose sorted set a third stream prepares.  In the FP64
+// path the closing kernels also take the next step's opening linear drifts.  100 pl x 1000 tp, FP64:
+// 92 -> 60 us a step, with the velocity updates in the kicks' launches.  Events: 7 the test
+// particles have read rend and the central-body record, 8 the scan has read the set and the copies.
+int discard_aside(swg_system *s, const Aside &aside) {
     swg_ctx *c = s->c;
-    const size_t n = s->npl;
-    SWG_TRY(ensure(c, s->snap, sizeof(double) * 6 * n));
-    SortedSet pl = sorted_pl(s, s->rh, s->vh, s->radius);
-    pl.rcopy = (double *)s->snap.ptr;
-    pl.vcopy = pl.rcopy + 3 * n;
-    if (s->behind) SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[8], 0), "event"));
-    SWG_TRY(sorted_set_prep(c, pl, 1, s->srt->npl_prep++ % 8 == 0, s->dt));
-    pl.r = pl.rcopy;
-    pl.v = pl.vcopy;
-    SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[4], c->stream), "event"));
+    const double dth = 0.5 * s->dt;
+    const bool ahead = exact(s) && aside.next;
+    if (!exact(s)) {  // (close_pl copies in the FP64 path)
+        if (s->behind) SWG_TRY(cuda_status(c, cudaStreamWaitEvent(c->stream, s->ev[8], 0), "event"));
+        SWG_TRY(cuda_status(c, cudaMemcpyAsync(s->rscan(), s->rh, 24 * (size_t)s->npl, cudaMemcpyDeviceToDevice, c->stream), "copy"));
+        SWG_TRY(cuda_status(c, cudaMemcpyAsync(s->vscan(), s->vh, 24 * (size_t)s->npl, cudaMemcpyDeviceToDevice, c->stream), "copy"));
+    }
+    const SortedSet pl = sorted_pl(s, s->rscan(), s->vscan(), s->radius), tp = sorted_tp(s, s->trh, s->tvh);
+    SWG_TRY(join(c, c->stream, s->side2, s->ev[4]));
+    SWG_TRY(on_stream(c, s->side2, [&] { return sorted_set_prep(c, pl, 1, s->srt->npl_prep++ % 8 == 0, s->dt); }));
+    SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[5], s->side2), "event"));
     s->behind = true;
+    s->ahead = ahead;
     return on_stream(c, s->side, [&] {
-        const SortedSet tp = sorted_tp(s, s->trh, s->tvh);
-        SWG_TRY(sorted_set_prep(c, tp, 1, s->srt->ntp_prep++ % 32 == 0, s->dt));
-        SWG_TRY(cuda_status(c, cudaStreamWaitEvent(s->side, s->ev[4], 0), "event"));
-        SWG_TRY(discard_scan(s, pl, tp));
+        if (s->srt->ntp_prep++ % 32 == 0) {  // a new order: from the closed state
+            SWG_TRY(tp_misc(s, CB_PTEND, dth, 3));
+            SWG_TRY(sorted_set_prep(c, tp, 1, true, s->dt));
+        } else {
+            SWG_TRY(sorted_tp_close(c, tp, TpClose{s->tlmask, s->tvb, s->dcb + CB_PTEND, dth}, s->trh, s->tvh, s->dt));
+        }
+        SWG_TRY(cuda_status(c, cudaEventRecord(s->ev[7], s->side), "event"));
+        SWG_TRY(cuda_status(c, cudaStreamWaitEvent(s->side, s->ev[5], 0), "event"));
+        SWG_TRY(discard_scan(s, pl, tp, ahead, dth));
         return cuda_status(c, cudaEventRecord(s->ev[8], s->side), "event");
     });
 }
 // what a step left on the side stream joins the context's stream
 int join_aside(swg_system *s) {
+    s->ahead = false;
     if (!s->behind) return SWG_OK;
     s->behind = false;
     return join(s->c, s->side, s->c->stream, s->ev[4]);
@@ -1476,11 +1513,15 @@ int swg_system_initialize(swg_system *s) {
 }
 
 static int steps(swg_system *s, int32_t nsteps) {
-    // HELIO: the test particles' discard scan runs beside the massive bodies' next step
-    const bool aside = s->integrator == SWG_HELIO && s->lclose && helio_fork(s);
-    if (aside) SWG_TRY(ensure_sorted(s));
+    Aside aside;  // HELIO
+    aside.on = s->integrator == SWG_HELIO && s->lclose && helio_fork(s);
+    if (aside.on) {
+        SWG_TRY(ensure_sorted(s));
+        SWG_TRY(ensure(s->c, s->snap, sizeof(double) * 6 * (size_t)s->npl));
+    }
     for (int32_t k = 0; k < nsteps; k++) {
         int rc;
+        aside.next = aside.on && k + 1 < nsteps;
         if (s->integrator == SWG_WHM)
             rc = whm_step(s, s->dt);
         else if (s->integrator == SWG_HELIO)
@@ -1488,7 +1529,7 @@ static int steps(swg_system *s, int32_t nsteps) {
         else
             rc = symba_step(s, s->dt);
         if (rc != SWG_OK) return rc;
-        SWG_TRY(aside ? discard_aside(s) : discard_step(s));
+        SWG_TRY(aside.on ? discard_aside(s, aside) : discard_step(s));
         if (s->h_flags[2] != 0) {  // recursion status of an earlier step, seen at a sync point
             s->c->err = "SyMBA local time step too small";
             return s->h_flags[2];
