@@ -37,7 +37,7 @@
 using namespace swg;
 using namespace swg::sdev;
 
-static_assert(KICK_FP64_TILE == 10 && ENC_TILE == 128, "tile sizes of the batched kernels");
+static_assert(KICK_FP64_TILE == 10 && KICK_FP64_TP_TILE == 9 && ENC_TILE == 128, "tile sizes of the batched kernels");
 
 // Arguments of the ensemble recursion kernel: the shared base plus per-system tables.
 struct EnsRecArgs {
@@ -590,7 +590,7 @@ int build_items(swg_ensemble *e) {
     auto ntp = [&](int s) { return e->h_ntp[s]; };
     auto plcost = [&](int s, int, int nr) { return (double)nr * e->h_npl[s]; };
     SWG_TRY(put_items(e, &e->it_fpl, &e->n_fpl, make_items(S, KICK_FP64_TILE, npl, plcost)));
-    SWG_TRY(put_items(e, &e->it_ftp, &e->n_ftp, make_items(S, KICK_FP64_TILE, ntp, plcost)));
+    SWG_TRY(put_items(e, &e->it_ftp, &e->n_ftp, make_items(S, KICK_FP64_TP_TILE, ntp, plcost)));
     auto tp_with_pl = [&](int s) { return e->h_npl[s] > 0 ? e->h_ntp[s] : 0; };
     SWG_TRY(put_items(e, &e->it_tsp, &e->n_tsp, make_items(S, ENC_SORTED_TILE, tp_with_pl, plcost)));
     {  // tp bound tiles of the sorted pl-tp checks

@@ -15,9 +15,9 @@
 // are issued as DFMA with a factor of one: the same rounding).  The square root, the
 // quotient and the products are formed outside that pipe (fp64_exact.cuh, the same bits), which
 // leaves five additions per pair and 3.2 for the fold: 8.2 instructions, 131 cycles, per 32
-// pairs and SM against ~40 before.  65,537 tp x 2047 pl: 10.3 -> 2.6 ms (16,384 pl: 22.6 -> 5.3 ms),
-// FP64 pipe 74%, ALU pipe 60%, issue slots 64% busy (ncu); four blocks of 40 registers per SM
-// (three of 56: 2.8 ms, two: 3.9 ms): the long chains of dependent instructions want warps.
+// pairs and SM against ~40 before.  65,537 tp x 2047 pl: 10.3 -> 2.5 ms (16,384 pl: 22.6 -> 5.3 ms),
+// FP64 pipe 77%, ALU pipe 60%, issue slots 68% busy (ncu): the long chains of dependent
+// instructions want warps (three blocks of 56 registers per SM: 2.8 ms, two: 3.9 ms).
 //
 #include <cuda_runtime.h>
 
@@ -26,11 +26,16 @@
 
 namespace swg {
 
-constexpr int FP64_RT = KICK_FP64_TILE;  // receivers per block of the batched forms
-constexpr int FP64_RTMAX = 10;           // most receivers per block (30 of the fold warp's 32 lanes)
+// Most receivers per block (which the batched forms use), and blocks per SM.  Ten receivers fill 30
+// of the fold warp's 32 lanes, with four blocks of 40 registers a thread.  The test particles' forms
+// spill little at 32 registers, where six blocks of nine fit: more chains of additions at a time
+// (2047 pl x 65,537 tp: 2.58 -> 2.53 ms; the pl-pl forms 5.28 -> 5.34 ms; blocks of eight 2.64 and
+// 5.51 ms, of seven 2.74 and 5.68 ms).
+constexpr int FP64_RT = KICK_FP64_TILE, FP64_BLOCKS = 4;
+constexpr int FP64_RT_TP = KICK_FP64_TP_TILE, FP64_BLOCKS_TP = 6;
 constexpr int PT = 32;                   // partners per round
 
-static_assert(3 * FP64_RTMAX <= 32, "one fold warp");
+static_assert(3 * FP64_RT <= 32 && 3 * FP64_RT_TP <= 32, "one fold warp");
 __host__ __device__ constexpr int fp64_threads(int rt) { return 32 * (rt + 1); }
 // doubles per partner of a stage (odd: conflict-free columns) and bytes of the ring
 __host__ __device__ constexpr int term_stride(int rt) { return (3 * rt) | 1; }
@@ -226,14 +231,14 @@ __device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int npl
 }
 
 template <bool RAD, int MODE>
-__global__ void __launch_bounds__(fp64_threads(FP64_RTMAX), 4)
+__global__ void __launch_bounds__(fp64_threads(FP64_RT), FP64_BLOCKS)
     k_kick_plpl_fp64(int RT, int npl, int nplm, const double *__restrict__ r, const double *__restrict__ Gm,
                      const double *__restrict__ R, double *__restrict__ acc, int acc_is_zero, KickVel kv) {
     extern __shared__ double sh[];
     fp64_group<RAD, MODE>(RT, npl, npl, nplm, r, r, Gm, R, nullptr, acc, acc_is_zero, blockIdx.x * RT, sh, kv);
 }
 
-__global__ void __launch_bounds__(fp64_threads(FP64_RTMAX), 4)
+__global__ void __launch_bounds__(fp64_threads(FP64_RT_TP), FP64_BLOCKS_TP)
     k_kick_tp_fp64(int RT, int ntp, int npl, const double *__restrict__ rtp, const double *__restrict__ rpl,
                    const double *__restrict__ Gm, const int32_t *__restrict__ lmask, double *__restrict__ acc,
                    int acc_is_zero, KickVel kv) {
@@ -249,7 +254,7 @@ __global__ void __launch_bounds__(fp64_threads(FP64_RTMAX), 4)
 // it every system is fully interacting (KICK_DIRECT).  With sys_flag, the pl-pl form kicks
 // only systems whose flag equals `phase`.
 template <bool RAD>
-__global__ void __launch_bounds__(fp64_threads(FP64_RT), 4)
+__global__ void __launch_bounds__(fp64_threads(FP64_RT), FP64_BLOCKS)
     k_kick_plpl_fp64_batched(const int4 *__restrict__ items, const int32_t *__restrict__ poff,
                              const int32_t *__restrict__ npl, const double *__restrict__ r,
                              const double *__restrict__ Gm, const double *__restrict__ R, double *__restrict__ acc,
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(fp64_threads(FP64_RT), 4)
         fp64_group<RAD, KICK_DIRECT>(FP64_RT, n, n, m, rs, rs, Gm + o, Rs, nullptr, as, acc_is_zero, w.y, sh);
 }
 
-__global__ void __launch_bounds__(fp64_threads(FP64_RT), 4)
+__global__ void __launch_bounds__(fp64_threads(FP64_RT_TP), FP64_BLOCKS_TP)
     k_kick_tp_fp64_batched(const int4 *__restrict__ items, const int32_t *__restrict__ toff,
                            const int32_t *__restrict__ ntp, const int32_t *__restrict__ poff,
                            const int32_t *__restrict__ npl, const double *__restrict__ rtp,
@@ -276,7 +281,7 @@ __global__ void __launch_bounds__(fp64_threads(FP64_RT), 4)
     extern __shared__ double sh[];
     const int4 w = items[blockIdx.x];
     const int ot = toff[w.x], op = poff[w.x];
-    fp64_group<false, KICK_TP>(FP64_RT, ntp[w.x], npl[w.x], 0, rtp + 3 * (size_t)ot, rpl + 3 * (size_t)op, Gm + op,
+    fp64_group<false, KICK_TP>(FP64_RT_TP, ntp[w.x], npl[w.x], 0, rtp + 3 * (size_t)ot, rpl + 3 * (size_t)op, Gm + op,
                                nullptr, lmask + ot, acc + 3 * (size_t)ot, acc_is_zero, w.y, sh);
 }
 
@@ -288,11 +293,11 @@ static inline int div_up_i(int64_t a, int64_t b) { return (int)((a + b - 1) / b)
 // work of its blocks (TERM_C cycles per receiver, FOLD_C per fold warp), at least the
 // fold's chain of 32 dependent additions (~2100 cycles); the fullest SM sets the time, and the
 // smallest blocks that reach it leave the least to wait for.
-static int fp64_rt(int num_sms, int n) {
+static int fp64_rt(int num_sms, int n, int most) {
     constexpr int TERM_C = 130, FOLD_C = 512, CHAIN_C = 2100;
     int best = 1;
     int64_t cost = INT64_MAX;
-    for (int rt = 1; rt <= FP64_RTMAX; rt++) {
+    for (int rt = 1; rt <= most; rt++) {
         const int64_t per_sm = div_up_i(div_up_i(n, rt), num_sms > 0 ? num_sms : 152);
         const int64_t c = per_sm * (rt * TERM_C + FOLD_C), t = c > CHAIN_C ? c : CHAIN_C;
         if (t < cost) {
@@ -306,7 +311,7 @@ static int fp64_rt(int num_sms, int n) {
 int kick_plpl_fp64(swg_ctx *c, int32_t npl, int32_t nplm, const double *r, const double *Gm, const double *R,
                    double *acc, int mode, int acc_is_zero, const KickVel &kv) {
     if (npl <= 0) return SWG_OK;
-    const int rt = fp64_rt(c->num_sms, npl), grid = div_up_i(npl, rt), th = fp64_threads(rt);
+    const int rt = fp64_rt(c->num_sms, npl, FP64_RT), grid = div_up_i(npl, rt), th = fp64_threads(rt);
     const cudaStream_t st = c->stream;
     if (mode == KICK_DIRECT) {
         if (R)
@@ -326,7 +331,7 @@ int kick_plpl_fp64(swg_ctx *c, int32_t npl, int32_t nplm, const double *r, const
 int kick_tp_fp64(swg_ctx *c, int32_t ntp, int32_t npl, const double *rtp, const double *rpl, const double *Gm,
                  const int32_t *lmask, double *acc, int acc_is_zero, const KickVel &kv) {
     if (ntp <= 0) return SWG_OK;
-    const int rt = fp64_rt(c->num_sms, ntp);
+    const int rt = fp64_rt(c->num_sms, ntp, FP64_RT_TP);
     k_kick_tp_fp64<<<div_up_i(ntp, rt), fp64_threads(rt), fp64_shared(rt), c->stream>>>(rt, ntp, npl, rtp, rpl, Gm, lmask, acc,
                                                                           acc_is_zero, kv);
     c->launches++;
@@ -352,7 +357,7 @@ int kick_tp_fp64_batched(swg_ctx *c, int nitems, const int4 *items, const int32_
                          const int32_t *poff, const int32_t *npl, const double *rtp, const double *rpl,
                          const double *Gm, const int32_t *lmask, double *acc, int acc_is_zero) {
     if (nitems <= 0) return SWG_OK;
-    k_kick_tp_fp64_batched<<<nitems, fp64_threads(FP64_RT), fp64_shared(FP64_RT), c->stream>>>(items, toff, ntp, poff, npl, rtp, rpl, Gm,
+    k_kick_tp_fp64_batched<<<nitems, fp64_threads(FP64_RT_TP), fp64_shared(FP64_RT_TP), c->stream>>>(items, toff, ntp, poff, npl, rtp, rpl, Gm,
                                                                             lmask, acc, acc_is_zero);
     c->launches++;
     return launch_status(c, "kick_tp_fp64_batched");

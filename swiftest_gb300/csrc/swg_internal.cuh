@@ -241,7 +241,7 @@ std::string tune_key(int device, const char *kind, int bucket);
 int tune_lookup(const std::string &key);
 void tune_store(const std::string &key, int variant);
 // receivers per item of the batched kernels
-constexpr int KICK_FP64_TILE = 10;
+constexpr int KICK_FP64_TILE = 10, KICK_FP64_TP_TILE = 9;
 constexpr int ENC_TILE = 128;
 constexpr int ENC_SORTED_TILE = 128;  // receivers per item of the radius-sorted pl-pl check
 constexpr int ENC_BOUND_TILE = 64;    // bodies per bound tile of the radius-sorted check
