@@ -5,6 +5,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fp64_exact.cuh"
 #include "swg_internal.cuh"
 
 namespace swg {
@@ -66,17 +67,19 @@ struct BodyF {
 
 __device__ __forceinline__ BodyF make_body(double x, double y, double z, double u, double v, double w, float renc) {
     BodyF o;
-    const float xh = __double2float_rn(x), yh = __double2float_rn(y), zh = __double2float_rn(z);
+    float xh, yh, zh, xl, yl, zl;
+    x_split(x, xh, xl);
+    x_split(y, yh, yl);
+    x_split(z, zh, zl);
     o.a = make_float4(xh, yh, zh, renc);
-    o.b = make_float4(__double2float_rn(x - (double)xh), __double2float_rn(y - (double)yh),
-                      __double2float_rn(z - (double)zh), sqrtf(xh * xh + yh * yh + zh * zh));
-    const float vx = __double2float_rn(u), vy = __double2float_rn(v), vz = __double2float_rn(w);
+    o.b = make_float4(xl, yl, zl, sqrtf(xh * xh + yh * yh + zh * zh));
+    const float vx = x_to_float_rn(u), vy = x_to_float_rn(v), vz = x_to_float_rn(w);
     o.v = make_float4(vx, vy, vz, sqrtf(vx * vx + vy * vy + vz * vz));
     return o;
 }
 __device__ __forceinline__ BodyF load_body(const double *r, const double *v, const double *renc, int i) {
     return make_body(r[3 * i], r[3 * i + 1], r[3 * i + 2], v[3 * i], v[3 * i + 1], v[3 * i + 2],
-                     renc ? __double2float_rn(renc[i]) : 0.f);
+                     renc ? x_to_float_rn(renc[i]) : 0.f);
 }
 
 // True when the pair certainly fails encounter_check_one.  The FP64 test accepts a

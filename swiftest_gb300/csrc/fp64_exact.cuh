@@ -182,6 +182,28 @@ __device__ __forceinline__ float x_to_float_rn(double x) {
     return __int_as_float((int)((f + up) | (hi & 0x80000000)));
 }
 
+// hi = (float)x, lo = (float)(x - hi), both rounded to nearest even: with x = +-(1.m) 2^e the
+// remainder is an integer of at most 29 bits times 2^(e - 52), so one integer conversion rounds it.
+static __device__ __noinline__ float2 x_native_split(double x) {
+    const float hi = (float)x;
+    return make_float2(hi, (float)(x - (double)hi));
+}
+__device__ __forceinline__ void x_split(double x, float &hi, float &lo) {
+    const int h = __double2hiint(x), l = __double2loint(x), m = h & 0x7fffffff;
+    const int e = (m >> 20) - 1023;
+    if ((unsigned)(e + 70) > 170u) {  // out of range (zeros too): lo may be subnormal, hi infinite
+        const float2 s = x_native_split(x);
+        hi = s.x;
+        lo = s.y;
+        return;
+    }
+    const unsigned f = __funnelshift_l(l, m - ((1023 - 127) << 20), 3);
+    const int rest = l & 0x1fffffff, up = (int)(((unsigned)rest + 0x0fffffffu + (f & 1u)) >> 29);
+    const int k = rest - (up << 29);
+    hi = __int_as_float((int)((f + up) | (h & 0x80000000)));
+    lo = (float)(h < 0 ? -k : k) * __int_as_float((e - 52 + 127) << 23);
+}
+
 __device__ __forceinline__ double x_half(double a) {
     const int h = __double2hiint(a);
     if (!x_ok(h & 0x7fffffff)) return 0.5 * a;

@@ -311,8 +311,8 @@ __global__ void k_kick_split(int n, const double *__restrict__ r, const double *
     split_hi_lo(r[3 * j + 0], a.x, b.x);
     split_hi_lo(r[3 * j + 1], a.y, b.y);
     split_hi_lo(r[3 * j + 2], a.z, b.z);
-    a.w = __double2float_rn(Gm[j]);
-    b.w = R ? __double2float_rn(R[j]) : 0.f;
+    a.w = x_to_float_rn(Gm[j]);
+    b.w = R ? x_to_float_rn(R[j]) : 0.f;
     A[j] = a;
     B[j] = b;
 }

@@ -8,6 +8,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fp64_exact.cuh"
+
 namespace swg {
 
 constexpr int MT = 64;        // partners per FP32 partial (mixed)
@@ -26,8 +28,7 @@ static __device__ __forceinline__ void ff_add(FF &a, float p) {
 }
 
 static __device__ __forceinline__ void split_hi_lo(double x, float &hi, float &lo) {
-    hi = __double2float_rn(x);
-    lo = __double2float_rn(x - (double)hi);
+    x_split(x, hi, lo);
 }
 
 // One receiving body of the mixed kick: its coordinates split into float hi/lo.
