@@ -950,7 +950,9 @@ void reset_kick_plans(swg_ensemble *e) {
 
 // pl-pl accelerations into ah (helio_kick_getacch_int_pl / symba_kick_getacch_int_pl) of all
 // systems, or (flag != nullptr) of the systems whose flag equals phase, on c->stream.
-int accel_int_pl(swg_ensemble *e, unsigned *head, const int32_t *flag = nullptr, int phase = 0, int acc_is_zero = 1) {
+// split_done (mixed path): recorded once the partners' float copies are there.
+int accel_int_pl(swg_ensemble *e, unsigned *head, const int32_t *flag = nullptr, int phase = 0, int acc_is_zero = 1,
+                 cudaEvent_t split_done = nullptr) {
     swg_ctx *c = e->c;
     const bool rad = e->integrator == SWG_SYMBA || e->lclose;
     const double *R = rad ? e->radius : nullptr;
@@ -958,6 +960,7 @@ int accel_int_pl(swg_ensemble *e, unsigned *head, const int32_t *flag = nullptr,
         float4 *pa = e->kend ? e->kA2 : e->kA, *pb = e->kend ? e->kB2 : e->kB;
         SWG_TRY(kick_split_launch(c, e->NPL, e->rh, e->Gmass, R, pa, pb, flag ? e->psys : nullptr, flag, phase));
         SWG_TRY(ensure_kick_plan(e, 0, rad, head, flag, phase));
+        if (split_done) SWG_TRY(cuda_status(c, cudaEventRecord(split_done, c->stream), "split"));
         if (e->kv[0] == KICK_SYMMETRIC) {  // never with semi-interacting bodies (ensure_kick_plan)
             SWG_TRY(kick_mixed_sym_batched(c, rad, e->n_sym, e->it_sym, e->poff, e->npl, e->sym_base, pa, pb,
                                            e->sym_part, e->sym_ppart, head, flag, phase, nullptr, 0, e->sym_warps,
@@ -984,12 +987,13 @@ int on_stream(swg_ctx *c, cudaStream_t st, F f) {
 // helio_kick_vb_pl (helio_kick.f90:91-132) with symba_kick_getacch_pl (symba_kick.f90:36-76).
 // have_acc: the accelerations are already in ah (see ens_step); update: apply vb += ah dt
 // here (close_pl applies the closing kick inside its sums instead).
-int kick_vb_pl(swg_ensemble *e, double dt, int lbeg, bool have_acc = false, bool update = true) {
+int kick_vb_pl(swg_ensemble *e, double dt, int lbeg, bool have_acc = false, bool update = true,
+               cudaEvent_t split_done = nullptr) {
     swg_ctx *c = e->c;
     if (e->NPL == 0) return SWG_OK;
     if (!have_acc) {
         ProfScope ps(e->prof, c->stream, PROF_KICK_PL);
-        SWG_TRY(accel_int_pl(e, e->head));
+        SWG_TRY(accel_int_pl(e, e->head, nullptr, 0, 1, split_done));
     }
     if (e->integrator == SWG_SYMBA && e->pp_n > 0) {
         SWG_TRY(ensure(c, e->pair_terms, (size_t)e->pp_n * (6 * sizeof(double) + 1)));
@@ -1662,11 +1666,13 @@ int helio_step_groups(swg_ensemble *e, double dt) {
     const double dth = 0.5 * dt;
     const int64_t T = e->tsplit, M = e->NTP;
     unsigned *h0 = e->head + 1, *h1 = e->head + 2;
-    SWG_TRY(kick_vb_pl(e, dth, 1));
-    // the pl-tp kick's tile shape is timed here, on this stream, before the side streams run
-    // beside it (as in the sequential step, which tunes at the same point)
+    // The test particles need the split positions alone, so their kick starts beside the pl-pl
+    // one and fills its tail and its sums (512 systems of 10-2000 pl: 0.5% of the step); not while a
+    // tile shape is still to be timed, which happens on this stream with nothing beside it
+    const bool beside = e->kv[0] >= 0 && e->kv[1] >= 0;
+    SWG_TRY(kick_vb_pl(e, dth, 1, false, true, beside ? e->ev_fork : nullptr));
     SWG_TRY(ensure_kick_plan(e, 1, false, e->head, nullptr, 0));
-    SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_fork, c->stream), "fork"));
+    if (!beside) SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_fork, c->stream), "fork"));
     SWG_TRY(cuda_status(c, cudaStreamWaitEvent(e->side, e->ev_fork, 0), "fork"));
     SWG_TRY(on_stream(c, e->side, [&] {
         SWG_TRY(tp_misc_range(e, 0, T, CB_PTBEG, dth, 2, 4));
