@@ -8,8 +8,9 @@
 // recursion, on the "any deeper encounter" flag of each sub-step.
 //
 // O(N) serial sums of the reference (the Sun's barycentric momentum in
-// helio_drift_linear_pl, vh2vb / vb2vh, WHM Jacobi prefix sums) run in one
-// thread in the reference's index order when the kick precision is FP64, so the
+// helio_drift_linear_pl, vh2vb / vb2vh, WHM Jacobi prefix sums) are added one term
+// after the other in the reference's index order when the kick precision is FP64, one
+// warp with a lane per component, so the
 // FP64 path reproduces the serial reference loop bit for bit; in the mixed path
 // they use a fixed-order block reduction.
 #include <cuda_runtime.h>
