@@ -356,16 +356,18 @@ __device__ __forceinline__ double d_norm2e(double a, double b, double c) {
         if (v[k] != 0.0) {
             const double absx = fabs(v[k]);
             if (scale < absx) {
-                const double q = scale / absx;
-                ssq = 1.0 + ssq * q * q;
+                if (scale != 0.0) {  // else q = 0: ssq stays 1
+                    const double q = xdiv(scale, absx);
+                    ssq = 1.0 + ssq * q * q;
+                }
                 scale = absx;
             } else {
-                const double q = absx / scale;
+                const double q = xdiv(absx, scale);
                 ssq = ssq + q * q;
             }
         }
     }
-    return scale * sqrt(ssq);
+    return scale * xsqrt(ssq);
 }
 
 // extents: body b (0..ntot-1) -> keys[b] = rmin, keys[ntot+b] = rmax, vals = extent index
@@ -450,6 +452,102 @@ __global__ void k_sas_sweep(int n1, const double *r1, const double *v1, const do
     }
 }
 
+// The sorted order of one system's extents, up to SAS_MERGED of them: each block forms and sorts a
+// tile of SAS_TILE in shared memory, then rounds of merges join up to SAS_WAYS runs each; an
+// extent's place is its place in its run plus, run by run, the count of extents before it there
+// (a binary search).  Ties keep the extents' order, as in the radix sort: equal keys count from the
+// runs before the own one only.  Bound by launches and dependent loads: two to five launches here,
+// up to 24 and a host read in the radix sort.  A whole pl-tp check, radix sort and this: 314 x 2501
+// bodies 168 -> 62 us, 2370 x 3650 220 -> 119, 8192 x 50,000 292 -> 198, 4000 x 200,000 462 -> 407,
+// 20,000 x 500,000 1012 and 1033, hence the line.  Merges of 16 runs: 50, 122, 191, 458 us; tiles of
+// 2048 took 60 us themselves.
+constexpr int SAS_TILE = 512, SAS_T = SAS_TILE / 2, SAS_WAYS = 8;
+constexpr int64_t SAS_MERGED = 524288;
+__global__ void __launch_bounds__(SAS_T) k_sas_tiles(int n1, const double *r1, const double *v1, const double *renc1,
+                                                     int n2, const double *r2, const double *v2, const double *renc2,
+                                                     uint64_t *keys, uint32_t *ids, float4 *FA, float4 *FB,
+                                                     float4 *FV) {
+    __shared__ uint64_t sk[SAS_TILE];
+    __shared__ uint16_t si[SAS_TILE];
+    const int ntot = n1 + n2, ne = 2 * ntot, base = blockIdx.x * SAS_TILE;
+    for (int l = threadIdx.x; l < SAS_TILE; l += SAS_T) {
+        const int e = base + l;
+        uint64_t k = ~0ull;  // beyond the last extent (after it also where its key is the same)
+        if (e < ne) {
+            const int b = e < ntot ? e : e - ntot;
+            const bool il1 = b < n1;
+            const double *r = il1 ? &r1[3 * b] : &r2[3 * (b - n1)];
+            const double rc = il1 ? renc1[b] : (renc2 ? renc2[b - n1] : 0.0);
+            const double rmag = d_norm2e(r[0], r[1], r[2]);
+            k = d2key(e < ntot ? rmag - RSWEEP_FACTOR * rc : rmag + RSWEEP_FACTOR * rc);
+            if (e < ntot) {
+                const BodyF o = il1 ? load_body(r1, v1, renc1, b) : load_body(r2, v2, renc2, b - n1);
+                FA[b] = o.a;
+                FB[b] = o.b;
+                FV[b] = o.v;
+            }
+        }
+        sk[l] = k;
+        si[l] = (uint16_t)l;
+    }
+    for (int k = 2; k <= SAS_TILE; k <<= 1)  // bitonic network on (key, place)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            const int i = 2 * (int)threadIdx.x - ((int)threadIdx.x & (j - 1)), q = i + j;
+            const uint64_t a = sk[i], b = sk[q];
+            const uint16_t x = si[i], y = si[q];
+            if ((a > b || (a == b && x > y)) == ((i & k) == 0)) {
+                sk[i] = b;
+                sk[q] = a;
+                si[i] = y;
+                si[q] = x;
+            }
+        }
+    __syncthreads();
+    for (int l = threadIdx.x; l < SAS_TILE && base + l < ne; l += SAS_T) {
+        keys[base + l] = sk[l];
+        ids[base + l] = (uint32_t)(base + si[l]);
+    }
+}
+// Runs of `run` extents in (keys, ids) to runs of SAS_WAYS run in (okeys, oids), or, in the last
+// round (okeys null), to the sorted order: oids and the positions of each body's two extents.
+__global__ void __launch_bounds__(256) k_sas_merge(int ntot, int run, const uint64_t *__restrict__ keys,
+                                                   const uint32_t *__restrict__ ids, uint64_t *okeys, uint32_t *oids,
+                                                   int32_t *ibeg, int32_t *iend) {
+    const int ne = 2 * ntot, q = blockIdx.x * 256 + threadIdx.x;
+    if (q >= ne) return;
+    const uint64_t key = keys[q];
+    const int own = q / run, r0 = own / SAS_WAYS * SAS_WAYS;
+    int place = r0 * run + (q - own * run);
+    int lo[SAS_WAYS - 1], beg[SAS_WAYS - 1], end[SAS_WAYS - 1];
+    // the searches go in step: each step waits for its loads
+#pragma unroll
+    for (int w = 0; w < SAS_WAYS - 1; w++) {
+        const int r = r0 + w + (r0 + w >= own);  // the group's runs but the own one
+        beg[w] = lo[w] = min(r * run, ne);
+        end[w] = min((r + 1) * run, ne);
+    }
+#pragma unroll 1
+    for (int step = run; step > 0; step >>= 1)
+#pragma unroll
+        for (int w = 0; w < SAS_WAYS - 1; w++)
+            // all before lo count; the next `step` do if the last of them does
+            if (lo[w] + step <= end[w]) {
+                const uint64_t k = keys[lo[w] + step - 1];
+                if (k < key || (k == key && r0 + w < own)) lo[w] += step;
+            }
+#pragma unroll
+    for (int w = 0; w < SAS_WAYS - 1; w++) place += lo[w] - beg[w];
+    const uint32_t e = ids[q];
+    oids[place] = e;
+    if (okeys)
+        okeys[place] = key;
+    else if (e < (uint32_t)ntot)
+        ibeg[e] = place + 1;
+    else
+        iend[e - ntot] = place + 1;
+}
+
 // keys | vals | ibeg | iend | radix-sort scratch, each 256-byte aligned
 static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 size_t sas_scratch_bytes(int ntot) {
@@ -478,20 +576,41 @@ int sas_launch(swg_ctx *c, int n1, const double *r1, const double *v1, const dou
     int32_t *iend = ibeg + ntot;
     float4 *FA = (float4 *)(p += align256((size_t)ntot * 8)), *FB = FA + ntot, *FV = FB + ntot;
     void *rs = p + align256((size_t)ntot * 3 * sizeof(float4));
-    k_sas_extents<<<(ntot + 127) / 128, 128, 0, c->stream>>>(nb1, r1, renc1, nb2, r2, renc2, keys, vals);
-    c->launches++;
-    if (nb1 > 0) {
+    const bool merged = !seg_of && ne <= SAS_MERGED;
+    if (merged) {
+        uint64_t *bkeys = (uint64_t *)rs;  // the radix sort's scratch holds 16 bytes an extent
+        uint32_t *bids = (uint32_t *)(bkeys + ne), *ids = bids + ne;
+        const int tiles = (int)((ne + SAS_TILE - 1) / SAS_TILE), grid = (int)((ne + 255) / 256);
+        k_sas_tiles<<<tiles, SAS_T, 0, c->stream>>>(nb1, r1, v1, renc1, nb2, r2, v2, renc2, keys, ids, FA, FB, FV);
+        int64_t run = SAS_TILE;
+        uint64_t *from = keys, *to = bkeys;
+        uint32_t *idf = ids, *idt = bids;
+        for (; run * SAS_WAYS < ne; run *= SAS_WAYS) {
+            k_sas_merge<<<grid, 256, 0, c->stream>>>(ntot, (int)run, from, idf, to, idt, nullptr, nullptr);
+            std::swap(from, to);
+            std::swap(idf, idt);
+            c->launches++;
+        }
+        k_sas_merge<<<grid, 256, 0, c->stream>>>(ntot, (int)run, from, idf, nullptr, vals, ibeg, iend);
+        c->launches += 2;
+    } else {
+        k_sas_extents<<<(ntot + 127) / 128, 128, 0, c->stream>>>(nb1, r1, renc1, nb2, r2, renc2, keys, vals);
+        c->launches++;
+    }
+    if (!merged && nb1 > 0) {
         k_encounter_prep<<<(nb1 + 255) / 256, 256, 0, c->stream>>>(nb1, r1, v1, renc1, FA, FB, FV);
         c->launches++;
     }
-    if (nb2 > 0) {
+    if (!merged && nb2 > 0) {
         k_encounter_prep<<<(nb2 + 255) / 256, 256, 0, c->stream>>>(nb2, r2, v2, renc2, FA + nb1, FB + nb1, FV + nb1);
         c->launches++;
     }
-    // stable radix sort by extent; the extents enter in index order, so ties keep it
-    SWG_TRY(radix_sort_kv(c, ne, keys, vals, rs, seg_of, seg_bits, host_skip));
-    k_sas_positions<<<(int)((ne + 255) / 256), 256, 0, c->stream>>>(ntot, vals, ibeg, iend);
-    c->launches++;
+    if (!merged) {
+        // stable radix sort by extent; the extents enter in index order, so ties keep it
+        SWG_TRY(radix_sort_kv(c, ne, keys, vals, rs, seg_of, seg_bits, host_skip));
+        k_sas_positions<<<(int)((ne + 255) / 256), 256, 0, c->stream>>>(ntot, vals, ibeg, iend);
+        c->launches++;
+    }
     k_sas_sweep<<<(unsigned)((32 * (int64_t)ntot + 127) / 128), 128, 0, c->stream>>>(
         nb1, r1, v1, renc1, nb2, r2, v2, renc2, single, shift2, dt, vals, ibeg, iend, FA, FB, FV, cap, o1, o2, olv,
         count);

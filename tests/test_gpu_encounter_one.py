@@ -1,10 +1,12 @@
-"""TRIANGULAR checks of one pair of lists on both sides of the line from which they go over
+"""SORTSWEEP checks at the edges of the merge sort's tiles and rounds and of its range, and
+TRIANGULAR checks of one pair of lists on both sides of the line from which they go over
 radius-sorted tiles (encounter.cu SORTED_PAIRS): the oracle's lists, with segments, sub-tiles
 and receiver tiles left partly filled, and with bodies whose bounds are not finite."""
 import numpy as np
 import pytest
 
 from oracle import oracle as O
+from swiftest_gb300 import SWG_ENC_SORTSWEEP
 from swiftest_gb300 import initial_conditions as IC
 
 pytestmark = pytest.mark.gpu
@@ -52,5 +54,34 @@ def test_pltp(ctx, npl, ntp, odd):
     g = ctx.encounter_check_all_pltp(r, v, tr, tv, renc, 0.005, cap=200000)
     o = O.encounter_pltp(r, v, tr, tv, renc, 0.005)
     assert len(o[0]) > 0
+    for a, b in zip(g, o):
+        assert np.array_equal(a, b)
+
+
+# extents (two per body): one tile of 512 and its edge, one, two, three and four merge rounds, past
+# the range (the radix sort)
+@pytest.mark.parametrize("npl,ntp", [(1, 1), (7, 248), (7, 249), (7, 250), (50, 1998), (50, 1999), (33, 16351),
+                                     (33, 16352), (31, 131041), (31, 131042), (20, 262124), (20, 262125)])
+def test_pltp_sortsweep(ctx, npl, ntp):
+    r, v, renc, tr, tv = _disk(npl + ntp, npl, ntp)
+    tr[::1 + ntp // 200] = tr[0]  # equal extents in many tiles
+    if npl > 6:
+        r[3] = r[5]
+        tr[1::2 + ntp // 100] = r[5] * (1 + 1e-4)
+    g = ctx.encounter_check_all_pltp(r, v, tr, tv, renc, 0.005, mode=SWG_ENC_SORTSWEEP, cap=200000)
+    o = O.encounter_pltp(r, v, tr, tv, renc, 0.005, mode=SWG_ENC_SORTSWEEP)
+    assert npl == 1 or len(o[0]) > 0
+    for a, b in zip(g, o):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [2, 255, 256, 257, 2049, 16385])
+def test_plpl_sortsweep(ctx, n):
+    r, v, renc, _, _ = _disk(n, n, 0)
+    few = slice(0, n, 1 + n // 50)
+    r[few], renc[few] = r[0], renc[0]  # coincident bodies
+    r[1 : n : 1 + n // 20] *= 0.0  # extents around zero
+    g = ctx.encounter_check_all_plpl(r, v, 0.1 * renc, 0.005, mode=SWG_ENC_SORTSWEEP, cap=10000)
+    o = O.encounter_plpl(r, v, 0.1 * renc, 0.005, mode=SWG_ENC_SORTSWEEP)
     for a, b in zip(g, o):
         assert np.array_equal(a, b)
