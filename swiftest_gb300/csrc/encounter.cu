@@ -157,184 +157,155 @@ __global__ void __launch_bounds__(ET) k_encounter_tri_batched(
 }
 
 // ------------------------------------------------------------------ sorting
-// Generic (key, val) sort, ascending by (key, val).  Padding uses all-ones.
-constexpr int SORT_SMEM_N = 4096;  // elements sorted in one CTA (48 KB)
-
-__device__ __forceinline__ bool kv_greater(uint64_t ka, uint32_t va, uint64_t kb, uint32_t vb) {
-    return ka > kb || (ka == kb && va > vb);
-}
-
-__global__ void k_bitonic_shared(uint64_t *keys, uint32_t *vals, int64_t n_pad, int kmax_global) {
-    // Sorts each SORT_SMEM_N segment completely (kmax_global == 0) or finishes the
-    // merge stages j < SORT_SMEM_N of a global stage k (kmax_global == k).
-    __shared__ uint64_t sk[SORT_SMEM_N];
-    __shared__ uint32_t sv[SORT_SMEM_N];
-    const int64_t base = (int64_t)blockIdx.x * SORT_SMEM_N;
-    const int len = (int)((n_pad - base) < (int64_t)SORT_SMEM_N ? (n_pad - base) : (int64_t)SORT_SMEM_N);
-    for (int t = threadIdx.x; t < len; t += blockDim.x) {
-        sk[t] = keys[base + t];
-        sv[t] = vals[base + t];
-    }
-    __syncthreads();
-    if (kmax_global == 0) {
-        for (int k = 2; k <= len; k <<= 1) {
-            for (int jj = k >> 1; jj > 0; jj >>= 1) {
-                for (int t = threadIdx.x; t < len; t += blockDim.x) {
-                    const int p = t ^ jj;
-                    if (p > t) {
-                        const int64_t gt = base + t;
-                        const bool up = ((gt & k) == 0);
-                        const bool sw = up ? kv_greater(sk[t], sv[t], sk[p], sv[p]) : kv_greater(sk[p], sv[p], sk[t], sv[t]);
-                        if (sw) {
-                            uint64_t tk = sk[t];
-                            sk[t] = sk[p];
-                            sk[p] = tk;
-                            uint32_t tv = sv[t];
-                            sv[t] = sv[p];
-                            sv[p] = tv;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-    } else {
-        const int64_t k = kmax_global;
-        for (int jj = SORT_SMEM_N >> 1; jj > 0; jj >>= 1) {
-            for (int t = threadIdx.x; t < len; t += blockDim.x) {
-                const int p = t ^ jj;
-                if (p > t) {
-                    const int64_t gt = base + t;
-                    const bool up = ((gt & k) == 0);
-                    const bool sw = up ? kv_greater(sk[t], sv[t], sk[p], sv[p]) : kv_greater(sk[p], sv[p], sk[t], sv[t]);
-                    if (sw) {
-                        uint64_t tk = sk[t];
-                        sk[t] = sk[p];
-                        sk[p] = tk;
-                        uint32_t tv = sv[t];
-                        sv[t] = sv[p];
-                        sv[p] = tv;
-                    }
-                }
-            }
+// Ascending bitonic network over the N keys (a power of two) at sk, N / 2 threads of the block (all
+// of it calls); places (optional) move along, and order equal keys.
+template <bool PLACES>
+__device__ __forceinline__ void blk_bitonic(int N, uint64_t *sk, uint16_t *si) {
+    for (int k = 2; k <= N; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
             __syncthreads();
+            const int t = threadIdx.x, i = 2 * t - (t & (j - 1)), q = i + j;
+            if (t >= N / 2) continue;
+            const uint64_t a = sk[i], b = sk[q];
+            const bool more = a > b || (PLACES && a == b && si[i] > si[q]);
+            if (more == ((i & k) == 0)) {
+                sk[i] = b;
+                sk[q] = a;
+                if (PLACES) {
+                    const uint16_t x = si[i];
+                    si[i] = si[q];
+                    si[q] = x;
+                }
+            }
         }
-    }
-    for (int t = threadIdx.x; t < len; t += blockDim.x) {
-        keys[base + t] = sk[t];
-        vals[base + t] = sv[t];
-    }
-}
-
-__global__ void k_bitonic_global(uint64_t *keys, uint32_t *vals, int64_t n_pad, int64_t k, int64_t jj) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= n_pad) return;
-    const int64_t p = t ^ jj;
-    if (p <= t) return;
-    const bool up = ((t & k) == 0);
-    const uint64_t kt = keys[t], kp = keys[p];
-    const uint32_t vt = vals[t], vp = vals[p];
-    const bool sw = up ? kv_greater(kt, vt, kp, vp) : kv_greater(kp, vp, kt, vt);
-    if (sw) {
-        keys[t] = kp;
-        keys[p] = kt;
-        vals[t] = vp;
-        vals[p] = vt;
-    }
-}
-
-__global__ void k_fill_pad(uint64_t *keys, uint32_t *vals, int64_t n, int64_t n_pad) {
-    const int64_t t = n + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < n_pad) {
-        keys[t] = ~0ull;
-        vals[t] = ~0u;
-    }
-}
-
-int64_t sort_padded_len(int64_t n) {
-    int64_t p = 1;
-    while (p < n) p <<= 1;
-    return p < 2 ? 2 : p;
-}
-
-// keys/vals must have room for sort_padded_len(n) elements.
-int sort_kv(swg_ctx *c, int64_t n, uint64_t *keys, uint32_t *vals) {
-    if (n <= 1) return SWG_OK;
-    const int64_t n_pad = sort_padded_len(n);
-    if (n_pad > n) {
-        k_fill_pad<<<(int)((n_pad - n + 255) / 256), 256, 0, c->stream>>>(keys, vals, n, n_pad);
-        c->launches++;
-    }
-    const int64_t nseg = (n_pad + SORT_SMEM_N - 1) / SORT_SMEM_N;
-    k_bitonic_shared<<<(int)nseg, 512, 0, c->stream>>>(keys, vals, n_pad, 0);
-    c->launches++;
-    for (int64_t k = 2 * (int64_t)SORT_SMEM_N; k <= n_pad; k <<= 1) {
-        for (int64_t jj = k >> 1; jj >= SORT_SMEM_N; jj >>= 1) {
-            k_bitonic_global<<<(int)((n_pad + 255) / 256), 256, 0, c->stream>>>(keys, vals, n_pad, k, jj);
-            c->launches++;
-        }
-        k_bitonic_shared<<<(int)nseg, 512, 0, c->stream>>>(keys, vals, n_pad, (int)k);
-        c->launches++;
-    }
-    return launch_status(c, "sort_kv");
-}
-
-// pack (i1,i2,lv) into key=(i1<<32|i2), val=lv ; and back
-__global__ void k_pack_pairs(int64_t n, const int32_t *i1, const int32_t *i2, const int32_t *lv, uint64_t *keys,
-                             uint32_t *vals) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    keys[t] = ((uint64_t)(uint32_t)i1[t] << 32) | (uint64_t)(uint32_t)i2[t];
-    vals[t] = (uint32_t)lv[t];
-}
-// unpack, dropping repeated (i1,i2) keys (they carry the same lvdotr); the
-// surviving count goes to *nout.  Single pass with a block-wide prefix via atomics
-// is not order-preserving, so compaction uses a flag + scan in one block.
-__global__ void k_unpack_unique(int64_t n, const uint64_t *keys, const uint32_t *vals, int32_t *i1, int32_t *i2,
-                                int32_t *lv, unsigned long long *nout) {
-    // one block; sequential chunks with block scan
-    __shared__ int64_t s_base;
-    __shared__ int s_scan[1024];
-    if (threadIdx.x == 0) s_base = 0;
     __syncthreads();
-    for (int64_t c0 = 0; c0 < n; c0 += blockDim.x) {
+}
+// The place of key q when each group of MERGE_WAYS sorted runs of `run` keys (a power of two) is merged:
+// its place in its run plus, run by run, the count of keys before it there.  Equal keys keep their
+// order: they count from the runs before the own one only.
+constexpr int MERGE_WAYS = 8, MERGE_TILE = 512;
+template <class I>  // I: holds n + MERGE_WAYS run
+__device__ __forceinline__ I merge_place(I q, I n, I run, const uint64_t *__restrict__ keys) {
+    const uint64_t key = keys[q];
+    const I own = q / run, r0 = own / MERGE_WAYS * MERGE_WAYS;
+    I place = r0 * run + (q - own * run);
+    I lo[MERGE_WAYS - 1], beg[MERGE_WAYS - 1], end[MERGE_WAYS - 1];
+    // the searches go in step: each step waits for its loads
+#pragma unroll
+    for (int w = 0; w < MERGE_WAYS - 1; w++) {
+        const I r = r0 + w + (r0 + w >= own);  // the group's runs but the own one
+        beg[w] = lo[w] = min(r * run, n);
+        end[w] = min((r + 1) * run, n);
+    }
+#pragma unroll 1
+    for (I step = run; step > 0; step >>= 1)
+#pragma unroll
+        for (int w = 0; w < MERGE_WAYS - 1; w++)
+            // all before lo count; the next `step` do if the last of them does
+            if (lo[w] + step <= end[w]) {
+                const uint64_t k = keys[lo[w] + step - 1];
+                if (k < key || (k == key && r0 + w < own)) lo[w] += step;
+            }
+#pragma unroll
+    for (int w = 0; w < MERGE_WAYS - 1; w++) place += lo[w] - beg[w];
+    return place;
+}
+
+// Pairs (i1, i2, lv) sorted by (i1, i2), repeats dropped (they carry the same lv, 0 or 1).  One key
+// holds all three.  Up to PAIRS_BLOCK pairs in one block and launch; more in tiles and merges.
+// One key-value network of four launches before: a check of 4096 pl x 40,001 tp 99.7 -> 85.8 us, a
+// sort-and-sweep check of 20,000 x 500,000 (20,000 pairs) 969 -> 766 us.
+constexpr int PAIRS_BLOCK = 2048;
+__device__ __forceinline__ uint64_t pair_key(int i1, int i2, int lv) {
+    return ((uint64_t)(uint32_t)i1 << 32) | ((uint64_t)(uint32_t)i2 << 1) | (uint64_t)(lv != 0);
+}
+__device__ __forceinline__ void write_pair(uint64_t k, int64_t o, int32_t *i1, int32_t *i2, int32_t *lv) {
+    i1[o] = (int32_t)(k >> 32);
+    i2[o] = (int32_t)((uint32_t)k >> 1);
+    lv[o] = (int32_t)(k & 1);
+}
+// keep(t) of the block's elements t in [0, n) to the places after each other, whole block of 1024
+template <class K, class W>
+__device__ __forceinline__ int64_t blk_compact(int64_t n, K keep, W write) {
+    __shared__ int cnt[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int64_t base = 0;
+    for (int64_t c0 = 0; c0 < n; c0 += 1024) {
         const int64_t t = c0 + threadIdx.x;
-        int keep = 0;
-        if (t < n) keep = (t == 0) || (keys[t] != keys[t - 1]);
-        s_scan[threadIdx.x] = keep;
+        const bool on = t < n && keep(t);
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) cnt[w] = __popc(m);
         __syncthreads();
-        for (int off = 1; off < (int)blockDim.x; off <<= 1) {
-            int add = (threadIdx.x >= (unsigned)off) ? s_scan[threadIdx.x - off] : 0;
-            __syncthreads();
-            s_scan[threadIdx.x] += add;
-            __syncthreads();
+        int c = cnt[lane];
+        for (int off = 1; off < 32; off <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, c, off);
+            if (lane >= off) c += x;
         }
-        if (keep) {
-            const int64_t o = s_base + s_scan[threadIdx.x] - 1;
-            i1[o] = (int32_t)(keys[t] >> 32);
-            i2[o] = (int32_t)(keys[t] & 0xffffffffull);
-            lv[o] = (int32_t)vals[t];
-        }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) s_base += s_scan[threadIdx.x];
+        const int before = w ? __shfl_sync(0xffffffffu, c, (w + 31) & 31) : 0, total = __shfl_sync(0xffffffffu, c, 31);
+        if (on) write(t, base + before + __popc(m & ((1u << lane) - 1)));
+        base += total;
         __syncthreads();
     }
-    if (threadIdx.x == 0) *nout = (unsigned long long)s_base;
+    return base;
+}
+__global__ void __launch_bounds__(1024) k_pairs_block(int n, int N, int32_t *i1, int32_t *i2, int32_t *lv,
+                                                      unsigned long long *nout) {
+    __shared__ uint64_t sk[PAIRS_BLOCK];
+    for (int t = threadIdx.x; t < N; t += 1024) sk[t] = t < n ? pair_key(i1[t], i2[t], lv[t]) : ~0ull;
+    blk_bitonic<false>(N, sk, nullptr);
+    const int64_t m = blk_compact(
+        n, [&](int64_t t) { return t == 0 || (sk[t] >> 1) != (sk[t - 1] >> 1); },
+        [&](int64_t t, int64_t o) { write_pair(sk[t], o, i1, i2, lv); });
+    if (threadIdx.x == 0) *nout = (unsigned long long)m;
+}
+__global__ void __launch_bounds__(MERGE_TILE / 2) k_pairs_tiles(int64_t n, const int32_t *i1, const int32_t *i2,
+                                                                const int32_t *lv, uint64_t *keys) {
+    __shared__ uint64_t sk[MERGE_TILE];
+    const int64_t base = blockIdx.x * (int64_t)MERGE_TILE;
+    for (int l = threadIdx.x; l < MERGE_TILE; l += MERGE_TILE / 2)
+        sk[l] = base + l < n ? pair_key(i1[base + l], i2[base + l], lv[base + l]) : ~0ull;
+    blk_bitonic<false>(MERGE_TILE, sk, nullptr);
+    for (int l = threadIdx.x; l < MERGE_TILE && base + l < n; l += MERGE_TILE / 2) keys[base + l] = sk[l];
+}
+template <class I>
+__global__ void __launch_bounds__(256) k_pairs_merge(I n, I run, const uint64_t *__restrict__ keys, uint64_t *okeys) {
+    const I q = blockIdx.x * (I)256 + threadIdx.x;
+    if (q < n) okeys[merge_place(q, n, run, keys)] = keys[q];
+}
+__global__ void __launch_bounds__(1024) k_pairs_unique(int64_t n, const uint64_t *__restrict__ keys, int32_t *i1,
+                                                       int32_t *i2, int32_t *lv, unsigned long long *nout) {
+    const int64_t m = blk_compact(
+        n, [&](int64_t t) { return t == 0 || (keys[t] >> 1) != (keys[t - 1] >> 1); },
+        [&](int64_t t, int64_t o) { write_pair(keys[t], o, i1, i2, lv); });
+    if (threadIdx.x == 0) *nout = (unsigned long long)m;
 }
 
-// scratch: 12 bytes per padded element
-size_t sort_pairs_scratch_bytes(int64_t n) { return (size_t)sort_padded_len(n) * 12 + 256; }
+// scratch: two buffers of keys
+size_t sort_pairs_scratch_bytes(int64_t n) { return (size_t)n * 16 + 256; }
 
 int sort_pairs_unique(swg_ctx *c, int64_t n, int32_t *i1, int32_t *i2, int32_t *lv, void *scratch,
                       unsigned long long *d_nout) {
     if (n <= 0) return SWG_OK;
-    const int64_t n_pad = sort_padded_len(n);
-    uint64_t *keys = (uint64_t *)scratch;
-    uint32_t *vals = (uint32_t *)(keys + n_pad);
-    k_pack_pairs<<<(int)((n + 255) / 256), 256, 0, c->stream>>>(n, i1, i2, lv, keys, vals);
+    if (n <= PAIRS_BLOCK) {
+        int N = 2;
+        while (N < n) N <<= 1;
+        k_pairs_block<<<1, 1024, 0, c->stream>>>((int)n, N, i1, i2, lv, d_nout);
+        c->launches++;
+        return launch_status(c, "sort_pairs_unique");
+    }
+    uint64_t *from = (uint64_t *)scratch, *to = from + n;
+    k_pairs_tiles<<<(int)((n + MERGE_TILE - 1) / MERGE_TILE), MERGE_TILE / 2, 0, c->stream>>>(n, i1, i2, lv, from);
     c->launches++;
-    SWG_TRY(sort_kv(c, n, keys, vals));
-    k_unpack_unique<<<1, 1024, 0, c->stream>>>(n, keys, vals, i1, i2, lv, d_nout);
+    for (int64_t run = MERGE_TILE; run < n; run *= MERGE_WAYS) {
+        const int grid = (int)((n + 255) / 256);
+        if (n <= 1 << 27)
+            k_pairs_merge<int><<<grid, 256, 0, c->stream>>>((int)n, (int)run, from, to);
+        else
+            k_pairs_merge<int64_t><<<grid, 256, 0, c->stream>>>(n, run, from, to);
+        c->launches++;
+        std::swap(from, to);
+    }
+    k_pairs_unique<<<1, 1024, 0, c->stream>>>(n, from, i1, i2, lv, d_nout);
     c->launches++;
     return launch_status(c, "sort_pairs_unique");
 }
@@ -453,15 +424,13 @@ __global__ void k_sas_sweep(int n1, const double *r1, const double *v1, const do
 }
 
 // The sorted order of one system's extents, up to SAS_MERGED of them: each block forms and sorts a
-// tile of SAS_TILE in shared memory, then rounds of merges join up to SAS_WAYS runs each; an
-// extent's place is its place in its run plus, run by run, the count of extents before it there
-// (a binary search).  Ties keep the extents' order, as in the radix sort: equal keys count from the
-// runs before the own one only.  Bound by launches and dependent loads: two to five launches here,
+// tile of SAS_TILE in shared memory, then rounds of merges join up to MERGE_WAYS runs each
+// (merge_place).  Ties keep the extents' order, as in the radix sort.  Bound by launches and dependent loads: two to five launches here,
 // up to 24 and a host read in the radix sort.  A whole pl-tp check, radix sort and this: 314 x 2501
 // bodies 168 -> 62 us, 2370 x 3650 220 -> 119, 8192 x 50,000 292 -> 198, 4000 x 200,000 462 -> 407,
 // 20,000 x 500,000 1012 and 1033, hence the line.  Merges of 16 runs: 50, 122, 191, 458 us; tiles of
 // 2048 took 60 us themselves.
-constexpr int SAS_TILE = 512, SAS_T = SAS_TILE / 2, SAS_WAYS = 8;
+constexpr int SAS_TILE = MERGE_TILE, SAS_T = SAS_TILE / 2;
 constexpr int64_t SAS_MERGED = 524288;
 __global__ void __launch_bounds__(SAS_T) k_sas_tiles(int n1, const double *r1, const double *v1, const double *renc1,
                                                      int n2, const double *r2, const double *v2, const double *renc2,
@@ -490,58 +459,24 @@ __global__ void __launch_bounds__(SAS_T) k_sas_tiles(int n1, const double *r1, c
         sk[l] = k;
         si[l] = (uint16_t)l;
     }
-    for (int k = 2; k <= SAS_TILE; k <<= 1)  // bitonic network on (key, place)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            __syncthreads();
-            const int i = 2 * (int)threadIdx.x - ((int)threadIdx.x & (j - 1)), q = i + j;
-            const uint64_t a = sk[i], b = sk[q];
-            const uint16_t x = si[i], y = si[q];
-            if ((a > b || (a == b && x > y)) == ((i & k) == 0)) {
-                sk[i] = b;
-                sk[q] = a;
-                si[i] = y;
-                si[q] = x;
-            }
-        }
-    __syncthreads();
+    blk_bitonic<true>(SAS_TILE, sk, si);
     for (int l = threadIdx.x; l < SAS_TILE && base + l < ne; l += SAS_T) {
         keys[base + l] = sk[l];
         ids[base + l] = (uint32_t)(base + si[l]);
     }
 }
-// Runs of `run` extents in (keys, ids) to runs of SAS_WAYS run in (okeys, oids), or, in the last
+// Runs of `run` extents in (keys, ids) to runs of MERGE_WAYS run in (okeys, oids), or, in the last
 // round (okeys null), to the sorted order: oids and the positions of each body's two extents.
 __global__ void __launch_bounds__(256) k_sas_merge(int ntot, int run, const uint64_t *__restrict__ keys,
                                                    const uint32_t *__restrict__ ids, uint64_t *okeys, uint32_t *oids,
                                                    int32_t *ibeg, int32_t *iend) {
     const int ne = 2 * ntot, q = blockIdx.x * 256 + threadIdx.x;
     if (q >= ne) return;
-    const uint64_t key = keys[q];
-    const int own = q / run, r0 = own / SAS_WAYS * SAS_WAYS;
-    int place = r0 * run + (q - own * run);
-    int lo[SAS_WAYS - 1], beg[SAS_WAYS - 1], end[SAS_WAYS - 1];
-    // the searches go in step: each step waits for its loads
-#pragma unroll
-    for (int w = 0; w < SAS_WAYS - 1; w++) {
-        const int r = r0 + w + (r0 + w >= own);  // the group's runs but the own one
-        beg[w] = lo[w] = min(r * run, ne);
-        end[w] = min((r + 1) * run, ne);
-    }
-#pragma unroll 1
-    for (int step = run; step > 0; step >>= 1)
-#pragma unroll
-        for (int w = 0; w < SAS_WAYS - 1; w++)
-            // all before lo count; the next `step` do if the last of them does
-            if (lo[w] + step <= end[w]) {
-                const uint64_t k = keys[lo[w] + step - 1];
-                if (k < key || (k == key && r0 + w < own)) lo[w] += step;
-            }
-#pragma unroll
-    for (int w = 0; w < SAS_WAYS - 1; w++) place += lo[w] - beg[w];
+    const int place = merge_place(q, ne, run, keys);
     const uint32_t e = ids[q];
     oids[place] = e;
     if (okeys)
-        okeys[place] = key;
+        okeys[place] = keys[q];
     else if (e < (uint32_t)ntot)
         ibeg[e] = place + 1;
     else
@@ -585,7 +520,7 @@ int sas_launch(swg_ctx *c, int n1, const double *r1, const double *v1, const dou
         int64_t run = SAS_TILE;
         uint64_t *from = keys, *to = bkeys;
         uint32_t *idf = ids, *idt = bids;
-        for (; run * SAS_WAYS < ne; run *= SAS_WAYS) {
+        for (; run * MERGE_WAYS < ne; run *= MERGE_WAYS) {
             k_sas_merge<<<grid, 256, 0, c->stream>>>(ntot, (int)run, from, idf, to, idt, nullptr, nullptr);
             std::swap(from, to);
             std::swap(idf, idt);

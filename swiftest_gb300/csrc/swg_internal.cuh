@@ -256,7 +256,6 @@ int drift_masked(swg_ctx *c, double mu, double *x, double *v, int32_t n, const i
                  bool fast = false);
 
 // encounter.cu -- encounter checks and sorting
-int64_t sort_padded_len(int64_t n);
 // Stable LSD radix sort of (key, val) by key (radix_sort.cu); with seg_of, the segment id
 // seg_of[val] (seg_bits wide) is the most significant part of the key.  host_skip: read a
 // digit histogram back to the host to skip constant digits (synchronizes the stream).

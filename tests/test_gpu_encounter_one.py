@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from swiftest_gb300 import SWG_ENC_SORTSWEEP
+from swiftest_gb300 import SWG_ENC_SORTSWEEP, SWG_ENC_TRIANGULAR
 from swiftest_gb300 import initial_conditions as IC
 
 pytestmark = pytest.mark.gpu
@@ -83,5 +83,21 @@ def test_plpl_sortsweep(ctx, n):
     r[1 : n : 1 + n // 20] *= 0.0  # extents around zero
     g = ctx.encounter_check_all_plpl(r, v, 0.1 * renc, 0.005, mode=SWG_ENC_SORTSWEEP, cap=10000)
     o = O.encounter_plpl(r, v, 0.1 * renc, 0.005, mode=SWG_ENC_SORTSWEEP)
+    for a, b in zip(g, o):
+        assert np.array_equal(a, b)
+
+
+# lists of one block's sort and its edge, one and two merge rounds and their edge, with every pair
+# found from both sides by the sweep
+@pytest.mark.parametrize("mode", [SWG_ENC_TRIANGULAR, SWG_ENC_SORTSWEEP])
+@pytest.mark.parametrize("m,n", [(1, 1), (2, 1), (32, 64), (7, 293), (45, 91), (64, 65), (90, 400)])
+def test_list_lengths(ctx, m, n, mode):
+    rng = np.random.default_rng(m * n)
+    r, tr = rng.normal(size=(m, 3)) * 1e-3 + [1.0, 0, 0], rng.normal(size=(n, 3)) * 1e-3 + [1.0, 0, 0]
+    v, tv = rng.normal(size=(m, 3)), rng.normal(size=(n, 3))
+    renc = np.full(m, 0.5)  # every pair
+    g = ctx.encounter_check_all_pltp(r, v, tr, tv, renc, 0.005, mode=mode, cap=40000)
+    o = O.encounter_pltp(r, v, tr, tv, renc, 0.005, mode=mode)
+    assert len(o[0]) == m * n or mode == SWG_ENC_SORTSWEEP
     for a, b in zip(g, o):
         assert np.array_equal(a, b)
