@@ -42,6 +42,21 @@ __global__ void k_encounter_prep(int n, const double *__restrict__ r, const doub
     V[i] = o.v;
 }
 
+// both lists of a check in one launch
+__global__ void k_encounter_prep2(int n1, const double *__restrict__ r1, const double *__restrict__ v1,
+                                  const double *__restrict__ renc1, float4 *F1, int n2, const double *__restrict__ r2,
+                                  const double *__restrict__ v2, const double *__restrict__ renc2, float4 *F2) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n1 + n2) return;
+    const bool first = t < n1;
+    const int i = first ? t : t - n1, n = first ? n1 : n2;
+    const BodyF o = load_body(first ? r1 : r2, first ? v1 : v2, first ? renc1 : renc2, i);
+    float4 *F = first ? F1 : F2;
+    F[i] = o.a;
+    F[n + i] = o.b;
+    F[2 * n + i] = o.v;
+}
+
 constexpr int EP = 64;  // partners per shared-memory tile
 
 
@@ -214,7 +229,7 @@ __device__ __forceinline__ I merge_place(I q, I n, I run, const uint64_t *__rest
 // Pairs (i1, i2, lv) sorted by (i1, i2), repeats dropped (they carry the same lv, 0 or 1).  One key
 // holds all three.  Up to PAIRS_BLOCK pairs in one block and launch; more in tiles and merges.
 // One key-value network of four launches before: a check of 4096 pl x 40,001 tp 99.7 -> 85.8 us, a
-// sort-and-sweep check of 20,000 x 500,000 (20,000 pairs) 969 -> 766 us.
+// sort-and-sweep check of 20,000 x 500,000 969 -> 766 us.
 constexpr int PAIRS_BLOCK = 2048;
 __device__ __forceinline__ uint64_t pair_key(int i1, int i2, int lv) {
     return ((uint64_t)(uint32_t)i1 << 32) | ((uint64_t)(uint32_t)i2 << 1) | (uint64_t)(lv != 0);
@@ -566,16 +581,15 @@ int encounter_launch(swg_ctx *c, int mode, int n1, const double *r1, const doubl
     // float copies for the prefilter: list 1 then (unless it is the same list) list 2
     float4 *A1 = (float4 *)sas_scratch, *B1 = A1 + n1, *V1 = B1 + n1;
     float4 *A2 = A1, *B2 = B1, *V2 = V1;
-    k_encounter_prep<<<(n1 + 255) / 256, 256, 0, c->stream>>>(n1, r1, v1, renc1, A1, B1, V1);
-    c->launches++;
     const bool same = upper && r2 == r1;
     if (!same) {
         A2 = V1 + n1;
         B2 = A2 + n2;
         V2 = B2 + n2;
-        k_encounter_prep<<<(n2 + 255) / 256, 256, 0, c->stream>>>(n2, r2, v2, renc2, A2, B2, V2);
-        c->launches++;
     }
+    const int np = n1 + (same ? 0 : n2);
+    k_encounter_prep2<<<(np + 127) / 128, 128, 0, c->stream>>>(n1, r1, v1, renc1, A1, np - n1, r2, v2, renc2, A2);
+    c->launches++;
     const int bx = (n2 + ET - 1) / ET;
     const int target = 4 * (c->num_sms > 0 ? c->num_sms : 152);
     int nchunk = (target + bx - 1) / bx;
@@ -684,8 +698,9 @@ namespace swg {
 
 // From this many pair tests on, a TRIANGULAR check of one list, or of massive bodies against test
 // particles, goes over radius-sorted tiles, which test a few percent of a disk's pairs but take
-// three launches and about 50 us; the all-pairs kernel tests 4.2e5 pairs per us.
-constexpr int64_t SORTED_PAIRS = 20000000;
+// two launches more; whole calls all-pairs / sorted: 300 x 20,000 66 / 67 us, 1000 x 10,000 72 / 72,
+// 400 x 50,000 93 / 72, 8192 x 50,000 935 / 112.
+constexpr int64_t SORTED_PAIRS = 10000000;
 
 int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1, const double *r1,
                          const double *v1, const double *renc1, int32_t n2, const double *r2, const double *v2,

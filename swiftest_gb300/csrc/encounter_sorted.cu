@@ -489,7 +489,7 @@ int encounter_plpl_sorted_batched(swg_ctx *c, int nsys, int nmax, const int32_t 
 // The radial order only steers the cull, so a long list is ordered in segments of SEG bodies,
 // one block each, instead of one block for all: a segment's sub-tiles are wider by its share of
 // the list, the list found is the same.  4096 pl x 40,001 tp: the check's kernel 23 us with segments
-// of 2048 or 4096 (98 us with 1024), the order 14 and 23 us; the whole call 480 -> 98 us.
+// of 2048 or 4096 (98 us with 1024), the order 14 and 23 us; the whole call 480 -> 86 us.
 constexpr int SEG = 2048, SEG_BITS = 16;
 static_assert(SEG % SB == 0, "segments are whole bound tiles");
 
