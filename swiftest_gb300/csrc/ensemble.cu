@@ -1755,26 +1755,21 @@ int ens_step(swg_ensemble *e, double dt) {
     bool have_acc = false;
     if (symba) {
         const int64_t nmax = std::max(e->NPL, e->NTP);
+        const bool beside = !e->prof.on && e->NPL > 0;
         k_symba_reset<<<grid_for(nmax, 256), 256, 0, c->stream>>>((int)e->NPL, (int)e->NTP, e->levelg, e->levelm,
                                                                    e->nplenc, e->ntpenc, e->lmask, e->tlevelg,
                                                                    e->tlevelm, e->tnplenc, e->tlmask, e->status,
-                                                                   e->tstatus);
+                                                                   e->tstatus,
+                                                                   beside ? StepSnap{e->rh, e->vb, e->trh, e->tvb, e->snap}
+                                                                          : StepSnap());
         SWG_TRY(L(c, "symba_reset"));
-        if (!e->prof.on && e->NPL > 0) {
+        if (beside) {
             // The level-0 checks read a copy of the start-of-step state on the side stream
             // while this stream runs the per-system sums and the first pair accelerations,
             // which do not depend on the lists; the lists are joined before the pair
             // subtraction.  Same arithmetic as the sequential order.
             const size_t n = e->NPL, m = e->NTP;
             double *sr = e->snap, *sv = sr + 3 * n, *st = sv + 3 * n, *stv = st + 3 * m;
-            SWG_TRY(cuda_status(c, cudaMemcpyAsync(sr, e->rh, 24 * n, cudaMemcpyDeviceToDevice, c->stream), "snap"));
-            SWG_TRY(cuda_status(c, cudaMemcpyAsync(sv, e->vb, 24 * n, cudaMemcpyDeviceToDevice, c->stream), "snap"));
-            if (m) {
-                SWG_TRY(cuda_status(c, cudaMemcpyAsync(st, e->trh, 24 * m, cudaMemcpyDeviceToDevice, c->stream),
-                                    "snap"));
-                SWG_TRY(cuda_status(c, cudaMemcpyAsync(stv, e->tvb, 24 * m, cudaMemcpyDeviceToDevice, c->stream),
-                                    "snap"));
-            }
             SWG_TRY(cuda_status(c, cudaEventRecord(e->ev_fork, c->stream), "fork"));
             SWG_TRY(cuda_status(c, cudaStreamWaitEvent(e->side, e->ev_fork, 0), "fork"));
             SWG_TRY(on_stream(c, e->side, [&] { return level0_launch(e, dt, sr, sv, st, stv); }));

@@ -2159,11 +2159,28 @@ static __global__ void k_kick_update(int n, double *v, const double *__restrict_
 // symba_step_reset_system (symba_step.f90:265-331) + set_renc(0).  The reference sets
 // lmask = .true. because removed bodies have left the arrays; here they stay in place with
 // status INACTIVE, so lmask is status /= INACTIVE.
+// snap: with a destination, a copy of the state for the level-0 checks that run beside the step's
+// opening (copies of their own took 2-3 us each).
+struct StepSnap {
+    const double *rh = nullptr, *vb = nullptr, *trh = nullptr, *tvb = nullptr;
+    double *to = nullptr;  // rh, vb, trh, tvb one after the other
+};
 static __global__ void k_symba_reset(int npl, int ntp, int32_t *levelg, int32_t *levelm, int32_t *nplenc, int32_t *ntpenc,
                               int32_t *lmask, int32_t *tlevelg, int32_t *tlevelm, int32_t *tnplenc,
                               int32_t *tlmask, const int32_t *__restrict__ status,
-                              const int32_t *__restrict__ tstatus) {
+                              const int32_t *__restrict__ tstatus, StepSnap snap) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (snap.to) {
+        const int64_t n = 3 * (int64_t)npl, m = 3 * (int64_t)ntp, stride = (int64_t)gridDim.x * blockDim.x;
+        for (int64_t k = i; k < n; k += stride) {
+            snap.to[k] = snap.rh[k];
+            snap.to[n + k] = snap.vb[k];
+        }
+        for (int64_t k = i; k < m; k += stride) {
+            snap.to[2 * n + k] = snap.trh[k];
+            snap.to[2 * n + m + k] = snap.tvb[k];
+        }
+    }
     if (i < npl) {
         levelg[i] = -1;
         levelm[i] = -1;

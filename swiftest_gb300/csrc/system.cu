@@ -1285,9 +1285,15 @@ int join_aside(swg_system *s) {
 int symba_step(swg_system *s, double dt) {
     swg_ctx *c = s->c;
     const int nmax = std::max(s->npl, s->ntp);
+    const size_t n = s->npl, m = s->ntp;
+    StepSnap snap;
+    if (!s->prof.on && n > 0) {
+        SWG_TRY(ensure(c, s->snap, sizeof(double) * 6 * (n + m)));
+        snap = StepSnap{s->rh, s->vb, s->trh, s->tvb, (double *)s->snap.ptr};
+    }
     k_symba_reset<<<grid_for(nmax, 256), 256, 0, c->stream>>>(s->npl, s->ntp, s->levelg, s->levelm, s->nplenc,
                                                                s->ntpenc, s->lmask, s->tlevelg, s->tlevelm,
-                                                               s->tnplenc, s->tlmask, s->status, s->tstatus);
+                                                               s->tnplenc, s->tlmask, s->status, s->tstatus, snap);
     SWG_TRY(L(c, "symba_reset"));
     s->lfirst_tp = s->lfirstkick;
     s->lfirst_pl = s->lfirstkick;
@@ -1313,15 +1319,7 @@ int symba_step(swg_system *s, double dt) {
     // HELIO step take first and which do not need the lists; the lists are joined before
     // the encounter-pair subtraction.  Every kernel's arithmetic is unchanged.
     SWG_TRY(ensure_side(s));
-    const size_t n = s->npl, m = s->ntp;
-    SWG_TRY(ensure(c, s->snap, sizeof(double) * 6 * (n + m)));
     double *sr = (double *)s->snap.ptr, *sv = sr + 3 * n, *st = sv + 3 * n, *stv = st + 3 * m;
-    SWG_TRY(cuda_status(c, cudaMemcpyAsync(sr, s->rh, 24 * n, cudaMemcpyDeviceToDevice, c->stream), "snap"));
-    SWG_TRY(cuda_status(c, cudaMemcpyAsync(sv, s->vb, 24 * n, cudaMemcpyDeviceToDevice, c->stream), "snap"));
-    if (m) {
-        SWG_TRY(cuda_status(c, cudaMemcpyAsync(st, s->trh, 24 * m, cudaMemcpyDeviceToDevice, c->stream), "snap"));
-        SWG_TRY(cuda_status(c, cudaMemcpyAsync(stv, s->tvb, 24 * m, cudaMemcpyDeviceToDevice, c->stream), "snap"));
-    }
     SWG_TRY(join(c, c->stream, s->side, s->ev[5]));
     const double dth = 0.5 * dt;
     if (s->lfirst_pl) SWG_TRY(vh2vb_pl(s));
