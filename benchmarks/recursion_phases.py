@@ -43,10 +43,10 @@ def _patch(s: str) -> str:
         "    blk_build_adjacency(a, nbpl, nbtp);\n    PH(0, t0)\n    RecStage S{};")
     rep("        stg_load(a, S, nbpl, nbtp);\n    }", "        stg_load(a, S, nbpl, nbtp);\n    }\n    PH(11, t0)")
     for call, k in (("stg_list_check(a, S, irecp, dtl, &s_any, s_rs);", 1),
-                    ("stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);\n                stg_drift", 2),
+                    ("stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);\n                stg_drift", 2),
                     ("stg_drift(a, S, nbpl, nbtp, ireci, dtl, inv_gm);", 3),
                     ("blk_list_check(a, irecp, dtl, &s_any, s_rs);", 1),
-                    ("blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);\n                blk_drift", 2),
+                    ("blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);\n                blk_drift", 2),
                     ("blk_drift(a, nbpl, nbtp, ireci, dtl, inv_gm);", 3)):
         if call.endswith("stg_drift") or call.endswith("blk_drift"):
             head, tail = call.split("\n")
@@ -57,8 +57,8 @@ def _patch(s: str) -> str:
         "            if (threadIdx.x == 0) atomicAdd(&g_ph[10], 1ull);\n            const int any = s_any;")
     rep("        // after the deeper levels (or none) for loop j of level ireci\n",
         "        // after the deeper levels (or none) for loop j of level ireci\n        PH(8, t0)\n")
-    rep("            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);\n        if (a.lclose) {",
-        "            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);\n        PH(4, t0)\n"
+    rep("            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);\n        if (a.lclose) {",
+        "            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);\n        PH(4, t0)\n"
         "        if (a.lclose) {")
     rep("                blk_collision_check(a, ireci, dtl, &s_any);",
         "                blk_collision_check(a, ireci, dtl, &s_any);\n            PH(5, t0)")

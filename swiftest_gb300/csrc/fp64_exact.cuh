@@ -210,28 +210,6 @@ __device__ __forceinline__ double x_half(double a) {
     return __hiloint2double(h - 0x100000, __double2loint(a));
 }
 
-// 1 / sqrt(x) to about one unit in the last place, x_ok(x): the FP32 pair of x_sqrt, then
-// one Newton step in FP64 (three dependent FP64 instructions: the shortest chain, for code
-// that waits for one result).
-__device__ __forceinline__ double x_rsqrt(double x) {
-    const int hi = __double2hiint(x), lo = __double2loint(x);
-    const int odd = (~hi >> 20) & 1;
-    const float mh = __int_as_float(((__funnelshift_l(lo, hi, 3) & 0xffffff) ^ 0x800000) + 0x3f800000);
-    const float ml = x_mant_lo(lo, odd);
-    const float y = x_rsqrt_approx(mh);
-    if (!x_ok(hi) || y < 0.5f) return rsqrt(x);  // y: another binade (one in 2^23)
-    const float th = y * y, tl = fmaf(y, y, -th);
-    const float e = fmaf(-mh, th, 1.0f) - fmaf(mh, tl, ml * th);
-    const float c = y * fmaf(0.375f * e, e, 0.5f * e);
-    // y + c as a double: the mantissa of y with c added in units of 2^-53, y in (1/2, 1]
-    const int yb = __float_as_int(y);
-    const uint64_t m = ((uint64_t)(uint32_t)((yb >> 3) + ((1023 - 127) << 20)) << 32 | ((uint32_t)yb << 29)) +
-                       (int64_t)__float2int_rn(c * 9007199254740992.0f);
-    // scaled by 2^-(k / 2), x = m 4^(k / 2)
-    const double r = __longlong_as_double((long long)(m - ((uint64_t)(uint32_t)(((hi - 0x3ff00000) >> 1) & 0xfff00000) << 32)));
-    return fma(x_half(r), fma(-(x * r), r, 1.0), r);
-}
-
 // ---- any operands: the exact forms above where they apply, else the native operation (out of
 // line).  xdiv and xsqrt give the bits of a / b and sqrt(x).
 static __device__ __noinline__ double x_native_div(double a, double b) { return a / b; }
@@ -257,7 +235,7 @@ __device__ __forceinline__ double xsqrt(double x) {
 // branch, one long chain per body, is faster inline).
 static __device__ __noinline__ double xdiv_call(double a, double b) { return xdiv(a, b); }
 static __device__ __noinline__ double xsqrt_call(double x) { return xsqrt(x); }
-static __device__ __noinline__ double x_rsqrt_call(double x) { return x_rsqrt(x); }
+static __device__ __noinline__ double rsqrt_call(double x) { return rsqrt(x); }
 static __device__ __noinline__ double x_native_mul(double a, double b) { return a * b; }
 __device__ __forceinline__ double xmul(double a, double b) {
     const int ah = __double2hiint(a), bh = __double2hiint(b);

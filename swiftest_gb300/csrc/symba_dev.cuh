@@ -620,16 +620,19 @@ __device__ __forceinline__ double d_shell_base(bool isp, double rhill1, double r
 
 // The kick factors of one pair at level irec (symba_kick_list_plpl / _pltp, symba_kick.f90:126-340):
 // kp / km: the +1 / -1 kick acts (r^2 not below the next shell); fp / fm: its factor.  base:
-// d_shell_base.  Mixed path: isb = 1 / sqrt(base), so 1 / sqrt(ri) is a product with the table ik[k] =
-// RSHELL^-k / (1 - RSHELL); the -1 kick's inner limit is the +1 kick's outer one.  FP64 path: the
+// d_shell_base.  Mixed path: reciprocal square roots of r^2 and of the one shell radius that the pair
+// lies in (the -1 kick's inner limit is the +1 kick's outer one), CUDA's own, off by 0.506 units in
+// the last place at most; an FP32 pair with one Newton step was off by 0.99, with
+// 1 / sqrt(ri) as a product of 1 / sqrt(base) and a table of RSHELL^-k the polynomial's
+// error grew from 1.8 to 2.5 units of 2^-53 rms, for a kick of 4.85k instead of 5.0k cycles.  FP64 path: the
 // reference's operations, with IEEE square roots and quotients (fp64_exact.cuh) and the correctly
 // rounded r^-1.5 shared with the oracle.
 struct KickFac {
     bool kp, km;
     double fp, fm;
 };
-__device__ __forceinline__ KickFac d_kick_factors(bool fast, bool both, double base, double isb, const double *dx,
-                                                  double shell_p, double shell_m, double ik_p, double ik_m) {
+__device__ __forceinline__ KickFac d_kick_factors(bool fast, bool both, double base, const double *dx, double shell_p,
+                                                  double shell_m) {
     KickFac k;
     const double ri_p = base * shell_p, ri_m = base * shell_m;
     constexpr double R2 = RSHELL * RSHELL;
@@ -639,14 +642,13 @@ __device__ __forceinline__ KickFac d_kick_factors(bool fast, bool both, double b
         const bool out_p = !x_less(r2, ri_p);
         k.km = both && out_p;
         if (!k.kp) return k;
-        const double y = x_rsqrt_call(r2), r = r2 * y, ir3 = (y * y) * y;
-        auto shell = [&](double q) {  // rr = (1 - r / sqrt(ri)) / (1 - RSHELL); 1 - 3 rr^2 + 2 rr^3 as 1 + rr^2 (2 rr - 3)
-            const double rr = fma(-r, q, 1.0 / (1.0 - RSHELL));
-            return ir3 * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
-        };
+        const double y = rsqrt_call(r2), r = r2 * y, ir3 = (y * y) * y;
         k.fp = k.fm = ir3;
-        if (!out_p) k.fp = shell(isb * ik_p);
-        else if (k.km && x_less(r2, ri_m)) k.fm = shell(isb * ik_m);
+        const double ri = out_p ? ri_m : ri_p;
+        if (out_p && !(k.km && x_less(r2, ri))) return k;  // outside both shells
+        // rr = (1 - r / sqrt(ri)) / (1 - RSHELL); 1 - 3 rr^2 + 2 rr^3 as 1 + rr^2 (2 rr - 3)
+        const double rr = fma(-r, rsqrt_call(ri), 1.0) * (1.0 / (1.0 - RSHELL));
+        (out_p ? k.fm : k.fp) = ir3 * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
         return k;
     }
     const double r2 = dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
@@ -771,9 +773,9 @@ static __device__ void blk_list_check(const RecArgs &a, int irec, double dt, int
 // (r^2 < rim1).  terms: 12 doubles per entry, the +1 pair terms then the -1 pair terms.
 // The reference's lmask refresh at entry is kept by the step loop instead (lmask ==
 // status /= INACTIVE wherever the recursion runs).
-// pw[m] = d_powi(RSHELL, m), m <= 2 MAXLEV; ik[k] = RSHELL^-k / (1 - RSHELL) (mixed path).
+// pw[m] = d_powi(RSHELL, m), m <= 2 MAXLEV.
 static __device__ void blk_kick_lists(const RecArgs &a, int nbpl, int nbtp, double dt, int irec, bool both,
-                                      const double *pw, const double *ik) {
+                                      const double *pw) {
     const int64_t npp = a.npp, npt = a.npt;
     if (npp + npt == 0) return;
     const int irm1 = irec - 1;
@@ -806,8 +808,7 @@ static __device__ void blk_kick_lists(const RecArgs &a, int nbpl, int nbtp, doub
         const double *rj = isp ? &a.rh[3 * j] : &a.trh[3 * j];
         double dx[3];
         for (int d = 0; d < 3; d++) dx[d] = rj[d] - a.rh[3 * i + d];
-        const KickFac f = d_kick_factors(a.fast, both, base, a.fast ? x_rsqrt(base) : 0.0, dx, shell_p, shell_m,
-                                         ik[irec], ik[irec - 1]);
+        const KickFac f = d_kick_factors(a.fast, both, base, dx, shell_p, shell_m);
         if (c == 0) {
             a.good[k] = f.kp ? 1 : 2;
             a.good2[k] = both ? (f.km ? 1 : 2) : 0;
@@ -1139,7 +1140,7 @@ struct RecStage {
     double *r, *v;                 // per slot: position, velocity (3 each)
     double *gm, *rhs, *rad;        // per slot: G*m, Hill radius * rhscale, radius (0 for test particles)
     double *terms;                 // 12 per entry
-    double *base, *isb;            // per entry: d_shell_base and (mixed path) 1 / its square root
+    double *base;                  // per entry: d_shell_base
     int32_t *lev, *st, *gidx;      // per slot: levelg / tlevelg, status / tstatus, global index
     int32_t *s1, *s2;              // per entry: slots of index1 and index2
     int32_t *est, *elev, *elv;     // per entry: status, level, lvdotr
@@ -1153,7 +1154,7 @@ constexpr size_t REC_STAGE_MAX = 160 * 1024, REC_STAGE_ENS = 64 * 1024;
 // (a pl-tp entry names one pl and one tp), and 2 npp + npt adjacency entries.
 __host__ __device__ inline size_t rec_stage_bytes(int64_t npp, int64_t npt) {
     const int64_t n = npp + npt, nb = 2 * n;
-    return (size_t)(9 * nb + 14 * n) * 8 + (size_t)(4 * nb + 5 * n + 2 * npp + npt) * 4 + (size_t)(3 * n + 16);
+    return (size_t)(9 * nb + 13 * n) * 8 + (size_t)(4 * nb + 5 * n + 2 * npp + npt) * 4 + (size_t)(3 * n + 16);
 }
 static __device__ RecStage rec_stage_carve(void *base, int64_t npp, int64_t npt) {
     const int64_t n = npp + npt, nb = 2 * n;
@@ -1166,8 +1167,7 @@ static __device__ RecStage rec_stage_carve(void *base, int64_t npp, int64_t npt)
     S.rad = d + 8 * nb;
     S.terms = d + 9 * nb;
     S.base = S.terms + 12 * n;
-    S.isb = S.base + n;
-    int32_t *i = (int32_t *)(S.isb + n);
+    int32_t *i = (int32_t *)(S.base + n);
     S.lev = i;
     S.st = i + nb;
     S.gidx = i + 2 * nb;
@@ -1215,7 +1215,6 @@ static __device__ void stg_load(const RecArgs &a, const RecStage &S, int nbpl, i
         S.s1[k] = a.mark_pl[i] - 1;
         S.s2[k] = isp ? a.mark_pl[j] - 1 : a.mark_tp[j] - 1;
         S.base[k] = d_shell_base(isp, a.rhill[i], isp ? a.rhill[j] : 0.0, a.rhscale * a.rhscale);
-        S.isb[k] = a.fast ? x_rsqrt(S.base[k]) : 0.0;
         S.elv[k] = l[2 * cap + q];
         S.est[k] = l[3 * cap + q];
         S.elev[k] = l[4 * cap + q];
@@ -1288,7 +1287,7 @@ static __device__ void stg_list_check(const RecArgs &a, const RecStage &S, int i
 }
 // blk_kick_lists on the stage (same pair terms, same per-body order)
 static __device__ void stg_kick_lists(const RecArgs &a, const RecStage &S, int nbpl, int nbtp, double dt, int irec,
-                                      bool both, const double *pw, const double *ik) {
+                                      bool both, const double *pw) {
     const int npp = (int)a.npp, n = (int)(a.npp + a.npt);  // the stage holds a few hundred entries
     if (n == 0) return;
     const int irm1 = irec - 1;
@@ -1311,8 +1310,7 @@ static __device__ void stg_kick_lists(const RecArgs &a, const RecStage &S, int n
         }
         double dx[3];
         for (int d = 0; d < 3; d++) dx[d] = S.r[3 * b2 + d] - S.r[3 * b1 + d];
-        const KickFac f =
-            d_kick_factors(a.fast, both, S.base[k], S.isb[k], dx, shell_p, shell_m, ik[irec], ik[irec - 1]);
+        const KickFac f = d_kick_factors(a.fast, both, S.base[k], dx, shell_p, shell_m);
         if (c == 0) {
             S.good[k] = f.kp ? 1 : 2;
             S.good2[k] = both ? (f.km ? 1 : 2) : 0;
@@ -1419,14 +1417,12 @@ static __device__ void blk_symba_recursion_t(const RecArgs &a, void *stage) {
     // shell-radius powers, formed once per launch with the per-call algorithms (same bits):
     // s_pw[m] = d_powi(RSHELL, m) (the kick's shell radii), s_rs[k] = RSHELL^k by repeated
     // products (d_renc, the list check's encounter radii)
-    // s_ik[k] = RSHELL^-k / (1 - RSHELL) (the mixed path's shell polynomial)
-    __shared__ double s_pw[2 * MAXLEV + 2], s_rs[MAXLEV + 1], s_ik[MAXLEV + 1];
+    __shared__ double s_pw[2 * MAXLEV + 2], s_rs[MAXLEV + 1];
     // each level's step dt / 3^k and the underflow test of symba_step.f90:196-201, formed
     // once per launch as the loop would form them (the FP64 divides are long on GB300)
     __shared__ double s_dtl[MAXLEV];
     __shared__ unsigned char s_under[MAXLEV];
     for (int m = threadIdx.x; m < 2 * MAXLEV + 2; m += blockDim.x) s_pw[m] = d_powi(RSHELL, m);
-    for (int k = threadIdx.x; k <= MAXLEV; k += blockDim.x) s_ik[k] = xdiv_call(1.0 / (1.0 - RSHELL), d_powi(RSHELL, k));
     for (int k = threadIdx.x; k < MAXLEV; k += blockDim.x) {
         double p3 = 1.0;
         for (int q = 0; q < k; q++) p3 *= 3.0;
@@ -1507,11 +1503,11 @@ static __device__ void blk_symba_recursion_t(const RecArgs &a, void *stage) {
             __syncthreads();
             if constexpr (STAGED) {
                 stg_list_check(a, S, irecp, dtl, &s_any, s_rs);
-                stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
+                stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
                 stg_drift(a, S, nbpl, nbtp, ireci, dtl, inv_gm);
             } else {
                 blk_list_check(a, irecp, dtl, &s_any, s_rs);
-                blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
+                blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
                 blk_drift(a, nbpl, nbtp, ireci, dtl, inv_gm);
             }
             const int any = s_any;
@@ -1532,9 +1528,9 @@ static __device__ void blk_symba_recursion_t(const RecArgs &a, void *stage) {
         }
         // after the deeper levels (or none) for loop j of level ireci
         if constexpr (STAGED)
-            stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
+            stg_kick_lists(a, S, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
         else
-            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw, s_ik);
+            blk_kick_lists(a, nbpl, nbtp, dth, irecp, ireci != 0, s_pw);
         if (a.lclose) {
             if (threadIdx.x == 0) s_any = 0;
             __syncthreads();

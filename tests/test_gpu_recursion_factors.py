@@ -1,0 +1,81 @@
+"""Accuracy of the recursion's kick factors in the mixed path (symba_dev.cuh d_kick_factors): against
+extended precision on the host, no larger than with a native rsqrt each of r^2 and the
+shell's radius.  The device function is compiled into a probe."""
+import ctypes as C
+import subprocess
+
+import numpy as np
+import pytest
+
+from swiftest_gb300 import build as B
+
+pytestmark = pytest.mark.gpu
+
+RSHELL = 0.48075  # the ratio of two shells' radii
+N, LEVELS = 400000, 9
+
+PROBE = r"""
+#include "symba_dev.cuh"
+using namespace swg;
+__global__ void k(int n, const double *r2, const double *base, const int *lev, const double *pw, double *o) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double d[3] = {sqrt(r2[i]), 0.0, 0.0}, x = fma(d[0], d[0], 0.0);
+    const int l = lev[i];
+    o[i] = x;
+    // the pair's shell: the +1 kick's at level l, or the -1 kick's from level l + 1
+    const sdev::KickFac a = sdev::d_kick_factors(true, false, base[i], d, pw[2 * l], 0.0);
+    const sdev::KickFac b = sdev::d_kick_factors(true, true, base[i], d, pw[2 * (l + 1)], pw[2 * l]);
+    o[n + i] = a.fp;
+    o[2 * n + i] = b.fm;
+    const double ri = base[i] * pw[2 * l], y = rsqrt(x), r = x * y;
+    const double rr = fma(-r, rsqrt(ri), 1.0) * (1.0 / (1.0 - RSHELL));
+    o[3 * n + i] = ((y * y) * y) * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
+    o[4 * n + i] = ri;
+}
+extern "C" int probe(int n, const double *r2, const double *base, const int *lev, int m, const double *pw, double *o) {
+    const size_t b = sizeof(double) * n;
+    double *d;
+    int *l;
+    if (cudaMalloc(&d, 8 * b + 8 * m) || cudaMalloc(&l, 4 * n)) return 1;
+    cudaMemcpy(d, r2, b, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + n, base, b, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + 8 * n, pw, 8 * m, cudaMemcpyHostToDevice);
+    cudaMemcpy(l, lev, 4 * n, cudaMemcpyHostToDevice);
+    k<<<(n + 127) / 128, 128>>>(n, d, d + n, l, d + 8 * n, d + 2 * n);
+    cudaMemcpy(o, d + 2 * n, 5 * b, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    cudaFree(l);
+    return (int)cudaGetLastError();
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def values(tmp_path_factory):
+    tmp = tmp_path_factory.mktemp("probe")
+    (tmp / "probe.cu").write_text(PROBE)
+    subprocess.run([B.nvcc(), *B.ARCH, *B.NVFLAGS, "-I", str(B.CSRC), "-shared", "-o", str(tmp / "probe.so"),
+                    str(tmp / "probe.cu")], check=True)
+    rng = np.random.default_rng(1)
+    base = 10.0 ** rng.uniform(-12, -2, N)
+    lev = rng.integers(0, LEVELS, N).astype(np.int32)
+    pw = RSHELL ** np.arange(2 * LEVELS + 2)
+    # inside the shell, clear of its two edges (whose sides the factors do not share)
+    r2 = base * pw[2 * lev] * rng.uniform(RSHELL * (1 + 1e-9), 1 - 1e-9, N) ** 2
+    o = np.zeros((5, N))
+    p = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    assert C.CDLL(str(tmp / "probe.so")).probe(N, p(r2), p(base), p(lev), len(pw), p(pw), p(o)) == 0
+    return o
+
+
+def test_shell_factors(values):
+    x, fp, fm, native, ri = values
+    x, ri = x.astype(np.longdouble), ri.astype(np.longdouble)
+    r = np.sqrt(x)
+    rr = (1 - r / np.sqrt(ri)) / (1 - np.longdouble(RSHELL))
+    ir3 = 1 / (x * r)
+    exact = ir3 * (1 - 3 * rr ** 2 + 2 * rr ** 3)
+    rms = lambda v: float(np.sqrt((((v - exact) / ir3) ** 2).mean()) * 2.0 ** 53)  # noqa: E731
+    # the sample's spread of an rms over 400,000 values is 0.1 to 0.2%
+    assert rms(fp) < 1.01 * rms(native) and rms(fm) < 1.01 * rms(native)
