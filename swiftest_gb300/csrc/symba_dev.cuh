@@ -1142,9 +1142,11 @@ struct RecStage {
     double *terms;                 // 12 per entry
     double *base;                  // per entry: d_shell_base
     int32_t *lev, *st, *gidx;      // per slot: levelg / tlevelg, status / tstatus, global index
-    int32_t *s1, *s2;              // per entry: slots of index1 and index2
-    int32_t *est, *elev, *elv;     // per entry: status, level, lvdotr
+    int32_t *est;                  // per entry: status
     int32_t *adj_end, *adj;        // the adjacency of blk_build_adjacency
+    uint16_t *s1, *s2;             // per entry: slots of index1 and index2
+    int8_t *elev;                  // per entry: level (below MAXLEV)
+    uint8_t *elv;                  // per entry: lvdotr
     uint8_t *lenc, *good, *good2;  // per entry
 };
 // Largest stage of a single-system launch, and of each block of an ensemble launch (every
@@ -1152,10 +1154,17 @@ struct RecStage {
 constexpr size_t REC_STAGE_MAX = 160 * 1024, REC_STAGE_ENS = 64 * 1024;
 // Bytes of the stage for npp pl-pl and npt pl-tp entries: at most two bodies per entry
 // (a pl-tp entry names one pl and one tp), and 2 npp + npt adjacency entries.
-__host__ __device__ inline size_t rec_stage_bytes(int64_t npp, int64_t npt) {
+__host__ __device__ constexpr size_t rec_stage_bytes(int64_t npp, int64_t npt) {
     const int64_t n = npp + npt, nb = 2 * n;
-    return (size_t)(9 * nb + 13 * n) * 8 + (size_t)(4 * nb + 5 * n + 2 * npp + npt) * 4 + (size_t)(3 * n + 16);
+    return (size_t)(9 * nb + 13 * n) * 8 + (size_t)(4 * nb + n + 2 * npp + npt) * 4 + (size_t)(4 * n) +
+           (size_t)(5 * n + 16);
 }
+// Short fields keep an entry at 301 bytes.  A list that just misses the stage takes the global
+// arrays: 526 pl-pl entries of one system, mixed, 6.5 ms a step there and 5.4 on the stage.
+static_assert(rec_stage_bytes(544, 0) <= REC_STAGE_MAX && rec_stage_bytes(0, 551) <= REC_STAGE_MAX &&
+                  rec_stage_bytes(217, 0) <= REC_STAGE_ENS && rec_stage_bytes(0, 220) <= REC_STAGE_ENS,
+              "lists of this length are staged");
+static_assert(MAXLEV < 128 && REC_STAGE_MAX / 297 * 2 < 65536, "levels fit 8 bits, slots 16");
 static __device__ RecStage rec_stage_carve(void *base, int64_t npp, int64_t npt) {
     const int64_t n = npp + npt, nb = 2 * n;
     RecStage S;
@@ -1172,16 +1181,16 @@ static __device__ RecStage rec_stage_carve(void *base, int64_t npp, int64_t npt)
     S.st = i + nb;
     S.gidx = i + 2 * nb;
     S.adj_end = i + 3 * nb;
-    S.s1 = i + 4 * nb;
+    S.est = i + 4 * nb;
+    S.adj = S.est + n;
+    S.s1 = (uint16_t *)(S.adj + 2 * npp + npt);
     S.s2 = S.s1 + n;
-    S.est = S.s2 + n;
-    S.elev = S.est + n;
-    S.elv = S.elev + n;
-    S.adj = S.elv + n;
-    uint8_t *b = (uint8_t *)(S.adj + 2 * npp + npt);
-    S.lenc = b;
-    S.good = b + n;
-    S.good2 = b + 2 * n;
+    S.elev = (int8_t *)(S.s2 + n);
+    uint8_t *b = (uint8_t *)(S.elev + n);
+    S.elv = b;
+    S.lenc = b + n;
+    S.good = b + 2 * n;
+    S.good2 = b + 3 * n;
     return S;
 }
 // Copy the listed bodies and the list entries in (after blk_build_adjacency: mark_pl /
@@ -1212,12 +1221,12 @@ static __device__ void stg_load(const RecArgs &a, const RecStage &S, int nbpl, i
         const int32_t *l = isp ? a.pp : a.pt;
         const int64_t cap = isp ? a.ppcap : a.ptcap;
         const int i = l[q] - 1, j = l[cap + q] - 1;
-        S.s1[k] = a.mark_pl[i] - 1;
-        S.s2[k] = isp ? a.mark_pl[j] - 1 : a.mark_tp[j] - 1;
+        S.s1[k] = (uint16_t)(a.mark_pl[i] - 1);
+        S.s2[k] = (uint16_t)(isp ? a.mark_pl[j] - 1 : a.mark_tp[j] - 1);
         S.base[k] = d_shell_base(isp, a.rhill[i], isp ? a.rhill[j] : 0.0, a.rhscale * a.rhscale);
-        S.elv[k] = l[2 * cap + q];
+        S.elv[k] = (uint8_t)l[2 * cap + q];
         S.est[k] = l[3 * cap + q];
-        S.elev[k] = l[4 * cap + q];
+        S.elev[k] = (int8_t)l[4 * cap + q];
     }
     for (int64_t e = threadIdx.x; e < 2 * a.npp + a.npt; e += blockDim.x) S.adj[e] = a.adj[e];
     __syncthreads();
@@ -1266,7 +1275,7 @@ static __device__ void stg_list_check(const RecArgs &a, const RecStage &S, int i
             }
             int lvd;
             const bool le = d_list_pair(a.fast, isp, xr, vr, S.rhs[b1], S.rhs[b2], rs_pow[irec], S.rad[b1], S.rad[b2], dt, lvd);
-            S.elv[k] = lvd;
+            S.elv[k] = (uint8_t)lvd;
             le_out = (uint8_t)le;
         }
         S.lenc[k] = le_out;
@@ -1281,7 +1290,7 @@ static __device__ void stg_list_check(const RecArgs &a, const RecStage &S, int i
         atomicMax(&a.levelm[S.gidx[b1]], irec);
         S.lev[b2] = irec;
         atomicMax(isp ? &a.levelm[S.gidx[b2]] : &a.tlevelm[S.gidx[b2]], irec);
-        S.elev[k] = irec;
+        S.elev[k] = (int8_t)irec;
     }
     __syncthreads();
 }
@@ -1378,7 +1387,7 @@ static __device__ void stg_set_recur_levels(const RecArgs &a, const RecStage &S,
     for (int b = spread_tid(); b < nbpl + nbtp; b += blockDim.x)
         if (S.lev[b] == irecp) S.lev[b] = ireci;
     for (int64_t k = threadIdx.x; k < a.npp + a.npt; k += blockDim.x)
-        if (S.elev[k] == irecp) S.elev[k] = ireci;
+        if (S.elev[k] == irecp) S.elev[k] = (int8_t)ireci;
     __syncthreads();
 }
 // blk_collision_check on the stage
