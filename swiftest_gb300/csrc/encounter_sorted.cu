@@ -230,7 +230,8 @@ struct WarpStage {
 // that is not apart the lanes stage its partners in the warp's shared slots and each lane
 // runs its receiver against them.  nplm (optional, GMTINY): per system the count of fully
 // interacting bodies; a pair of two bodies both at local index >= nplm[s] is not tested
-// (the reference checks plm x pl only: encounter_check_all_plplm).
+// (the reference checks plm x pl only: encounter_check_all_plplm).  pchunk > 0: the item's
+// fourth field c selects the partner sub-tiles [c pchunk, (c + 1) pchunk), as in k_pltp_sorted.
 __global__ void __launch_bounds__(SQ) k_encounter_sorted(const int4 *__restrict__ items, const int32_t *__restrict__ poff,
                                                          const int32_t *__restrict__ tbase,
                                                          const int32_t *__restrict__ perm, const float4 *__restrict__ A,
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(SQ) k_encounter_sorted(const int4 *__restrict_
                                                          double dt, long long cap, int32_t *__restrict__ o1,
                                                          int32_t *__restrict__ o2, int32_t *__restrict__ olv,
                                                          unsigned long long *__restrict__ count,
-                                                         const int32_t *__restrict__ nplm) {
+                                                         const int32_t *__restrict__ nplm, int pchunk) {
     __shared__ WarpStage st_all[SQ / 32];
     const int4 w = items[blockIdx.x];
     const int s = w.x, q0 = w.y, nr = w.z;
@@ -264,9 +265,13 @@ __global__ void __launch_bounds__(SQ) k_encounter_sorted(const int4 *__restrict_
     const float dtf = __double2float_ru(fabs(dt)) * (1.0f + 1e-6f);
     const int gm = nplm ? o + nplm[s] : INT32_MAX;  // first semi-interacting body (global index)
     const int pend = qb - 1;  // partners p < q <= qb - 1
-    const int nsub = (pend + 31) / 32;
-    for (int u0 = 0; u0 < nsub; u0 += 32) {
-        const bool keep = u0 + lane < nsub && !tiles_apart(S[u0 + lane], QW);
+    int ubeg = 0, uend = (pend + 31) / 32;
+    if (pchunk > 0) {
+        ubeg = w.w * pchunk;
+        uend = min(uend, ubeg + pchunk);
+    }
+    for (int u0 = ubeg; u0 < uend; u0 += 32) {
+        const bool keep = u0 + lane < uend && !tiles_apart(S[u0 + lane], QW);
         unsigned m = __ballot_sync(0xffffffffu, keep);
         while (m) {
             const int p0 = 32 * (u0 + __ffs(m) - 1);
@@ -480,7 +485,7 @@ int encounter_plpl_sorted_batched(swg_ctx *c, int nsys, int nmax, const int32_t 
     c->launches++;
     SWG_TRY(launch_status(c, "sorted_prep"));
     k_encounter_sorted<<<nitems, SQ, 0, c->stream>>>(items, poff, tbase, perm, F, F + NPL, F + 2 * NPL, bounds, r,
-                                                     v, renc, dt, cap, o1, o2, olv, count, nplm);
+                                                     v, renc, dt, cap, o1, o2, olv, count, nplm, 0);
     c->launches++;
     return launch_status(c, "encounter_sorted");
 }
@@ -492,6 +497,12 @@ int encounter_plpl_sorted_batched(swg_ctx *c, int nsys, int nmax, const int32_t 
 // of 2048 or 4096 (98 us with 1024), the order 14 and 23 us; the whole call 480 -> 86 us.
 constexpr int SEG = 2048, SEG_BITS = 16;
 static_assert(SEG % SB == 0, "segments are whole bound tiles");
+// Items of a check, each 128 receivers by a chunk of the partners' sub-tiles: enough to fill the GPU
+// also where the radial bounds leave most pairs (narrow rings, long steps, large radii).  One list
+// takes four times as many, half of them beyond its triangle.  One list of 8192 bodies, one item per 128
+// receivers / 1024 / 2048 / 4096 items: a ring 1e-4 wide 890 / 199 / 163 / 164 us (all pairs 399), a disk
+// with a step of 0.05 2182 / 948 / 869 / 544 (874), with 0.005 95 / 75 / 78 / 82 (179).
+constexpr int ONE_BLOCKS = 1024;
 
 // The two lists of one check (n2 == 0: one list); per list its order, float copies and bounds.
 struct OneLists {
@@ -543,11 +554,10 @@ OnePlan one_plan(int n1, int n2, char *base) {
     p.seg2 = up(n2, SEG);
     p.l.nt1 = up(n1, SB);
     p.nt2 = up(n2, SB);
-    // about 1024 blocks, so that the check fills the GPU
     const int nq = up(n2 ? n2 : n1, SQ), nsub = up(n1, 32);
-    p.nchunk = n2 ? std::max(1, std::min(nsub, 1024 / std::max(nq, 1))) : 1;
-    p.pchunk = n2 ? up(nsub, p.nchunk) : 0;
-    if (n2) p.nchunk = up(nsub, p.pchunk);
+    p.nchunk = std::max(1, std::min(nsub, (n2 ? 1 : 4) * ONE_BLOCKS / std::max(nq, 1)));
+    p.pchunk = up(nsub, p.nchunk);
+    p.nchunk = up(nsub, p.pchunk);
     p.nitems = nq * p.nchunk;
     size_t at = 0;
     auto take = [&](size_t bytes) {
@@ -590,7 +600,7 @@ int encounter_sorted_one(swg_ctx *c, int n1, const double *r1, const double *v1,
     if (n2 == 0) {
         k_encounter_sorted<<<p.nitems, SQ, 0, c->stream>>>(l.items, l.meta, l.meta, l.perm1, l.F1, l.F1 + n1,
                                                            l.F1 + 2 * (size_t)n1, l.b1, r1, v1, renc1, dt, cap, o1, o2,
-                                                           olv, count, nullptr);
+                                                           olv, count, nullptr, p.pchunk);
         c->launches++;
         return launch_status(c, "encounter_sorted");
     }
