@@ -699,8 +699,11 @@ namespace swg {
 // From this many pair tests on, a TRIANGULAR check of one list, or of massive bodies against test
 // particles, goes over radius-sorted tiles, which test a few percent of a disk's pairs but take
 // two launches more; whole calls all-pairs / sorted: 300 x 20,000 66 / 67 us, 1000 x 10,000 72 / 72,
-// 400 x 50,000 93 / 72, 8192 x 50,000 935 / 112.
+// 400 x 50,000 93 / 72, 8192 x 50,000 935 / 112.  Against fewer massive bodies than SORTED_PL the
+// ordering of the test particles costs more than it saves: 8 x 1,251,251 97 / 135 us, 32 x 312,813
+// 61 / 74, 48 x 2,000,001 292 / 249, 64 x 156,407 105 / 83.
 constexpr int64_t SORTED_PAIRS = 10000000;
+constexpr int SORTED_PL = 64;
 
 int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1, const double *r1,
                          const double *v1, const double *renc1, int32_t n2, const double *r2, const double *v2,
@@ -714,7 +717,7 @@ int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1,
         SWG_TRY(ensure(c, w.raw, (size_t)w.rawcap * 3 * sizeof(int32_t)));
     }
     const int64_t pairs = kind == 0 ? (int64_t)n1 * n1 / 2 : (int64_t)n1 * n2;
-    const bool sorted = mode == SWG_ENC_TRIANGULAR && kind != 1 && pairs >= SORTED_PAIRS;
+    const bool sorted = mode == SWG_ENC_TRIANGULAR && kind != 1 && n1 >= SORTED_PL && pairs >= SORTED_PAIRS;
     SWG_TRY(ensure(c, w.sort, sorted ? encounter_sorted_one_bytes(n1, kind == 0 ? 0 : n2)
                                      : encounter_scratch_bytes(mode, n1, kind == 0 ? n1 : n2)));
     unsigned long long h_count = 0;

@@ -43,3 +43,16 @@ def test_ring_time(ctx):
     own = best(lambda: ctx.encounter_check_all_plpl(r, v, renc, 0.005, cap=100000))
     both = best(lambda: ctx.encounter_check_all_pltp(r, v, r, v, renc, 0.005, cap=100000))
     assert own < 1.5 * both
+
+
+# below and from the count of massive bodies on with which long lists are sorted (encounter.cu SORTED_PL)
+@pytest.mark.parametrize("npl", [1, 8, 63, 64])
+def test_few_massive_bodies(ctx, npl):
+    _, pl, tp = IC.make_system(seed=npl, npl=npl, ntp=10000000 // npl + 1 if npl > 1 else 1000, amin=0.3, amax=3.0)
+    near = slice(0, len(tp["rh"]), 1 + len(tp["rh"]) // 500)
+    tp["rh"][near] = pl["rh"][0] * (1 + 1e-5)
+    args = pl["rh"], pl["vh"], tp["rh"], tp["vh"], 3.0 * pl["rhill"], 0.005
+    g, o = ctx.encounter_check_all_pltp(*args, cap=100000), O.encounter_pltp(*args)
+    assert len(o[0]) > 100
+    for a, b in zip(g, o):
+        assert np.array_equal(a, b)
