@@ -6,7 +6,8 @@
 // fastest.  Choices are kept for the process and appended to a small text file so later
 // runs skip the timing: $SWG_TUNE_CACHE if set, else $HOME/.cache/swiftest_gb300/kick_tune.txt
 // (no file is written when neither is available).  One line per choice: "<key> <variant>".
-// The symmetric pl-pl kick's strip length is kept the same way, as log2(strip).
+// The symmetric pl-pl kick's shape is kept the same way, packed into one number (ensure_kick_plan).
+// The file is read as it is found: whoever looks a choice up checks that it is one of its own.
 #include <cuda_runtime.h>
 #include <sys/stat.h>
 
@@ -46,7 +47,7 @@ void load_locked() {
     char key[512];
     int v = 0;
     while (std::fscanf(f, "%511s %d", key, &v) == 2)
-        if (v >= 0 && v < 512) g_tune[key] = v;  // packed shapes; callers check the range of their own keys
+        if (v >= 0) g_tune[key] = v;
     std::fclose(f);
 }
 

@@ -930,7 +930,7 @@ int ensure_kick_plan(swg_ensemble *e, int k, bool rad, unsigned *head, const int
         const std::string key =
             tune_key(c->device, k == 0 ? (rad ? "kick_pl_rad" : "kick_pl") : "kick_tp", size_bucket(e, k));
         v = tune_lookup(key);
-        if (v < 0) {
+        if (v < 0 || v >= KICK_NVARIANT) {  // not cached, or not a shape
             SWG_TRY(time_kick_variants(e, k, rad, head, flag, phase, &v));
             tune_store(key, v);
         }
