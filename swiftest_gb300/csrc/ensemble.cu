@@ -216,7 +216,7 @@ int upload(swg_ctx *c, T *dst, const std::vector<T> &src) {
 constexpr int ENS_SUM_T = 256;
 
 // one block per system: swiftest_util_coord_vh2vb_pl (only systems whose first-step
-// flag is set when lfirst != nullptr), helio_drift_linear_pl, swiftest_util_coord_vb2vh_pl
+// flag is set when lfirst != nullptr), helio_drift_linear_pl
 __global__ void __launch_bounds__(ENS_SUM_T) k_ens_vh2vb(const int32_t *__restrict__ poff, const int32_t *__restrict__ npl,
                                                   const int32_t *__restrict__ lfirst, const double *__restrict__ Gm,
                                                   const double *__restrict__ vh, double *vb,
@@ -237,17 +237,6 @@ __global__ void __launch_bounds__(ENS_SUM_T) k_ens_lindrift(const int32_t *__res
     const size_t o = poff[s];
     blk_lindrift_pl(npl[s], Gm + o, vb + 3 * o, lmask + o, GMcb[s], rh + 3 * o, dt, dcb + CB_N * s, slot, exact, sh);
 }
-__global__ void __launch_bounds__(ENS_SUM_T) k_ens_vb2vh(const int32_t *__restrict__ poff, const int32_t *__restrict__ npl,
-                                                  const double *__restrict__ Gm, const double *__restrict__ vb,
-                                                  const int32_t *__restrict__ status, double *vh,
-                                                  const double *__restrict__ GMcb, double *dcb, int exact) {
-    const int s = blockIdx.x;
-    if (npl[s] == 0) return;
-    __shared__ SumScratch sh;
-    const size_t o = poff[s];
-    blk_vb2vh_pl(npl[s], Gm + o, vb + 3 * o, status + o, vh + 3 * o, GMcb[s], dcb + CB_N * s, exact, sh);
-}
-
 // closing linear drift and vb2vh of the FP64 path
 __global__ void __launch_bounds__(ENS_SUM_T) k_ens_close(const int32_t *__restrict__ poff, const int32_t *__restrict__ npl,
                                                   const double *__restrict__ Gm, const double *__restrict__ vb,
@@ -1077,12 +1066,9 @@ int vh2vb_pl(swg_ensemble *e, bool first_only) {
                                                   e->vb, e->GMcb, e->dcb, exact(e));
     return L(e->c, "ens_vh2vb");
 }
-int vb2vh_pl(swg_ensemble *e) {
+int vb2vh_pl(swg_ensemble *e) {  // mixed path; the FP64 path's is part of k_ens_close
     if (e->NPL == 0) return SWG_OK;
-    if (!exact(e)) return chunk_sum<SUM_VB2VH>(e, nullptr, e->vb, e->status, e->vb, e->vh, 0.0, 0);
-    k_ens_vb2vh<<<e->nsys, ENS_SUM_T, 0, e->c->stream>>>(e->poff, e->npl, e->Gmass, e->vb, e->status, e->vh, e->GMcb, e->dcb,
-                                                  exact(e));
-    return L(e->c, "ens_vb2vh");
+    return chunk_sum<SUM_VB2VH>(e, nullptr, e->vb, e->status, e->vb, e->vh, 0.0, 0);
 }
 // The mixed path's closing pl half-step in two passes over the chunks (close_pl): the
 // closing velocity kick (k_kick_update's operation, with the copy of rh to rcopy for the

@@ -228,40 +228,8 @@ static __device__ void blk_vh2vb_pl(int npl, const double *__restrict__ Gm,
     }
 }
 
-// swiftest_util_coord_vb2vh_pl (swiftest_util.f90:363-392), reverse-order sum.  The
-// reference divides every term by GMcb; the non-exact path multiplies by the reciprocal
-// instead (an FP64 divide is ~20 instructions on the narrow FP64 pipe).
-static __device__ void blk_vb2vh_pl(int npl, const double *__restrict__ Gm,
-                                                 const double *__restrict__ vb, const int32_t *__restrict__ status,
-                                                 double *vh, double GMcb, double *dcb, int exact, SumScratch &sh) {
-    const double inv = 1.0 / GMcb;
-    auto term = [&](int i, double &x, double &y, double &z) -> unsigned char {
-        if (exact) {
-            x = xdiv(Gm[i] * vb[3 * i + 0], GMcb);
-            y = xdiv(Gm[i] * vb[3 * i + 1], GMcb);
-            z = xdiv(Gm[i] * vb[3 * i + 2], GMcb);
-        } else {
-            const double g = Gm[i] * inv;
-            x = g * vb[3 * i + 0];
-            y = g * vb[3 * i + 1];
-            z = g * vb[3 * i + 2];
-        }
-        return status[i] != ST_INACTIVE;
-    };
-    const Sum3 s = ordered_sum3(npl, true, exact != 0, term, -1.0, sh);
-    if (threadIdx.x == 0) {
-        dcb[CB_VB + 0] = s.x;
-        dcb[CB_VB + 1] = s.y;
-        dcb[CB_VB + 2] = s.z;
-    }
-    for (int i = threadIdx.x; i < npl; i += blockDim.x) {
-        vh[3 * i + 0] = vb[3 * i + 0] - s.x;
-        vh[3 * i + 1] = vb[3 * i + 1] - s.y;
-        vh[3 * i + 2] = vb[3 * i + 2] - s.z;
-    }
-}
-
-// The end of a step in the FP64 path: helio_drift_linear_pl, then swiftest_util_coord_vb2vh_pl.  The
+// The end of a step in the FP64 path: helio_drift_linear_pl, then swiftest_util_coord_vb2vh_pl
+// (swiftest_util.f90:363-392, a reverse-order sum of terms each divided by GMcb).  The
 // linear drift leaves vb as it is, so both sums (one forward, one in reverse order) run
 // together, six lanes in one addition.  rcopy, vcopy: copies of the resulting state.  rnext: the
 // opening linear drift of a step that follows at once, whose sum is the closing one's (vb, the

@@ -135,13 +135,6 @@ __global__ void __launch_bounds__(RB) k_vh2vb_pl(int npl, const double *__restri
     __shared__ SumScratch sh;
     blk_vh2vb_pl(npl, Gm, vh, vb, GMcb, dcb, exact, sh);
 }
-__global__ void __launch_bounds__(RB) k_vb2vh_pl(int npl, const double *__restrict__ Gm,
-                                                 const double *__restrict__ vb, const int32_t *__restrict__ status,
-                                                 double *vh, double GMcb, double *dcb, int exact) {
-    __shared__ SumScratch sh;
-    blk_vb2vh_pl(npl, Gm, vb, status, vh, GMcb, dcb, exact, sh);
-}
-
 __global__ void __launch_bounds__(RB) k_close_pl(int npl, const double *__restrict__ Gm,
                                                  const double *__restrict__ vb, const int32_t *__restrict__ lmask,
                                                  const int32_t *__restrict__ status, double GMcb, double *rh,
@@ -461,11 +454,9 @@ int vh2vb_pl(swg_system *s) {
     k_vh2vb_pl<<<1, RB, 0, s->c->stream>>>(s->npl, s->Gmass, s->vh, s->vb, s->GMcb, s->dcb, exact(s));
     return L(s->c, "vh2vb_pl");
 }
-int vb2vh_pl(swg_system *s) {
+int vb2vh_pl(swg_system *s) {  // mixed path; the FP64 path's is part of close_pl
     if (s->npl == 0) return SWG_OK;
-    if (!exact(s)) return chunk_sum<SUM_VB2VH>(s, s->vb, s->status, s->vb, s->vh, 0.0, 0);
-    k_vb2vh_pl<<<1, RB, 0, s->c->stream>>>(s->npl, s->Gmass, s->vb, s->status, s->vh, s->GMcb, s->dcb, exact(s));
-    return L(s->c, "vb2vh_pl");
+    return chunk_sum<SUM_VB2VH>(s, s->vb, s->status, s->vb, s->vh, 0.0, 0);
 }
 // Steps in a row whose discard scan runs beside the next step (discard_aside): the state that
 // the scan reads, and (FP64 path) the next step's opening linear drift in the closing kernel.
