@@ -3,22 +3,24 @@
 // Restates encounter_check_all_plpl / _plplm / _pltp (src/encounter/encounter_check.f90:14-140)
 // in both of the reference's modes:
 //   * TRIANGULAR (:384-570): every pair is tested with encounter_check_one (:573-621).
+//     Long checks go over radius-sorted tiles instead (encounter_sorted.cu, SORTED_PAIRS).
 //   * SORTSWEEP  (:143-326, :763-988): 1-D radial bounding boxes |r| +- 1.1 renc,
-//     sorted by a stable radix sort on the extents (radix_sort.cu; ties by extent index);
+//     sorted by extent, ties by extent index: one system's in tiles that are merged
+//     (SAS_MERGED), longer lists and ensembles by a stable radix sort (radix_sort.cu);
 //     each body whose box holds >= 2 foreign extents strictly inside (the reference's
 //     loverlap test) tests the bodies whose extents lie inside.
 //
 // The encounter decision is made in FP64 with the reference's expression order
 // (this file is compiled with -fmad=false), so lists are bit-identical to the
-// reference loop.  In TRIANGULAR mode a conservative FP32 prefilter first
+// reference loop.  In both modes a conservative FP32 prefilter first
 // rejects pairs whose closest approach over the step provably exceeds the
 // encounter radius (min_t |x + v t| >= |x| - |v| |dt|; see prefilter_reject for
 // the margins).  Only pairs the FP64 test could accept reach it, so the
 // prefilter changes speed, never the list.
 //
 // Output: pairs are appended with an atomic counter (up to cap), then sorted by
-// (index1, index2) with a bitonic sort (single CTA in shared memory when the
-// padded length fits, else global compare-exchange passes); the lists are short.
+// (index1, index2), packed with lvdotr into one key: up to PAIRS_BLOCK pairs in one block,
+// longer lists in tiles of MERGE_TILE that are merged MERGE_WAYS at a time.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

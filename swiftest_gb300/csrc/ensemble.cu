@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(RECT) k_ens_symba_recursion(EnsRecArgs e, int 
 }
 
 // ---- WHM (whm_step.f90, whm_kick.f90, whm_coord.f90) of every system: one block per system
-// for the Jacobi running sums (FP64 path: one thread, in the reference's order)
+// for the Jacobi running sums (FP64 path: in the reference's order, a lane per component)
 enum { WHM_H2J = 0, WHM_J2H = 1, WHM_VH2VJ = 2 };
 __global__ void k_ens_whm_coord(int mode, const int32_t *__restrict__ poff, const int32_t *__restrict__ npl,
                                 const double *Gm, const double *eta, double *rh, double *vh, double *xj, double *vj,

@@ -18,10 +18,12 @@
 //     midpoint the exact remainder decides (Markstein's remainder test; neither a square
 //     root nor a quotient of 53-bit numbers is ever a midpoint).
 //
-// Valid for normal operands with exponents within +-XR_EXP of one (x_ok); the callers send
+// Valid for positive normal operands with a normal result.  The callers pass operands with exponents within
+// +-XR_EXP of one (x_ok), or results of such operands whose exponents stay normal, and send
 // everything else (zeros, subnormals, infinities, NaN, extreme exponents) to the native
-// operations.  Each function reports in `bad` the lanes it could not decide (an estimate
-// that falls into the neighbouring binade, about one in 2^22), which take the native form too.
+// operations.  Each function reports in `bad` the lanes it could not decide, which take the native
+// form too: an estimate that falls into the neighbouring binade, about one random operand in 2^22, and
+// in x_div every divisor that is a power of two (its reciprocal's estimate is one).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -130,7 +132,7 @@ __device__ __forceinline__ XNum x_num(double g) {
     return a;
 }
 
-// g / p, both x_ok.  The FP32 pair is off by at most 450 units in the last place; the
+// g / p, normal with a normal quotient.  The FP32 pair is off by at most 450 units in the last place; the
 // remainder wraps at 1024.
 __device__ __forceinline__ double x_div(const XNum &g, double p, bool &bad) {
     const int hi = __double2hiint(p), lo = __double2loint(p);

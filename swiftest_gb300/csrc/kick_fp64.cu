@@ -149,7 +149,7 @@ __device__ __forceinline__ void fp64_group(int RT, int nrecv, int npart, int npl
                 bad |= !x_ok(h) || !x_ok(__double2hiint(g));
                 if (RAD) near = !(__int_as_float((h - ((1023 - 127) << 20)) << 3) > __fadd_ru(rbi, radius_bound(R[j])));
                 const double s = x_sqrt(r2, bad);
-                const double p = x_mul(r2, s);
+                const double p = x_mul(r2, s);  // within 2^+-152: g / p and the terms stay normal
                 double fac;
                 if (MODE == KICK_SPLIT) {
                     const XNum one = {1.0f, 0.0f, 0x3ff00000, 0};

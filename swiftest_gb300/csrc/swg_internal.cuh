@@ -359,7 +359,8 @@ int encounter_sorted_one(swg_ctx *c, int n1, const double *r1, const double *v1,
                          int32_t *olv, unsigned long long *count, void *scratch);
 
 // Full check of one kind (0 plpl, 1 plplm, 2 pltp): sorted unique pairs in the
-// workspace's raw buffers; *n_out gets the count (host).  Synchronizes.
+// workspace's raw buffers; *n_out gets the count (host).  Waits for the count; a TRIANGULAR check
+// returns with the sort of its pairs queued on the stream.
 int encounter_check_kind(swg_ctx *c, EncWork &w, int kind, int mode, int32_t n1, const double *r1,
                          const double *v1, const double *renc1, int32_t n2, const double *r2, const double *v2,
                          const double *renc2, double dt, int64_t *n_out, int32_t **i1, int32_t **i2, int32_t **lv);

@@ -1702,10 +1702,10 @@ static __device__ void blk_energy_final(int n, int whm, const double *rh, const 
 // ---- WHM (Jacobi coordinates)
 // The reference's Jacobi conversions and the ah0 / ah2 accelerations are running sums over
 // the bodies in index order.  Here the whole block forms the terms (products and quotients)
-// into shared memory, the running sums are taken (exact: one thread per component adds
+// into shared memory, the running sums are taken (exact: one lane per component adds
 // them in index order with the reference's operands, so FP64 results stay bit-identical;
 // mixed path: a segmented warp scan per component), and the block uses them; bodies go
-// through in chunks of WCH.
+// through in chunks (whm_exact_running; mixed path: of WCH).
 constexpr int WCH = 512;
 struct WhmScratch {
     double t[6][WCH];      // terms, then (in place) inclusive running sums
