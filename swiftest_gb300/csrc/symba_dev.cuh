@@ -639,22 +639,17 @@ __device__ __forceinline__ KickFac d_kick_factors(bool fast, bool both, double b
 }
 
 // Component c's terms of one pair (t: the entry's terms + c): +1 kick of index1 and index2 at 0 and
-// 3, -1 kick at 6 and 9 (a pl-tp entry: the tp's at 0 and 6).
-__device__ __forceinline__ void kick_terms(bool fast, bool isp, const KickFac &f, double gm1, double gm2, double dc,
-                                           double *t) {
-    if (fast) {  // G m dc shared by the signs
-        const double g1 = gm1 * dc, g2 = gm2 * dc;
-        if (f.kp) t[0] = f.fp * (isp ? g2 : g1);
-        if (f.kp && isp) t[3] = f.fp * g1;
-        if (f.km) t[6] = f.fm * (isp ? g2 : g1);
-        if (f.km && isp) t[9] = f.fm * g1;
-        return;
+// 3, -1 kick at 6 and 9 (a pl-tp entry: the tp's at 0 and 6).  Factor times mass, then displacement, in
+// either path.
+__device__ __forceinline__ void kick_terms(bool isp, const KickFac &f, double gm1, double gm2, double dc, double *t) {
+    const double g2 = isp ? gm2 : gm1;
+    if (f.kp) {
+        t[0] = (f.fp * g2) * dc;
+        if (isp) t[3] = (f.fp * gm1) * dc;
     }
-    for (int sg = 0; sg < 2; sg++) {
-        if (!(sg == 0 ? f.kp : f.km)) continue;
-        const double fac = sg == 0 ? f.fp : f.fm;
-        t[6 * sg] = (isp ? fac * gm2 : fac * gm1) * dc;
-        if (isp) t[6 * sg + 3] = (fac * gm1) * dc;
+    if (f.km) {
+        t[6] = (f.fm * g2) * dc;
+        if (isp) t[9] = (f.fm * gm1) * dc;
     }
 }
 
@@ -782,7 +777,7 @@ static __device__ void blk_kick_lists(const RecArgs &a, int nbpl, int nbtp, doub
             a.good2[k] = both ? (f.km ? 1 : 2) : 0;
         }
         const double dc = c == 0 ? dx[0] : (c == 1 ? dx[1] : dx[2]);
-        kick_terms(a.fast, isp, f, a.Gm[i], isp ? a.Gm[j] : 0.0, dc, &a.terms[12 * k + c]);
+        kick_terms(isp, f, a.Gm[i], isp ? a.Gm[j] : 0.0, dc, &a.terms[12 * k + c]);
     }
     __syncthreads();
     // ordered per-body accumulation and the velocity kicks, +1 then -1; three items per body,
@@ -1293,7 +1288,7 @@ static __device__ void stg_kick_lists(const RecArgs &a, const RecStage &S, int n
             S.good2[k] = both ? (f.km ? 1 : 2) : 0;
         }
         const double dc = c == 0 ? dx[0] : (c == 1 ? dx[1] : dx[2]);
-        kick_terms(a.fast, isp, f, S.gm[b1], S.gm[b2], dc, &S.terms[12 * k + c]);
+        kick_terms(isp, f, S.gm[b1], S.gm[b2], dc, &S.terms[12 * k + c]);
     }
     __syncthreads();
     // three items per body, one per vector component c: each adds its component of the

@@ -1,6 +1,7 @@
 """Accuracy of the recursion's kick factors in the mixed path (symba_dev.cuh d_kick_factors): against
 extended precision on the host, no larger than with a native rsqrt each of r^2 and the
-shell's radius.  The device function is compiled into a probe."""
+shell's radius; and the order of the terms' products (kick_terms).  The device functions are compiled
+into a probe."""
 import ctypes as C
 import subprocess
 
@@ -32,18 +33,23 @@ __global__ void k(int n, const double *r2, const double *base, const int *lev, c
     const double rr = fma(-r, rsqrt(ri), 1.0) * (1.0 / (1.0 - RSHELL));
     o[3 * n + i] = ((y * y) * y) * fma(rr * rr, fma(2.0, rr, -3.0), 1.0);
     o[4 * n + i] = ri;
+    double t[12];
+    sdev::kick_terms(true, {true, true, a.fp, b.fm}, 3.0e-7, 7.0e-9, d[0], t);
+    o[5 * n + i] = t[0];
+    o[6 * n + i] = t[9];
+    o[7 * n + i] = d[0];
 }
 extern "C" int probe(int n, const double *r2, const double *base, const int *lev, int m, const double *pw, double *o) {
     const size_t b = sizeof(double) * n;
     double *d;
     int *l;
-    if (cudaMalloc(&d, 8 * b + 8 * m) || cudaMalloc(&l, 4 * n)) return 1;
+    if (cudaMalloc(&d, 10 * b + 8 * m) || cudaMalloc(&l, 4 * n)) return 1;
     cudaMemcpy(d, r2, b, cudaMemcpyHostToDevice);
     cudaMemcpy(d + n, base, b, cudaMemcpyHostToDevice);
-    cudaMemcpy(d + 8 * n, pw, 8 * m, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + 10 * n, pw, 8 * m, cudaMemcpyHostToDevice);
     cudaMemcpy(l, lev, 4 * n, cudaMemcpyHostToDevice);
-    k<<<(n + 127) / 128, 128>>>(n, d, d + n, l, d + 8 * n, d + 2 * n);
-    cudaMemcpy(o, d + 2 * n, 5 * b, cudaMemcpyDeviceToHost);
+    k<<<(n + 127) / 128, 128>>>(n, d, d + n, l, d + 10 * n, d + 2 * n);
+    cudaMemcpy(o, d + 2 * n, 8 * b, cudaMemcpyDeviceToHost);
     cudaFree(d);
     cudaFree(l);
     return (int)cudaGetLastError();
@@ -63,14 +69,14 @@ def values(tmp_path_factory):
     pw = RSHELL ** np.arange(2 * LEVELS + 2)
     # inside the shell, clear of its two edges (whose sides the factors do not share)
     r2 = base * pw[2 * lev] * rng.uniform(RSHELL * (1 + 1e-9), 1 - 1e-9, N) ** 2
-    o = np.zeros((5, N))
+    o = np.zeros((8, N))
     p = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
     assert C.CDLL(str(tmp / "probe.so")).probe(N, p(r2), p(base), p(lev), len(pw), p(pw), p(o)) == 0
     return o
 
 
 def test_shell_factors(values):
-    x, fp, fm, native, ri = values
+    x, fp, fm, native, ri = values[:5]
     x, ri = x.astype(np.longdouble), ri.astype(np.longdouble)
     r = np.sqrt(x)
     rr = (1 - r / np.sqrt(ri)) / (1 - np.longdouble(RSHELL))
@@ -79,3 +85,8 @@ def test_shell_factors(values):
     rms = lambda v: float(np.sqrt((((v - exact) / ir3) ** 2).mean()) * 2.0 ** 53)  # noqa: E731
     # the sample's spread of an rms over 400,000 values is 0.1 to 0.2%
     assert rms(fp) < 1.01 * rms(native) and rms(fm) < 1.01 * rms(native)
+
+
+def test_term_products(values):
+    _, fp, fm, _, _, t0, t9, d = values
+    assert np.array_equal(t0, (fp * 7.0e-9) * d) and np.array_equal(t9, (fm * 3.0e-7) * d)
