@@ -592,7 +592,7 @@ __device__ __forceinline__ double d_shell_base(bool isp, double rhill1, double r
 // lies in (the -1 kick's inner limit is the +1 kick's outer one), CUDA's own, off by 0.506 units in
 // the last place at most; an FP32 pair with one Newton step was off by 0.99, with
 // 1 / sqrt(ri) as a product of 1 / sqrt(base) and a table of RSHELL^-k the polynomial's
-// error grew from 1.8 to 2.5 units of 2^-53 rms, for a kick of 4.85k instead of 5.0k cycles.  FP64 path: the
+// error grew from 1.8 to 2.5 units of 2^-53 rms, for a kick of 4.9k instead of 5.1k cycles.  FP64 path: the
 // reference's operations, with IEEE square roots and quotients (fp64_exact.cuh) and the correctly
 // rounded r^-1.5 shared with the oracle.
 struct KickFac {
